@@ -76,6 +76,7 @@ struct HostTables {
   std::vector<double> t64;
   std::vector<float> t32, t32v;   // t32v: the FP32 kernels' layout (sf_internal.h)
   std::vector<float4> tdd;         // the FP64 table as dd rows (sf_internal.h)
+  std::vector<double> boys;        // Boys functions (sf_internal.h)
   RysAsym asym;
   RysAsym32 asym32;
 };
@@ -94,6 +95,8 @@ const HostTables &host_tables() {
     T.t32.assign(rys_tab_size(kTabDeg32), 0.0f);
     std::memset(&T.asym, 0, sizeof(T.asym));
     rys_build_tables(T.t64.data(), T.t32.data(), &T.asym);
+    T.boys.assign(kBoysTab, 0.0);
+    boys_build_table(T.boys.data());
     constexpr int D = kTabDeg32;
     T.t32v.assign(rys_tab32v_size(), 0.0f);
     for (int n = 1; n <= kMaxRoots; ++n)
@@ -317,7 +320,7 @@ struct sf_handle {
   DBuf<float4> d_pair32;           // packed FP32 pair geometry (KParams::pair32)
   DBuf<float> d_Ddd;               // density as dd (per build)
   DBuf<float> d_cx32, d_cy32, d_cz32;
-  DBuf<double> d_tab64;
+  DBuf<double> d_tab64, d_boys;
   DBuf<float> d_tab32;
   DBuf<double> d_Jh, d_Kh;
   DBuf<float> d_D32;
@@ -431,6 +434,16 @@ void fill_kparams(sf_handle *h) {
   k.nsm = h->nsm;
   k.natom = h->natom;
   k.err = h->d_err.p;
+}
+
+// tables of the one-electron kernels
+void one_params_tables(const sf_handle *h, OneParams *P) {
+  P->tab64 = h->kp.tab64;
+  P->asym = h->kp.asym;
+  P->pr = h->kp.pr;
+  P->rec = h->kp.p64.rec;
+  P->boys = h->d_boys.p;
+  for (int c = 0; c <= kNumPairClass; ++c) P->cstart[c] = h->cstart[c];
 }
 
 int upload_pairs(sf_handle *h) {
@@ -1412,6 +1425,7 @@ int sf_create(const sf_shell_desc *shells, int32_t nshell, sf_handle **out) {
   SF_CK(h->d_coefs.upload(h->coefs));
   const HostTables &T = host_tables();
   SF_CK(h->d_tab64.upload(T.t64));
+  SF_CK(h->d_boys.upload(T.boys));
   SF_CK(h->d_tab32.upload(T.t32v));
   SF_CK(h->d_tabdd.upload(T.tdd));
   SF_CK(h->d_Ddd.alloc(2 * (size_t)nao * nao));
@@ -2023,8 +2037,7 @@ int sf_grad_one_electron(sf_handle *h, const double *atom_xyz, const double *cha
   P.charges = charges;
   P.natom = natom;
   P.S = P.T = P.V = nullptr;
-  P.tab64 = h->kp.tab64;
-  P.asym = h->kp.asym;
+  one_params_tables(h, &P);
   SF_CK(launch_one_electron_grad(P, D, W, grad, (cudaStream_t)stream));
   return SF_OK;
 }
@@ -2146,8 +2159,7 @@ int sf_one_electron(sf_handle *h, const double *atom_xyz, const double *charges,
   P.S = S;
   P.T = T;
   P.V = V;
-  P.tab64 = h->kp.tab64;
-  P.asym = h->kp.asym;
+  one_params_tables(h, &P);
   SF_CK(launch_one_electron(P, (cudaStream_t)stream));
   return SF_OK;
 }

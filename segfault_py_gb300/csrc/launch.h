@@ -71,6 +71,10 @@ struct OneParams {
   double *S, *T, *V;
   const double *tab64;          // FP64 Rys rule (Boys values of the gradient kernel)
   RysAsym asym;
+  DevPairs pr;                  // canonical shell pairs, class c at [cstart[c], cstart[c + 1])
+  const double *rec;            // their primitive-pair records
+  int cstart[kNumPairClass + 1];
+  const double *boys;           // Boys functions (sf_internal.h)
 };
 
 cudaError_t launch_one_electron(const OneParams &P, cudaStream_t st);

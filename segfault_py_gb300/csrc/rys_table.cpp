@@ -17,9 +17,10 @@
 // precision); the weights follow from the Christoffel function
 // 1/w_i = sum_j p_j(u_i)^2 / ||p_j||^2.
 //
-// Tables: for x in [0, 64) on unit intervals a Chebyshev interpolant of degree
-// 11 (FP64) or 6 (FP32) per function, stored as monomial coefficients in
-// s = 2(x-j)-1 so that the device evaluates it by Horner.  For x >= 64 the
+// Tables: for x in [0, 64) a Chebyshev interpolant per function and interval,
+// stored as monomial coefficients in s (the interval mapped to [-1, 1]) so that
+// the device evaluates it by Horner: degree 11 (FP64) or 6 (FP32) on unit
+// intervals.  For x >= 64 the
 // rule is the large-x limit u_i = r_i / x, w_i = W_i / sqrt(x) (the half-range
 // Gauss-Hermite rule; the neglected terms are O(exp(-x))).
 #include <cmath>
@@ -31,8 +32,9 @@
 namespace sf {
 namespace {
 
-constexpr int kGL = 200;
+constexpr int kPoints = 200;
 
+template <int kGL>
 struct GaussLegendre {
   double x[kGL], w[kGL];
   GaussLegendre() {
@@ -58,14 +60,16 @@ struct GaussLegendre {
   }
 };
 
-const GaussLegendre &gl() {
-  static GaussLegendre g;
+template <int kGL>
+const GaussLegendre<kGL> &gl() {
+  static GaussLegendre<kGL> g;
   return g;
 }
 
-// exact n-point rule at x (u ascending)
+// exact n-point rule at x (u ascending), the measure on kGL points
+template <int kGL>
 void rys_exact(int n, double x, double *u, double *w) {
-  const GaussLegendre &G = gl();
+  const GaussLegendre<kGL> &G = gl<kGL>();
   const double T = (x <= 100.0) ? 1.0 : 10.0 / std::sqrt(x);
   double uu[kGL], om[kGL], p0[kGL], p1[kGL];
   for (int k = 0; k < kGL; ++k) {
@@ -150,7 +154,7 @@ void fill_table(T *tab, int deg) {
     for (int j = 0; j < kTabNint; ++j) {
       for (int k = 0; k <= deg; ++k) {
         double x = j + 0.5 * (sk[k] + 1.0);
-        rys_exact(n, x, &vals[k * 2 * n], &vals[k * 2 * n + n]);
+        rys_exact<kPoints>(n, x, &vals[k * 2 * n], &vals[k * 2 * n + n]);
       }
       for (int f = 0; f < 2 * n; ++f) {
         for (int i = 0; i <= deg; ++i) {
@@ -165,7 +169,57 @@ void fill_table(T *tab, int deg) {
   }
 }
 
+// Chebyshev interpolation at the kTabDegF + 1 nodes of a fine interval
+struct FineNodes {
+  double s[kTabDegF + 1], t[kTabDegF + 1][kTabDegF + 1];   // nodes, T_i at node k
+  FineNodes() {
+    const double pi = 3.14159265358979323846;
+    for (int k = 0; k <= kTabDegF; ++k) s[k] = std::cos(pi * (k + 0.5) / (kTabDegF + 1));
+    for (int i = 0; i <= kTabDegF; ++i)
+      for (int k = 0; k <= kTabDegF; ++k) t[i][k] = std::cos(i * std::acos(s[k]));
+  }
+  double x(int j, int k) const { return (j + 0.5 * (s[k] + 1.0)) / kTabHF; }
+  // monomial coefficients m[0 .. kTabDegF] from the values v[k * stride]
+  void fit(const double *v, int stride, double *m) const {
+    double c[kTabDegF + 1];
+    for (int i = 0; i <= kTabDegF; ++i) {
+      double a = 0.0;
+      for (int k = 0; k <= kTabDegF; ++k) a += v[k * stride] * t[i][k];
+      c[i] = a * 2.0 / (kTabDegF + 1) * (i == 0 ? 0.5 : 1.0);
+    }
+    cheb_to_mono(c, kTabDegF, m);
+  }
+};
+
 }  // namespace
+
+// Boys functions and e^-T (sf_internal.h), interpolated at the Chebyshev nodes
+// of every interval: the highest order from its power series
+// F_n = e^-T sum_i (2T)^i / ((2n+1)(2n+3)...(2n+2i+1)), the others by the
+// downward recursion.
+void boys_build_table(double *tab) {
+  constexpr int D = kTabDegF, NF = kBoysMax + 2;
+  const FineNodes N;
+  double v[(D + 1) * NF], m[D + 1];
+  for (int j = 0; j < kTabNintF; ++j) {
+    for (int k = 0; k <= D; ++k) {
+      const double T = N.x(j, k), e = std::exp(-T);
+      double *F = v + k * NF, term = 1.0 / (2 * kBoysMax + 1), sum = term;
+      for (int i = 1; i < 400 && term > 1e-18 * sum; ++i) {
+        term *= 2.0 * T / (2 * kBoysMax + 2 * i + 1);
+        sum += term;
+      }
+      F[kBoysMax] = e * sum;
+      for (int n = kBoysMax - 1; n >= 0; --n) F[n] = (2.0 * T * F[n + 1] + e) / (2 * n + 1);
+      F[kBoysMax + 1] = e;
+    }
+    for (int f = 0; f < NF; ++f) {
+      N.fit(v + f, NF, m);
+      double *row = tab + ((size_t)f * kTabNintF + j) * (D + 1);
+      for (int i = 0; i <= D; ++i) row[D - i] = m[i];
+    }
+  }
+}
 
 void rys_build_tables(double *tab64, float *tab32, RysAsym *asym) {
   fill_table<double>(tab64, kTabDeg64);
@@ -173,7 +227,7 @@ void rys_build_tables(double *tab64, float *tab32, RysAsym *asym) {
   const double X = 1e7;
   for (int n = 1; n <= kMaxRoots; ++n) {
     double u[kMaxRoots], w[kMaxRoots];
-    rys_exact(n, X, u, w);
+    rys_exact<kPoints>(n, X, u, w);
     for (int i = 0; i < n; ++i) {
       asym->r[n][i] = u[i] * X;
       asym->w[n][i] = w[i] * std::sqrt(X);

@@ -40,6 +40,15 @@ __host__ __device__ constexpr int rys_tab_offset(int n, int deg) {
 }
 __host__ __device__ constexpr int rys_tab_size(int deg) { return rys_tab_offset(kMaxRoots + 1, deg); }
 
+// The Boys functions F_0 .. F_kBoysMax and e^-T on intervals of 1/kTabHF, degree
+// kTabDegF: per function and interval the kTabDegF + 1 coefficients from high to
+// low order.
+constexpr int kTabHF = 8;
+constexpr int kTabNintF = 64 * kTabHF;
+constexpr int kTabDegF = 7;
+constexpr int kBoysMax = 5;
+constexpr int kBoysTab = (kBoysMax + 2) * kTabNintF * (kTabDegF + 1);
+
 // Layout of the FP32 table read by the kernels: per n-root block, interval j,
 // root r, one row of kTab32Row floats holding the coefficient pairs
 // (u_k, w_k) from k = kTabDeg32 down to 0 (the Horner order): one root costs
@@ -106,6 +115,7 @@ struct RysAsym32 {                      // the same constants rounded to FP32
 
 // host-side: build tables (rys_table.cpp)
 void rys_build_tables(double *tab64, float *tab32, RysAsym *asym);
+void boys_build_table(double *tab);
 void rys_eval_host(const double *tab64, const float *tab32, const RysAsym &as, int n, double x, int fp32,
                    double *u, double *w);
 
