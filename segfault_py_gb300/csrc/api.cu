@@ -75,7 +75,7 @@ struct DBuf {
 struct HostTables {
   std::vector<double> t64;
   std::vector<float> t32, t32v;   // t32v: the FP32 kernels' layout (sf_internal.h)
-  std::vector<float4> tdd;         // the FP64 table as dd rows (sf_internal.h)
+  std::vector<float4> tdd;         // the fine table as dd rows (sf_internal.h)
   std::vector<double> boys;        // Boys functions (sf_internal.h)
   RysAsym asym;
   RysAsym32 asym32;
@@ -97,6 +97,8 @@ const HostTables &host_tables() {
     rys_build_tables(T.t64.data(), T.t32.data(), &T.asym);
     T.boys.assign(kBoysTab, 0.0);
     boys_build_table(T.boys.data());
+    std::vector<double> fine(rys_fine_size());
+    rys_build_fine(fine.data());
     constexpr int D = kTabDeg32;
     T.t32v.assign(rys_tab32v_size(), 0.0f);
     for (int n = 1; n <= kMaxRoots; ++n)
@@ -114,15 +116,20 @@ const HostTables &host_tables() {
         T.asym32.r[n][i] = (float)T.asym.r[n][i];
         T.asym32.w[n][i] = (float)T.asym.w[n][i];
       }
-    constexpr int D64 = kTabDeg64;
+    constexpr int DF = kTabDegF;
     T.tdd.assign(rys_tabdd_size(), make_float4(0.f, 0.f, 0.f, 0.f));
     for (int n = 1; n <= kMaxRoots; ++n)
-      for (int j = 0; j < kTabNint; ++j)
+      for (int j = 0; j < kTabNintF; ++j)
         for (int r = 0; r < n; ++r) {
-          float4 *row = T.tdd.data() + rys_tabdd_offset(n) + (j * n + r) * (D64 + 1);
-          const double *src = T.t64.data() + rys_tab_offset(n, D64) + j * (D64 + 1) * 2 * n;
-          for (int k = D64; k >= 0; --k) {
-            float4 &c = row[D64 - k];
+          float4 *row = T.tdd.data() + rys_tabdd_offset(n) + (j * n + r) * kTabDDRow;
+          const double *src = fine.data() + rys_fine_offset(n) + j * (DF + 1) * 2 * n;
+          float *top = reinterpret_cast<float *>(row);
+          for (int k = 0; k < kDDTop; ++k) {
+            top[2 * k] = (float)src[(DF - k) * 2 * n + r];
+            top[2 * k + 1] = (float)src[(DF - k) * 2 * n + n + r];
+          }
+          for (int k = DF - kDDTop; k >= 0; --k) {
+            float4 &c = row[(kDDTop + 1) / 2 + DF - kDDTop - k];
             dd_split(src[k * 2 * n + r], c.x, c.y);
             dd_split(src[k * 2 * n + n + r], c.z, c.w);
           }

@@ -10,7 +10,9 @@
 // The building blocks are the error-free transformations of Knuth (TwoSum),
 // Dekker (FastTwoSum) and the FMA form of TwoProduct; the "sloppy" addition
 // and the multiplication follow the double-double algorithms of Hida, Li and
-// Bailey (QD library paper, 2001), written here for float pairs.
+// Bailey (QD library paper, 2001), written here for float pairs.  The leading
+// product of each is __fmul_rn: a plain one may be contracted into a following
+// addition, whose rounding error the transformation then no longer captures.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -45,14 +47,14 @@ __device__ __forceinline__ dd operator-(dd a) { return dd(-a.hi, -a.lo); }
 __device__ __forceinline__ dd operator-(dd a, dd b) { return a + (-b); }
 
 __device__ __forceinline__ dd operator*(dd a, dd b) {
-  const float p = a.hi * b.hi;
+  const float p = __fmul_rn(a.hi, b.hi);
   float e = fmaf(a.hi, b.hi, -p);
   e = fmaf(a.hi, b.lo, e);
   e = fmaf(a.lo, b.hi, e);
   return dd_fast_two_sum(p, e);
 }
 __device__ __forceinline__ dd operator*(dd a, float b) {
-  const float p = a.hi * b;
+  const float p = __fmul_rn(a.hi, b);
   float e = fmaf(a.hi, b, -p);
   e = fmaf(a.lo, b, e);
   return dd_fast_two_sum(p, e);
@@ -63,11 +65,29 @@ __device__ __forceinline__ dd operator*(int b, dd a) { return a * (float)b; }
 
 // a*b + c with one renormalisation
 __device__ __forceinline__ dd dd_fma(dd a, dd b, dd c) {
-  const float p = a.hi * b.hi;
+  const float p = __fmul_rn(a.hi, b.hi);
   float e = fmaf(a.hi, b.hi, -p);
   e = fmaf(a.hi, b.lo, e);
   e = fmaf(a.lo, b.hi, e);
   dd s = dd_two_sum(p, c.hi);
+  return dd_fast_two_sum(s.hi, s.lo + (e + c.lo));
+}
+
+__device__ __forceinline__ dd dd_fma(float a, dd b, dd c) {
+  const float p = __fmul_rn(a, b.hi);
+  float e = fmaf(a, b.hi, -p);
+  e = fmaf(a, b.lo, e);
+  dd s = dd_two_sum(p, c.hi);
+  return dd_fast_two_sum(s.hi, s.lo + (e + c.lo));
+}
+
+// a*b + c for |c| >= |a b|
+__device__ __forceinline__ dd dd_fma_big(dd a, dd b, dd c) {
+  const float p = __fmul_rn(a.hi, b.hi);
+  float e = fmaf(a.hi, b.hi, -p);
+  e = fmaf(a.hi, b.lo, e);
+  e = fmaf(a.lo, b.hi, e);
+  dd s = dd_fast_two_sum(c.hi, p);
   return dd_fast_two_sum(s.hi, s.lo + (e + c.lo));
 }
 
@@ -78,19 +98,66 @@ __device__ __forceinline__ dd &operator*=(dd &a, float b) { return a = a * b; }
 
 __device__ __forceinline__ bool operator>=(dd a, float b) { return a.hi > b || (a.hi == b && a.lo >= 0.0f); }
 
-// 1/a: FP32 reciprocal seed, one Newton step y + y (1 - a y) in dd
-__device__ __forceinline__ dd dd_recip(dd a) {
-  const float y0 = 1.0f / a.hi;
-  const dd y(y0);
-  const dd r = dd(1.0f) - a * y;
-  return y + y * r;
+// a*b without the renormalisation: |lo| up to two units of hi's last place,
+// for a factor of dd_acc
+__device__ __forceinline__ dd dd_mul_raw(dd a, dd b) {
+  const float p = __fmul_rn(a.hi, b.hi);
+  float e = fmaf(a.hi, b.hi, -p);
+  e = fmaf(a.hi, b.lo, e);
+  e = fmaf(a.lo, b.hi, e);
+  return dd(p, e);
 }
 
-// 1/sqrt(a): FP32 seed, one Newton step y (3/2 - a/2 y^2) in dd
+// s += a*b for a sum that stays unnormalised (lo gathers the rounding of hi
+// and of the products): 12 instructions, a multiplication and an addition with
+// their renormalisations take 18.  dd_norm before anything but another dd_acc.
+__device__ __forceinline__ void dd_acc(dd &s, dd a, dd b) {
+  const dd m = dd_mul_raw(a, b);
+  const dd t = dd_two_sum(s.hi, m.hi);
+  s = dd(t.hi, s.lo + (t.lo + m.lo));
+}
+__device__ __forceinline__ dd dd_norm(dd a) { return dd_two_sum(a.hi, a.lo); }
+
+// 1 - a for 0 <= a <= 1
+__device__ __forceinline__ dd dd_one_minus(dd a) {
+  const dd s = dd_fast_two_sum(1.0f, -a.hi);
+  return dd_fast_two_sum(s.hi, s.lo - a.lo);
+}
+
+// k*a for a small integer k (2 a is exact)
+__device__ __forceinline__ dd dd_times(int k, dd a) {
+  return k == 1 ? a : k == 2 ? dd(2.0f * a.hi, 2.0f * a.lo) : a * (float)k;
+}
+
+// 1/a: FP32 reciprocal seed y, residual 1 - a y = r - e (r exact, e its FP32
+// rounding terms, about 2^-24): y + y (r - e) + y (r - e)^2, the product y r exact
+__device__ __forceinline__ dd dd_recip(dd a) {
+  const float y = 1.0f / a.hi;
+  const float p = __fmul_rn(a.hi, y);
+  const float e = fmaf(a.lo, y, fmaf(a.hi, y, -p));
+  const float r = 1.0f - p, t = r - e;
+  const float c = __fmul_rn(y, r);
+  const float d = fmaf(y, r, -c) + y * fmaf(t, t, -e);
+  const dd s = dd_fast_two_sum(y, c);
+  return dd_fast_two_sum(s.hi, s.lo + d);
+}
+
+// 1/sqrt(a): FP32 seed y, residual 1 - a y^2 = r - e (r exact), then
+// y + y (r - e) / 2 + 3/8 y (r - e)^2, the product y r / 2 exact: relative error
+// 4e-15 (with the whole correction in FP32, 2e-14, which the 1/(p+q) in the
+// Rys argument x amplifies by x)
 __device__ __forceinline__ dd dd_rsqrt(dd a) {
-  const dd y(rsqrtf(a.hi));
-  const dd h = a * 0.5f;
-  return y * (dd(1.5f) - h * (y * y));
+  const float y = rsqrtf(a.hi);
+  const float q = __fmul_rn(y, y), ql = fmaf(y, y, -q);
+  const float p = __fmul_rn(a.hi, q);
+  float e = fmaf(a.hi, q, -p);
+  e = fmaf(a.hi, ql, e);
+  e = fmaf(a.lo, q, e);
+  const float r = 1.0f - p, h = 0.5f * r, t = r - e;
+  const float c = __fmul_rn(y, h);
+  const float d = fmaf(y, h, -c) + y * (0.375f * t * t - 0.5f * e);
+  const dd s = dd_fast_two_sum(y, c);
+  return dd_fast_two_sum(s.hi, s.lo + d);
 }
 
 __device__ __forceinline__ dd dd_shfl_xor(unsigned mask, dd v, int lane_mask) {

@@ -68,6 +68,16 @@ __device__ __forceinline__ void load_exps(const KParams &kp, int prim, R &e0, R 
   e1 = ldg_r(rec + 1);
 }
 
+// s += a*b and raw products: dd sums stay unnormalised (dd_acc) until grad_norm
+template <typename R>
+__device__ __forceinline__ void grad_acc(R &s, R a, R b) {
+  if constexpr (std::is_same<R, dd>::value) dd_acc(s, a, b);
+  else s += a * b;
+}
+__device__ __forceinline__ dd grad_sum(dd a, dd b, dd c) {   // 2 alpha sp - sm
+  return dd_fma(dd(2.0f * a.hi, 2.0f * a.lo), dd_norm(b), -dd_norm(c));
+}
+
 // T == 1: one lane per quartet, every table in registers, compile-time indices
 template <int LA, int LB, int LC, int LD, typename R>
 __device__ __forceinline__ void grad_t1(const KParams &kp, const QGeom<R> &g, const R (&gam)[QC<LA, LB, LC, LD>::NABCD],
@@ -96,6 +106,44 @@ __device__ __forceinline__ void grad_t1(const KParams &kp, const QGeom<R> &g, co
     for (int c = 0; c < 3; ++c)
 #pragma unroll
       for (int d = 0; d < 3; ++d) sp[c][d] = sm[c][d] = (R)0;
+    if constexpr (std::is_same<R, dd>::value) {
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        const RootDD c(s, u[r]);
+        dd I[3][SZ];
+        rys_2d_dd<LA + 1, LB + 1, LC + 1, LD, true>(dd(1.0f), dd_fma(-c.tq, s.pqx, s.pax), dd_fma(c.tp, s.pqx, s.qcx),
+                                                    c.b00, c.b10, c.b01, g.ABx, g.CDx, I[0]);
+        rys_2d_dd<LA + 1, LB + 1, LC + 1, LD, true>(dd(1.0f), dd_fma(-c.tq, s.pqy, s.pay), dd_fma(c.tp, s.pqy, s.qcy),
+                                                    c.b00, c.b10, c.b01, g.ABy, g.CDy, I[1]);
+        rys_2d_dd<LA + 1, LB + 1, LC + 1, LD, false>(s.pref * wr[r], dd_fma(-c.tq, s.pqz, s.paz),
+                                                     dd_fma(c.tp, s.pqz, s.qcz), c.b00, c.b10, c.b01, g.ABz, g.CDz,
+                                                     I[2]);
+#pragma unroll
+        for (int o = 0; o < Q::NABCD; ++o) {
+          const dd ix = I[0][G::eoff(o, 0)], iy = I[1][G::eoff(o, 1)], iz = gam[o] * I[2][G::eoff(o, 2)];
+          const dd wd[3] = {G::eoff(o, 1) ? iy * iz : iz, G::eoff(o, 0) ? ix * iz : iz,
+                            gam[o] * (G::eoff(o, 0) == 0 ? iy : G::eoff(o, 1) == 0 ? ix : ix * iy)};
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            const int e = G::eoff(o, d);
+            const int ea = cart_e(LA, Q::ca(o), d), eb = cart_e(LB, Q::cb(o), d), ec = cart_e(LC, Q::cc(o), d);
+            dd_acc(sp[0][d], wd[d], I[d][e + G::SA]);
+            dd_acc(sp[1][d], wd[d], I[d][e + G::SB]);
+            dd_acc(sp[2][d], wd[d], I[d][e + G::SC]);
+            if (ea) dd_acc(sm[0][d], dd_times(ea, wd[d]), I[d][e - G::SA]);
+            if (eb) dd_acc(sm[1][d], dd_times(eb, wd[d]), I[d][e - G::SB]);
+            if (ec) dd_acc(sm[2][d], dd_times(ec, wd[d]), I[d][e - G::SC]);
+          }
+        }
+      }
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        gA[d] += grad_sum(al, sp[0][d], sm[0][d]);
+        gB[d] += grad_sum(be, sp[1][d], sm[1][d]);
+        gC[d] += grad_sum(ga, sp[2][d], sm[2][d]);
+      }
+      continue;
+    } else {
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
       const R uu = u[r];
@@ -132,6 +180,7 @@ __device__ __forceinline__ void grad_t1(const KParams &kp, const QGeom<R> &g, co
       gA[d] += (R)2 * al * sp[0][d] - sm[0][d];
       gB[d] += (R)2 * be * sp[1][d] - sm[1][d];
       gC[d] += (R)2 * ga * sp[2][d] - sm[2][d];
+    }
     }
   }
 }
@@ -262,18 +311,24 @@ __device__ __forceinline__ void grad_quartet(const KParams &kp, const ClassWork 
     for (int task = t; task < 3 * NR; task += T) {
       const int r = task % NR, d = task / NR;
       const R uu = tab[GP::ROOTS + r], ww = tab[GP::ROOTS + NR + r];
-      const R b00 = (R)0.5 * s.r2 * uu;
-      const R b10 = s.i2p * ((R)1 - s.aq * uu);
-      const R b01 = s.i2q * ((R)1 - s.ap * uu);
-      const R tq = s.aq * uu, tp = s.ap * uu;
       const R pa = d == 0 ? s.pax : d == 1 ? s.pay : s.paz;
       const R qc = d == 0 ? s.qcx : d == 1 ? s.qcy : s.qcz;
       const R pq = d == 0 ? s.pqx : d == 1 ? s.pqy : s.pqz;
       const R ab = d == 0 ? g.ABx : d == 1 ? g.ABy : g.ABz;
       const R cd = d == 0 ? g.CDx : d == 1 ? g.CDy : g.CDz;
       const R g0 = d == 2 ? s.pref * ww : (R)1;
-      rys_2d<LA + 1, LB + 1, LC + 1, LD, R>(g0, pa - tq * pq, qc + tp * pq, b00, b10, b01, ab, cd,
-                                            tab + (d * NR + r) * SZ);
+      if constexpr (std::is_same<R, dd>::value) {
+        const RootDD c(s, uu);
+        rys_2d_dd<LA + 1, LB + 1, LC + 1, LD, false>(g0, dd_fma(-c.tq, pq, pa), dd_fma(c.tp, pq, qc), c.b00, c.b10, c.b01,
+                                                     ab, cd, tab + (d * NR + r) * SZ);
+      } else {
+        const R b00 = (R)0.5 * s.r2 * uu;
+        const R b10 = s.i2p * ((R)1 - s.aq * uu);
+        const R b01 = s.i2q * ((R)1 - s.ap * uu);
+        const R tq = s.aq * uu, tp = s.ap * uu;
+        rys_2d<LA + 1, LB + 1, LC + 1, LD, R>(g0, pa - tq * pq, qc + tp * pq, b00, b10, b01, ab, cd,
+                                              tab + (d * NR + r) * SZ);
+      }
     }
     __syncwarp(gmask);
     R sp[3][3], sm[3][3];   // [centre A,B,C][direction]: + and - shift sums
@@ -297,12 +352,18 @@ __device__ __forceinline__ void grad_quartet(const KParams &kp, const ClassWork 
           for (int d = 0; d < 3; ++d) {
             const int e = ex[k] >> (6 * d);
             const int ea = e & 3, eb = (e >> 2) & 3, ec = (e >> 4) & 3;
-            sp[0][d] += wd[d] * td[d][G::SA];
-            sp[1][d] += wd[d] * td[d][G::SB];
-            sp[2][d] += wd[d] * td[d][G::SC];
-            if (ea) sm[0][d] += (R)ea * wd[d] * td[d][-G::SA];
-            if (eb) sm[1][d] += (R)eb * wd[d] * td[d][-G::SB];
-            if (ec) sm[2][d] += (R)ec * wd[d] * td[d][-G::SC];
+            grad_acc(sp[0][d], wd[d], td[d][G::SA]);
+            grad_acc(sp[1][d], wd[d], td[d][G::SB]);
+            grad_acc(sp[2][d], wd[d], td[d][G::SC]);
+            if constexpr (std::is_same<R, dd>::value) {
+              if (ea) dd_acc(sm[0][d], dd_times(ea, wd[d]), td[d][-G::SA]);
+              if (eb) dd_acc(sm[1][d], dd_times(eb, wd[d]), td[d][-G::SB]);
+              if (ec) dd_acc(sm[2][d], dd_times(ec, wd[d]), td[d][-G::SC]);
+            } else {
+              if (ea) sm[0][d] += (R)ea * wd[d] * td[d][-G::SA];
+              if (eb) sm[1][d] += (R)eb * wd[d] * td[d][-G::SB];
+              if (ec) sm[2][d] += (R)ec * wd[d] * td[d][-G::SC];
+            }
           }
         }
       }
@@ -310,9 +371,15 @@ __device__ __forceinline__ void grad_quartet(const KParams &kp, const ClassWork 
     __syncwarp(gmask);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      gA[d] += (R)2 * al * sp[0][d] - sm[0][d];
-      gB[d] += (R)2 * be * sp[1][d] - sm[1][d];
-      gC[d] += (R)2 * ga * sp[2][d] - sm[2][d];
+      if constexpr (std::is_same<R, dd>::value) {
+        gA[d] += grad_sum(al, sp[0][d], sm[0][d]);
+        gB[d] += grad_sum(be, sp[1][d], sm[1][d]);
+        gC[d] += grad_sum(ga, sp[2][d], sm[2][d]);
+      } else {
+        gA[d] += (R)2 * al * sp[0][d] - sm[0][d];
+        gB[d] += (R)2 * be * sp[1][d] - sm[1][d];
+        gC[d] += (R)2 * ga * sp[2][d] - sm[2][d];
+      }
     }
   }
   }

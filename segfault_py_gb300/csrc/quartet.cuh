@@ -254,31 +254,38 @@ __device__ __forceinline__ void rys_roots_all_f32(const KParams &kp, float x, fl
   for (int i = 0; i < N; ++i) rys_row_f32(base + i * kTab32Row, s, u[i], w[i]);
 }
 
-// dd: the FP64 table's coefficients as dd rows: per n-root block, interval
-// j, root r, the (D+1) coefficients from k = D down to 0, each one 16-byte
-// (u_hi, u_lo, w_hi, w_lo); Horner in dd
-// The leading kDDTop coefficients (k = D .. D-kDDTop+1) are summed in plain
-// FP32: over every interval and root their terms add up to less than 5e-8 of
-// |c_0| (Chebyshev-fitted rows decay geometrically), so FP32 rounding there
-// stays below 1e-14 relative; the remaining rows run in dd.
-constexpr int kDDTop = 4;
+// dd: a row of the fine table as float pairs (sf_internal.h): the kDDTop
+// leading coefficients in plain FP32, the first double-float step from an FP32
+// value, the last one with |c_0| above everything that is added to it
+// (FastTwoSum), the others in full.  About 135 FP32 instructions per root and
+// weight instead of 250 for the degree-11 rows on unit intervals.
 __device__ __forceinline__ void rys_row_dd(const float4 *row, dd s, dd &u, dd &w) {
-  const float4 top = __ldg(row);
-  float uf = top.x, wf = top.z;
+  static_assert(kDDTop == 3, "row layout");
+  const float4 t0 = __ldg(row), t1 = __ldg(row + 1);
+  const float uf = fmaf(fmaf(t0.x, s.hi, t0.z), s.hi, t1.x);
+  const float wf = fmaf(fmaf(t0.y, s.hi, t0.w), s.hi, t1.y);
+  constexpr int K = kTabDegF - kDDTop;   // first double-float step
+  const float4 *r = row + 2;
+  const float4 ck = __ldg(r);
+  u = dd_fma(uf, s, dd(ck.x, ck.y));
+  w = dd_fma(wf, s, dd(ck.z, ck.w));
 #pragma unroll
-  for (int k = 1; k < kDDTop; ++k) {
-    const float4 c = __ldg(row + k);
-    uf = fmaf(uf, s.hi, c.x);
-    wf = fmaf(wf, s.hi, c.z);
-  }
-  u = dd(uf);
-  w = dd(wf);
-#pragma unroll
-  for (int k = kDDTop; k <= kTabDeg64; ++k) {
-    const float4 c = __ldg(row + k);
+  for (int k = 1; k < K; ++k) {
+    const float4 c = __ldg(r + k);
     u = dd_fma(u, s, dd(c.x, c.y));
     w = dd_fma(w, s, dd(c.z, c.w));
   }
+  const float4 c0 = __ldg(r + K);
+  u = dd_fma_big(u, s, dd(c0.x, c0.y));
+  w = dd_fma_big(w, s, dd(c0.z, c0.w));
+}
+
+// interval and position of x: j = floor(8 x), s = 16 x - (2 j + 1)
+__device__ __forceinline__ int rys_interval_dd(dd x, dd &s) {
+  const int j = (int)(x.hi * (float)kTabHF);
+  const dd t = dd_two_sum(__fmul_rn(x.hi, (float)(2 * kTabHF)), -(float)(2 * j + 1));
+  s = dd_fast_two_sum(t.hi, fmaf(x.lo, (float)(2 * kTabHF), t.lo));
+  return j;
 }
 
 template <int N>
@@ -292,11 +299,11 @@ __device__ __forceinline__ void rys_roots_all_dd(const KParams &kp, dd x, dd (&u
     }
     return;
   }
-  const int j = (int)x.hi;
-  const dd s = (x - dd((float)j)) * 2.0f - dd(1.0f);
-  const float4 *base = kp.tabdd + rys_tabdd_offset(N) + j * N * (kTabDeg64 + 1);
+  dd s;
+  const int j = rys_interval_dd(x, s);
+  const float4 *base = kp.tabdd + rys_tabdd_offset(N) + j * N * kTabDDRow;
 #pragma unroll
-  for (int i = 0; i < N; ++i) rys_row_dd(base + i * (kTabDeg64 + 1), s, u[i], w[i]);
+  for (int i = 0; i < N; ++i) rys_row_dd(base + i * kTabDDRow, s, u[i], w[i]);
 }
 
 // all n roots (u = t^2) and weights at x.  FP64: coefficient row k of an
@@ -385,9 +392,9 @@ __device__ __forceinline__ void rys_root_one(const KParams &kp, R x, int r, R &u
       w = kp.asymdd_w[N][r] * dd_rsqrt(x);
       return;
     }
-    const int j = (int)x.hi;
-    const dd s = (x - dd((float)j)) * 2.0f - dd(1.0f);
-    rys_row_dd(kp.tabdd + rys_tabdd_offset(N) + (j * N + r) * (kTabDeg64 + 1), s, u, w);
+    dd s;
+    const int j = rys_interval_dd(x, s);
+    rys_row_dd(kp.tabdd + rys_tabdd_offset(N) + (j * N + r) * kTabDDRow, s, u, w);
   } else {
     rys_root_one_f64<N>(kp, x, r, u, w);
   }
@@ -435,10 +442,80 @@ struct QC {
   }
 };
 
+// The recurrences of rys_2d in double-float: every product that is added to
+// something is one dd_fma (15 instructions instead of 18 for a product and a
+// sum with their own renormalisations), and where g0 is one (the x and y
+// tables; UNIT) nothing is multiplied by it.
+template <int LA, int LB, int LC, int LD, bool UNIT>
+__device__ __forceinline__ void rys_2d_dd(dd g0, dd c00, dd c00p, dd b00, dd b10, dd b01, dd ab, dd cd,
+                                          dd *__restrict__ I) {
+  constexpr int LAB = LA + LB, LCD = LC + LD;
+  dd G[LAB + 1][LCD + 1];
+  // x * G[i][k], and x * G[i][k] + y
+  auto mul = [&](dd x, int i, int k) { return UNIT && i == 0 && k == 0 ? x : x * G[i][k]; };
+  auto mad = [&](dd x, int i, int k, dd y) { return UNIT && i == 0 && k == 0 ? x + y : dd_fma(x, G[i][k], y); };
+  G[0][0] = g0;
+  if (LAB > 0) G[1][0] = mul(c00, 0, 0);
+#pragma unroll
+  for (int i = 1; i < LAB; ++i) G[i + 1][0] = dd_fma(c00, G[i][0], mul(dd_times(i, b10), i - 1, 0));
+  if (LCD > 0) {
+    G[0][1] = mul(c00p, 0, 0);
+#pragma unroll
+    for (int i = 1; i <= LAB; ++i) G[i][1] = dd_fma(c00p, G[i][0], mul(dd_times(i, b00), i - 1, 0));
+#pragma unroll
+    for (int k = 1; k < LCD; ++k) {
+      G[0][k + 1] = dd_fma(c00p, G[0][k], mul(dd_times(k, b01), 0, k - 1));
+#pragma unroll
+      for (int i = 1; i <= LAB; ++i)
+        G[i][k + 1] = dd_fma(c00p, G[i][k], dd_fma(dd_times(k, b01), G[i][k - 1], mul(dd_times(i, b00), i - 1, k)));
+    }
+  }
+  dd H[LA + 1][LB + 1][LCD + 1];
+#pragma unroll
+  for (int k = 0; k <= LCD; ++k) {
+    dd t[LAB + 1];
+#pragma unroll
+    for (int i = 0; i <= LAB; ++i) t[i] = G[i][k];
+#pragma unroll
+    for (int ia = 0; ia <= LA; ++ia) H[ia][0][k] = t[ia];
+#pragma unroll
+    for (int ib = 1; ib <= LB; ++ib) {
+#pragma unroll
+      for (int i = 0; i <= LAB - ib; ++i)
+        t[i] = ib == 1 && i == 0 ? mad(ab, 0, k, t[1]) : dd_fma(ab, t[i], t[i + 1]);
+#pragma unroll
+      for (int ia = 0; ia <= LA; ++ia) H[ia][ib][k] = t[ia];
+    }
+  }
+#pragma unroll
+  for (int ia = 0; ia <= LA; ++ia) {
+#pragma unroll
+    for (int ib = 0; ib <= LB; ++ib) {
+      dd t[LCD + 1];
+#pragma unroll
+      for (int k = 0; k <= LCD; ++k) t[k] = H[ia][ib][k];
+#pragma unroll
+      for (int ic = 0; ic <= LC; ++ic) I[((ia * (LB + 1) + ib) * (LC + 1) + ic) * (LD + 1) + 0] = t[ic];
+#pragma unroll
+      for (int id = 1; id <= LD; ++id) {
+#pragma unroll
+        for (int k = 0; k <= LCD - id; ++k)
+          t[k] = ia == 0 && ib == 0 && id == 1 && k == 0 ? mad(cd, 0, 0, t[1]) : dd_fma(cd, t[k], t[k + 1]);
+#pragma unroll
+        for (int ic = 0; ic <= LC; ++ic) I[((ia * (LB + 1) + ib) * (LC + 1) + ic) * (LD + 1) + id] = t[ic];
+      }
+    }
+  }
+}
+
 // Vertical recurrence + horizontal transfer for one root and one direction.
 // Output I[((ia*(LB+1)+ib)*(LC+1)+ic)*(LD+1)+id].
 template <int LA, int LB, int LC, int LD, typename R>
 __device__ __forceinline__ void rys_2d(R g0, R c00, R c00p, R b00, R b10, R b01, R ab, R cd, R *__restrict__ I) {
+  if constexpr (std::is_same<R, dd>::value) {
+    rys_2d_dd<LA, LB, LC, LD, false>(g0, c00, c00p, b00, b10, b01, ab, cd, I);
+    return;
+  } else {
   constexpr int LAB = LA + LB, LCD = LC + LD;
   R G[LAB + 1][LCD + 1];
   G[0][0] = g0;
@@ -492,6 +569,7 @@ __device__ __forceinline__ void rys_2d(R g0, R c00, R c00p, R b00, R b10, R b01,
         for (int ic = 0; ic <= LC; ++ic) I[((ia * (LB + 1) + ib) * (LC + 1) + ic) * (LD + 1) + id] = t[ic];
       }
     }
+  }
   }
 }
 
@@ -614,6 +692,18 @@ __device__ __forceinline__ void load_ket(const KParams &kp, const QGeom<R> &g, i
 template <typename R>
 __device__ __forceinline__ void set_prim_cd(const QGeom<R> &g, const KetRec<R> &k, PQ<R> &s, R p, R px, R py, R pz,
                                             R kab) {
+  if constexpr (std::is_same<R, dd>::value) {
+    s.i2q = k.i2q;
+    s.qcx = k.qx - g.Cx; s.qcy = k.qy - g.Cy; s.qcz = k.qz - g.Cz;
+    s.pqx = px - k.qx; s.pqy = py - k.qy; s.pqz = pz - k.qz;
+    const dd rr = dd_rsqrt(p + k.q);
+    s.r2 = rr * rr;
+    s.aq = k.q * s.r2;
+    s.ap = p * s.r2;
+    s.x = p * s.aq * dd_fma(s.pqz, s.pqz, dd_fma(s.pqy, s.pqy, s.pqx * s.pqx));
+    s.pref = kab * k.kcd * rr;
+    return;
+  } else {
   const R q = k.q, qx = k.qx, qy = k.qy, qz = k.qz, kcd = k.kcd;
   s.i2q = k.i2q;
   s.qcx = qx - g.Cx; s.qcy = qy - g.Cy; s.qcz = qz - g.Cz;
@@ -625,11 +715,18 @@ __device__ __forceinline__ void set_prim_cd(const QGeom<R> &g, const KetRec<R> &
   const R rho = p * s.aq;
   s.x = rho * (s.pqx * s.pqx + s.pqy * s.pqy + s.pqz * s.pqz);
   s.pref = kab * kcd * rr;
+  }
 }
 
 template <typename R>
 __device__ __forceinline__ void load_prim_cd(const KParams &kp, const QGeom<R> &g, int iq, PQ<R> &s, R p, R px, R py,
                                              R pz, R kab) {
+  if constexpr (std::is_same<R, dd>::value) {
+    KetRec<dd> k;
+    load_ket<dd>(kp, g, iq, k);
+    set_prim_cd<dd>(g, k, s, p, px, py, pz, kab);
+    return;
+  } else {
   R q, qx, qy, qz, kcd;
   load_rec<R>(prims_of<R>(kp).rec + (size_t)(g.cd_off + iq) * kPrimRec, q, qx, qy, qz, kcd, s.i2q);
   s.qcx = qx - g.Cx; s.qcy = qy - g.Cy; s.qcz = qz - g.Cz;
@@ -641,7 +738,22 @@ __device__ __forceinline__ void load_prim_cd(const KParams &kp, const QGeom<R> &
   const R rho = p * s.aq;
   s.x = rho * (s.pqx * s.pqx + s.pqy * s.pqy + s.pqz * s.pqz);
   s.pref = kab * kcd * rr;
+  }
 }
+
+// recurrence coefficients of one root u in double-float; tq = a_q u and
+// tp = a_p u lie in [0, 1] and come close to 1 for very different exponents,
+// so the differences 1 - tq, 1 - tp are formed before they are scaled
+struct RootDD {
+  dd b00, b10, b01, tq, tp;
+  __device__ __forceinline__ RootDD(const PQ<dd> &s, dd u) {
+    b00 = dd(0.5f * s.r2.hi, 0.5f * s.r2.lo) * u;
+    tq = s.aq * u;
+    tp = s.ap * u;
+    b10 = s.i2p * dd_one_minus(tq);
+    b01 = s.i2q * dd_one_minus(tp);
+  }
+};
 
 // float -> double without the FP64 pipe: re-pack sign, exponent (rebias
 // 127 -> 1023, i.e. + 896 << 20 in the high word) and mantissa with five
@@ -815,6 +927,30 @@ __device__ __forceinline__ void eval_t1(const KParams &kp, const QGeom<R> &g, R 
     iq = iqn;
     R u[NR], w[NR];
     roots_t1<NR, R>(kp, tab_s, s.x, u, w);
+    if constexpr (std::is_same<R, dd>::value) {
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        const RootDD c(s, u[r]);
+        dd Ix[SZ], Iy[SZ], Iz[SZ];
+        rys_2d_dd<LA, LB, LC, LD, true>(dd(1.0f), dd_fma(-c.tq, s.pqx, s.pax), dd_fma(c.tp, s.pqx, s.qcx), c.b00, c.b10,
+                                        c.b01, g.ABx, g.CDx, Ix);
+        rys_2d_dd<LA, LB, LC, LD, true>(dd(1.0f), dd_fma(-c.tq, s.pqy, s.pay), dd_fma(c.tp, s.pqy, s.qcy), c.b00, c.b10,
+                                        c.b01, g.ABy, g.CDy, Iy);
+        rys_2d_dd<LA, LB, LC, LD, false>(s.pref * w[r], dd_fma(-c.tq, s.pqz, s.paz), dd_fma(c.tp, s.pqz, s.qcz), c.b00,
+                                         c.b10, c.b01, g.ABz, g.CDz, Iz);
+        // Ix[0] = Iy[0] = 1
+#pragma unroll
+        for (int o = 0; o < Q::NABCD; ++o) {
+          const int ox = Q::toff(o, 0), oy = Q::toff(o, 1), oz = Q::toff(o, 2);
+          if (ox == 0 && oy == 0) acc[o] += Iz[oz];
+          else dd_acc(acc[o], ox == 0 ? Iy[oy] : oy == 0 ? Ix[ox] : dd_mul_raw(Ix[ox], Iy[oy]), Iz[oz]);
+        }
+      }
+      // per primitive quartet, so that lo does not grow over a long contraction
+#pragma unroll
+      for (int o = 0; o < Q::NABCD; ++o) acc[o] = dd_norm(acc[o]);
+      continue;
+    }
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
       const R uu = u[r];
@@ -912,24 +1048,36 @@ __device__ __forceinline__ void eval_grp(const KParams &kp, const QGeom<R> &g, R
     for (int task = t; task < 3 * NR; task += T) {
       const int r = task % NR, d = task / NR;
       const R uu = tab[GP::ROOTS + r], ww = tab[GP::ROOTS + NR + r];
-      const R b00 = (R)0.5 * s.r2 * uu;
-      const R b10 = s.i2p * ((R)1 - s.aq * uu);
-      const R b01 = s.i2q * ((R)1 - s.ap * uu);
-      const R tq = s.aq * uu, tp = s.ap * uu;
       const R pa = d == 0 ? s.pax : d == 1 ? s.pay : s.paz;
       const R qc = d == 0 ? s.qcx : d == 1 ? s.qcy : s.qcz;
       const R pq = d == 0 ? s.pqx : d == 1 ? s.pqy : s.pqz;
       const R ab = d == 0 ? g.ABx : d == 1 ? g.ABy : g.ABz;
       const R cd = d == 0 ? g.CDx : d == 1 ? g.CDy : g.CDz;
       const R g0 = d == 2 ? s.pref * ww : (R)1;
+      if constexpr (std::is_same<R, dd>::value) {
+        const RootDD c(s, uu);
+        rys_2d_dd<LA, LB, LC, LD, false>(g0, dd_fma(-c.tq, pq, pa), dd_fma(c.tp, pq, qc), c.b00, c.b10, c.b01, ab, cd,
+                                         tab + (d * NR + r) * SZ);
+        continue;
+      } else {
+      const R b00 = (R)0.5 * s.r2 * uu;
+      const R b10 = s.i2p * ((R)1 - s.aq * uu);
+      const R b01 = s.i2q * ((R)1 - s.ap * uu);
+      const R tq = s.aq * uu, tp = s.ap * uu;
       rys_2d<LA, LB, LC, LD, R>(g0, pa - tq * pq, qc + tp * pq, b00, b10, b01, ab, cd, tab + (d * NR + r) * SZ);
+      }
     }
     __syncwarp(gmask);
 #pragma unroll
     for (int j = 0; j < RPER; ++j) {
       if (t + j * T < GP::ROWS) {
         const int ox = off[j] & 1023, oy = (off[j] >> 10) & 1023, oz = off[j] >> 20;
-        if constexpr (INNER == 1) {
+        if constexpr (std::is_same<R, dd>::value) {
+#pragma unroll
+          for (int r = 0; r < NR; ++r)
+            dd_acc(acc[j], dd_mul_raw(tab[ox + r * SZ], tab[oy + r * SZ]), tab[oz + r * SZ]);
+          acc[j] = dd_norm(acc[j]);
+        } else if constexpr (INNER == 1) {
           R v = (R)0;
 #pragma unroll
           for (int r = 0; r < NR; ++r) v += tab[ox + r * SZ] * tab[oy + r * SZ] * tab[oz + r * SZ];

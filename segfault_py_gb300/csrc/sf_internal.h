@@ -40,12 +40,17 @@ __host__ __device__ constexpr int rys_tab_offset(int n, int deg) {
 }
 __host__ __device__ constexpr int rys_tab_size(int deg) { return rys_tab_offset(kMaxRoots + 1, deg); }
 
-// The Boys functions F_0 .. F_kBoysMax and e^-T on intervals of 1/kTabHF, degree
-// kTabDegF: per function and interval the kTabDegF + 1 coefficients from high to
-// low order.
+// The fine tables: intervals of 1/kTabHF, s = 2 (kTabHF x - j) - 1, degree
+// kTabDegF.  Rys rule in FP64 (the source of the double-float rows below),
+// layout as the unit tables.
 constexpr int kTabHF = 8;
 constexpr int kTabNintF = 64 * kTabHF;
 constexpr int kTabDegF = 7;
+__host__ __device__ constexpr int rys_fine_offset(int n) { return kTabNintF * (kTabDegF + 1) * (n - 1) * n; }
+__host__ __device__ constexpr int rys_fine_size() { return rys_fine_offset(kMaxRoots + 1); }
+
+// Boys functions F_0 .. F_kBoysMax and e^-T on the fine intervals: per function
+// and interval the kTabDegF + 1 coefficients from high to low order.
 constexpr int kBoysMax = 5;
 constexpr int kBoysTab = (kBoysMax + 2) * kTabNintF * (kTabDegF + 1);
 
@@ -58,10 +63,16 @@ constexpr int kTab32Row = 2 * (kTabDeg32 + 1);
 __host__ __device__ constexpr int rys_tab32v_offset(int n) { return kTabNint * kTab32Row * ((n - 1) * n / 2); }
 __host__ __device__ constexpr int rys_tab32v_size() { return rys_tab32v_offset(kMaxRoots + 1); }
 
-// Layout of the double-float copy of the FP64 table (in 16-byte units): per
-// n-root block, interval j, root r, the kTabDeg64+1 coefficients from
-// k = kTabDeg64 down to 0, each (u_hi, u_lo, w_hi, w_lo).
-__host__ __device__ constexpr int rys_tabdd_offset(int n) { return kTabNint * (kTabDeg64 + 1) * ((n - 1) * n / 2); }
+// Layout of the fine Rys table in double-float (in 16-byte units): per n-root
+// block, interval j, root r, one row: the kDDTop leading coefficients as FP32
+// pairs (u_k, w_k), two to a unit, then the others from high to low k as
+// (u_hi, u_lo, w_hi, w_lo).  The terms above s^4 add up to less than 5e-9 of
+// |c_0| over every interval and root, so their FP32 rounding is below 1e-15
+// relative and only five Horner steps need double-float arithmetic (eight of
+// twelve on unit intervals of degree 11).
+constexpr int kDDTop = 3;
+constexpr int kTabDDRow = (kDDTop + 1) / 2 + kTabDegF + 1 - kDDTop;
+__host__ __device__ constexpr int rys_tabdd_offset(int n) { return kTabNintF * kTabDDRow * ((n - 1) * n / 2); }
 __host__ __device__ constexpr int rys_tabdd_size() { return rys_tabdd_offset(kMaxRoots + 1); }
 
 __host__ __device__ constexpr int ncart(int l) { return (l + 1) * (l + 2) / 2; }
@@ -115,6 +126,7 @@ struct RysAsym32 {                      // the same constants rounded to FP32
 
 // host-side: build tables (rys_table.cpp)
 void rys_build_tables(double *tab64, float *tab32, RysAsym *asym);
+void rys_build_fine(double *tab);
 void boys_build_table(double *tab);
 void rys_eval_host(const double *tab64, const float *tab32, const RysAsym &as, int n, double x, int fp32,
                    double *u, double *w);
