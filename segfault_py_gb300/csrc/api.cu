@@ -340,6 +340,7 @@ struct sf_handle {
     int64_t quartets, prims;
     double flops;
     int64_t cost_hi;               // primitive cost of the segment's first quartet (tuning key)
+    double est = 0.0;              // cost estimate (or tuned time) the stream assignment uses
   };
   // autotuned primitive splits S = P*W, keyed by (class, precision, cost_hi)
   std::vector<sf_tune_entry> tune;
@@ -390,6 +391,15 @@ struct sf_handle {
     int covered = 0;                       // run by a persistent tier launch, not by its own
   };
   std::vector<Launch> plan;
+  // the plan as it is issued outside the profiling modes: the launches of one
+  // class, arithmetic and list kind (kept / demoted) as the segments of one
+  // kernel launch
+  struct Group {
+    int kind, cls, stream, demoted;
+    double est;
+    std::vector<ClassWork> w;
+  };
+  std::vector<Group> groups;
   bool plan_counts = false;                // quartet counts of the plan live on the device
   bool plan_grad = false;                  // the last plan was a gradient's
   // launch mode SF_LAUNCH_PERSISTENT: the FP32 register-path lists of a Fock
@@ -749,7 +759,10 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
     std::vector<sf_handle::Slice> sorted;
-    for (int k : order) sorted.push_back(h->slices[k]);
+    for (int k : order) {
+      sorted.push_back(h->slices[k]);
+      sorted.back().est = cost[k];
+    }
     h->slices.swap(sorted);
     std::sort(cost.begin(), cost.end(), std::greater<double>());
     bool has32 = false, hasacc = false;
@@ -945,6 +958,40 @@ int make_plan(sf_handle *h, bool grad, int active) {
   return SF_OK;
 }
 
+// The plan's launches merged for issue: those of one class, arithmetic and
+// list kind become the segments of one kernel launch (at most kMaxSegs, longer
+// plans continue in another), costliest segment first; the merged launches
+// are spread over the side streams as build_work spreads the slices.
+void make_groups(sf_handle *h) {
+  h->groups.clear();
+  bool has32 = false, hasacc = false;
+  for (const auto &L : h->plan) {
+    if (L.covered) continue;
+    const auto &sl = h->slices[L.slice];
+    if (!L.demoted) (L.kind == 1 ? has32 : hasacc) = true;
+    sf_handle::Group *g = nullptr;
+    for (auto &x : h->groups)
+      if (x.cls == sl.cls && x.kind == L.kind && x.demoted == L.demoted && x.w.size() < (size_t)kMaxSegs) g = &x;
+    if (!g) {
+      h->groups.push_back({L.kind, sl.cls, 0, L.demoted, 0.0, {}});
+      g = &h->groups.back();
+    }
+    g->w.push_back(L.w);
+    if (!L.demoted) g->est += sl.est;
+  }
+  for (auto &g : h->groups)
+    std::stable_sort(g.w.begin(), g.w.end(), [](const ClassWork &a, const ClassWork &b) { return a.max_cost > b.max_cost; });
+  std::stable_sort(h->groups.begin(), h->groups.end(),
+                   [](const sf_handle::Group &a, const sf_handle::Group &b) { return a.est > b.est; });
+  const bool mixed = has32 && hasacc;
+  std::vector<double> ca, cf;
+  for (const auto &g : h->groups) (mixed && g.kind != 1 ? ca : cf).push_back(g.est);
+  const std::vector<int> sa = lpt_streams(ca, 0, sf_handle::kHiStreams);
+  const std::vector<int> sf = lpt_streams(cf, mixed ? sf_handle::kHiStreams : 0, sf_handle::kSideStreams);
+  size_t ia = 0, ifp = 0;
+  for (auto &g : h->groups) g.stream = mixed && g.kind != 1 ? sa[ia++] : sf[ifp++];
+}
+
 // Run fn(k, stream) for every slice k on its side stream (forked from st,
 // joined back into st).
 template <typename F>
@@ -968,38 +1015,39 @@ int fan_out_list(sf_handle *h, cudaStream_t st, const std::vector<int> &stream_o
 // one launch of the current quartet lists, in its kind's arithmetic
 cudaError_t launch_slice(sf_handle *h, const sf_handle::Slice &s, const ClassWork &w, const double *D,
                          const float *D32, double *Jh, double *Kh, cudaStream_t st) {
-  if (s.prec == 0) return launch_jk_f64(s.cls, h->kp, w, D, Jh, Kh, st);
-  if (s.prec == 1) return launch_jk_f32(s.cls, h->kp, w, D32, Jh, Kh, st);
-  return launch_jk_dd(s.cls, h->kp, w, reinterpret_cast<const dd *>(h->d_Ddd.p), Jh, Kh, st);
+  if (s.prec == 0) return launch_jk_f64(s.cls, h->kp, &w, 1, D, Jh, Kh, st);
+  if (s.prec == 1) return launch_jk_f32(s.cls, h->kp, &w, 1, D32, Jh, Kh, st);
+  return launch_jk_dd(s.cls, h->kp, &w, 1, reinterpret_cast<const dd *>(h->d_Ddd.p), Jh, Kh, st);
 }
 
 int profiling_events(sf_handle *h, cudaStream_t st);
 
-// one launch of the plan: J/K digestion (Jh, Kh) or gradient (g) kernels in
-// the launch's arithmetic
-cudaError_t launch_one(sf_handle *h, const sf_handle::Launch &L, bool grad, const double *D, const float *D32,
-                       double *Jh, double *Kh, double *g, cudaStream_t st) {
-  const int cls = h->slices[L.slice].cls;
+// one launch of the plan, nw segments of class cls: J/K digestion (Jh, Kh) or
+// gradient (g) kernels in the launch's arithmetic
+cudaError_t launch_one(sf_handle *h, int cls, int kind, const ClassWork *w, int nw, bool grad, const double *D,
+                       const float *D32, double *Jh, double *Kh, double *g, cudaStream_t st) {
   const dd *Ddd = reinterpret_cast<const dd *>(h->d_Ddd.p);
   if (grad) {
-    if (L.kind == 0) return launch_grad_f64(cls, h->kp, L.w, D, g, st);
-    if (L.kind == 1) return launch_grad_f32(cls, h->kp, L.w, D32, g, st);
-    return launch_grad_dd(cls, h->kp, L.w, Ddd, g, st);
+    if (kind == 0) return launch_grad_f64(cls, h->kp, w, nw, D, g, st);
+    if (kind == 1) return launch_grad_f32(cls, h->kp, w, nw, D32, g, st);
+    return launch_grad_dd(cls, h->kp, w, nw, Ddd, g, st);
   }
-  if (L.kind == 0) return launch_jk_f64(cls, h->kp, L.w, D, Jh, Kh, st);
-  if (L.kind == 1) return launch_jk_f32(cls, h->kp, L.w, D32, Jh, Kh, st);
-  return launch_jk_dd(cls, h->kp, L.w, Ddd, Jh, Kh, st);
+  if (kind == 0) return launch_jk_f64(cls, h->kp, w, nw, D, Jh, Kh, st);
+  if (kind == 1) return launch_jk_f32(cls, h->kp, w, nw, D32, Jh, Kh, st);
+  return launch_jk_dd(cls, h->kp, w, nw, Ddd, Jh, Kh, st);
 }
 
-// Run every launch of the plan on its side stream (forked from st, joined
-// back into st); profiling 1: events bracket each launch on its own stream;
+// Run the plan on the side streams (forked from st, joined back into st): the
+// merged launches (make_groups), or in the profiling modes every launch by
+// itself; profiling 1: events bracket each launch on its own stream;
 // profiling 2: the launches are serialised on st, each between two events.
 int run_plan(sf_handle *h, bool grad, const double *D, const float *D32, double *Jh, double *Kh, double *g,
              cudaStream_t st, int profiling, int *launches) {
   if (profiling == 2) {
     for (size_t k = 0; k < h->plan.size(); ++k) {
       SF_CK(cudaEventRecord(h->ev[2 * k], st));
-      SF_CK(launch_one(h, h->plan[k], grad, D, D32, Jh, Kh, g, st));
+      const auto &L = h->plan[k];
+      SF_CK(launch_one(h, h->slices[L.slice].cls, L.kind, &L.w, 1, grad, D, D32, Jh, Kh, g, st));
       SF_CK(cudaEventRecord(h->ev[2 * k + 1], st));
       if (launches) ++*launches;
     }
@@ -1007,18 +1055,24 @@ int run_plan(sf_handle *h, bool grad, const double *D, const float *D32, double 
   }
   SF_CK(cudaEventRecord(h->fork_ev, st));
   bool used[sf_handle::kSideStreams] = {false};
-  for (const auto &L : h->plan)
-    if (!L.covered) used[L.stream] = true;
+  if (profiling)
+    for (const auto &L : h->plan) used[L.stream] = true;
+  else
+    for (const auto &G : h->groups) used[G.stream] = true;
   for (const auto &T : h->pplan) used[T.stream] = true;
   for (int j = 0; j < sf_handle::kSideStreams; ++j)
     if (used[j]) SF_CK(cudaStreamWaitEvent(h->side[j], h->fork_ev, 0));
-  for (size_t k = 0; k < h->plan.size(); ++k) {
+  for (size_t k = 0; profiling && k < h->plan.size(); ++k) {
     const auto &L = h->plan[k];
-    if (L.covered) continue;
     cudaStream_t ss = h->side[L.stream];
-    if (profiling) SF_CK(cudaEventRecord(h->ev[2 * k], ss));
-    SF_CK(launch_one(h, L, grad, D, D32, Jh, Kh, g, ss));
-    if (profiling) SF_CK(cudaEventRecord(h->ev[2 * k + 1], ss));
+    SF_CK(cudaEventRecord(h->ev[2 * k], ss));
+    SF_CK(launch_one(h, h->slices[L.slice].cls, L.kind, &L.w, 1, grad, D, D32, Jh, Kh, g, ss));
+    SF_CK(cudaEventRecord(h->ev[2 * k + 1], ss));
+    if (launches) ++*launches;
+  }
+  for (size_t k = 0; !profiling && k < h->groups.size(); ++k) {
+    const auto &G = h->groups[k];
+    SF_CK(launch_one(h, G.cls, G.kind, G.w.data(), (int)G.w.size(), grad, D, D32, Jh, Kh, g, h->side[G.stream]));
     if (launches) ++*launches;
   }
   // the persistent tier launches last: they take the SM slots the others leave
@@ -1044,6 +1098,7 @@ int run_call(sf_handle *h, bool grad, const double *D, const float *D32, double 
   if (rc) return rc;
   rc = make_plan(h, grad, active);
   if (rc) return rc;
+  if (!profiling) make_groups(h);
   if (profiling) {
     rc = profiling_events(h, st);
     if (rc) return rc;

@@ -186,7 +186,8 @@ __device__ __forceinline__ void grad_t1(const KParams &kp, const QGeom<R> &g, co
 }
 
 template <int LA, int LB, int LC, int LD, typename R, int T, typename A>
-__device__ __forceinline__ void grad_quartet(const KParams &kp, const ClassWork &w, const R *__restrict__ D, A *grad);
+__device__ __forceinline__ void grad_quartet(const KParams &kp, const ClassWork &w, int64_t cta,
+                                             const R *__restrict__ D, A *grad);
 
 // Gradient contributions of a CTA are summed in shared memory (3 slots per
 // atom) and written with one atomic per slot at the end: all quartets add
@@ -207,7 +208,11 @@ template <typename V>
 __device__ __forceinline__ double acc_value(V v, double) { return to_f64(v); }
 
 template <int LA, int LB, int LC, int LD, typename R, int T>
-__global__ void __launch_bounds__(kBlock) grad_kernel(KParams kp, ClassWork w, const R *__restrict__ D, double *grad) {
+__global__ void __launch_bounds__(kBlock) grad_kernel(KParams kp, const __grid_constant__ ClassMulti m,
+                                                      const R *__restrict__ D, double *grad) {
+  const int sg = m.find(blockIdx.x);
+  const ClassWork w = m.seg[sg];
+  const int64_t cta = (int)blockIdx.x - m.cta0[sg];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   using GP0 = GGrp<LA, LB, LC, LD, R, T>;
   using A = GradAcc<R>;
@@ -215,16 +220,16 @@ __global__ void __launch_bounds__(kBlock) grad_kernel(KParams kp, ClassWork w, c
   A *sgrad = reinterpret_cast<A *>(smem_raw + (T == 1 ? 0 : (size_t)(kBlock / T) * GP0::BUFN * sizeof(R)));
   const int TP0 = T * w.psplit;
   const int64_t nq = work_count(w);
-  const int64_t qfirst = ((int64_t)blockIdx.x * (kBlock / TP0)) / w.wsplit;
+  const int64_t qfirst = (cta * (kBlock / TP0)) / w.wsplit;
   if (qfirst >= nq) return;   // the whole CTA is past the end of the list
   if (cta_sum) {
     for (int i = threadIdx.x; i < 3 * kp.natom; i += blockDim.x) sgrad[i] = (A)0;
     __syncthreads();
   }
-  const int64_t q0 = ((int64_t)blockIdx.x * (kBlock / TP0) + threadIdx.x / TP0) / w.wsplit;
+  const int64_t q0 = (cta * (kBlock / TP0) + threadIdx.x / TP0) / w.wsplit;
   if (q0 < nq) {
-    if (cta_sum) grad_quartet<LA, LB, LC, LD, R, T, A>(kp, w, D, sgrad);
-    else grad_quartet<LA, LB, LC, LD, R, T, double>(kp, w, D, grad);
+    if (cta_sum) grad_quartet<LA, LB, LC, LD, R, T, A>(kp, w, cta, D, sgrad);
+    else grad_quartet<LA, LB, LC, LD, R, T, double>(kp, w, cta, D, grad);
   }
   if (cta_sum) {
     __syncthreads();
@@ -234,8 +239,8 @@ __global__ void __launch_bounds__(kBlock) grad_kernel(KParams kp, ClassWork w, c
 }
 
 template <int LA, int LB, int LC, int LD, typename R, int T, typename A>
-__device__ __forceinline__ void grad_quartet(const KParams &kp, const ClassWork &w, const R *__restrict__ D,
-                                             A *grad) {
+__device__ __forceinline__ void grad_quartet(const KParams &kp, const ClassWork &w, int64_t cta,
+                                             const R *__restrict__ D, A *grad) {
   using Q = QC<LA, LB, LC, LD>;
   using G = QG<LA, LB, LC, LD>;
   using GP = GGrp<LA, LB, LC, LD, R, T>;
@@ -243,7 +248,7 @@ __device__ __forceinline__ void grad_quartet(const KParams &kp, const ClassWork 
   const int P = w.psplit, W = w.wsplit;
   const int TP = T * P;
   const int grp = threadIdx.x / TP, t = threadIdx.x % T;
-  const int64_t gid = (int64_t)blockIdx.x * (kBlock / TP) + grp;
+  const int64_t gid = cta * (kBlock / TP) + grp;
   const int64_t q = gid / W;
   const int pl = (threadIdx.x / T) % P;
   const int sub = (int)(gid - q * W) * P + pl;   // primitive sub-group of the W*P
@@ -432,6 +437,14 @@ inline ClassWork grad_work(const ClassWork &w, int T, int nsm) {
   w2.psplit = P;
   w2.wsplit = S / P < kMaxWsplit ? S / P : kMaxWsplit;
   return w2;
+}
+
+// the segments of one gradient launch
+inline bool grad_segments(ClassMulti &m, const ClassWork *w, int nw, int T, int nsm) {
+  m.n = 0;
+  for (int k = 0; k < nw; ++k)
+    if (w[k].n > 0 && !add_segment(m, grad_work(w[k], T, nsm), T)) return false;
+  return true;
 }
 
 template <int LA, int LB, int LC, int LD, typename R>

@@ -12,25 +12,25 @@
 namespace sf {
 
 template <int LA, int LB, int LC, int LD>
-static cudaError_t run_grad_dd(const KParams &kp, const ClassWork &w, const dd *D, double *grad, cudaStream_t st) {
+static cudaError_t run_grad_dd(const KParams &kp, const ClassWork *w, int nw, const dd *D, double *grad, cudaStream_t st) {
   constexpr int T = tgrad(QC<LA, LB, LC, LD>::NABCD);
-  if (w.n <= 0) return cudaSuccess;
-  const ClassWork w2 = grad_work(w, T, kp.nsm);
-  const int G = kBlock / (T * w2.psplit);
+  ClassMulti m;
+  if (!grad_segments(m, w, nw, T, kp.nsm)) return cudaErrorInvalidValue;
+  if (m.n == 0) return cudaSuccess;
   constexpr size_t smem = grad_smem<LA, LB, LC, LD, dd>();
-  grad_kernel<LA, LB, LC, LD, dd, T><<<(unsigned)((w.n * w2.wsplit + G - 1) / G), kBlock, smem, st>>>(kp, w2, D, grad);
+  grad_kernel<LA, LB, LC, LD, dd, T><<<(unsigned)m.cta0[m.n], kBlock, smem, st>>>(kp, m, D, grad);
   return cudaGetLastError();
 }
 
 #define SF_DD_JOIN2(a, b) a##b
 #define SF_DD_JOIN(a, b) SF_DD_JOIN2(a, b)
 
-cudaError_t SF_DD_JOIN(launch_grad_dd_part, SF_DD_PART)(int cls, const KParams &kp, const ClassWork &w, const dd *D,
+cudaError_t SF_DD_JOIN(launch_grad_dd_part, SF_DD_PART)(int cls, const KParams &kp, const ClassWork *w, int nw, const dd *D,
                                                          double *grad, cudaStream_t st) {
   switch (cls) {
 #define SF_CASE(id, la, lb, lc, ld, t64, t32) \
   case id:                                    \
-    if constexpr (id % 4 == SF_DD_PART) return run_grad_dd<la, lb, lc, ld>(kp, w, D, grad, st); \
+    if constexpr (id % 4 == SF_DD_PART) return run_grad_dd<la, lb, lc, ld>(kp, w, nw, D, grad, st); \
     else return cudaErrorInvalidValue;
     SF_CLASS_LIST(SF_CASE)
 #undef SF_CASE

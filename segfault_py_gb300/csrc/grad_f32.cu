@@ -8,21 +8,21 @@
 namespace sf {
 
 template <int LA, int LB, int LC, int LD>
-static cudaError_t run_grad32(const KParams &kp, const ClassWork &w, const float *D, double *grad, cudaStream_t st) {
+static cudaError_t run_grad32(const KParams &kp, const ClassWork *w, int nw, const float *D, double *grad, cudaStream_t st) {
   constexpr int T = tgrad_r<float>(QC<LA, LB, LC, LD>::NABCD);
-  if (w.n <= 0) return cudaSuccess;
-  const ClassWork w2 = grad_work(w, T, kp.nsm);
-  const int G = kBlock / (T * w2.psplit);
+  ClassMulti m;
+  if (!grad_segments(m, w, nw, T, kp.nsm)) return cudaErrorInvalidValue;
+  if (m.n == 0) return cudaSuccess;
   constexpr size_t smem = grad_smem<LA, LB, LC, LD, float>();
-  grad_kernel<LA, LB, LC, LD, float, T><<<(unsigned)((w.n * w2.wsplit + G - 1) / G), kBlock, smem, st>>>(kp, w2, D, grad);
+  grad_kernel<LA, LB, LC, LD, float, T><<<(unsigned)m.cta0[m.n], kBlock, smem, st>>>(kp, m, D, grad);
   return cudaGetLastError();
 }
 
-cudaError_t launch_grad_f32(int cls, const KParams &kp, const ClassWork &w, const float *D, double *grad,
+cudaError_t launch_grad_f32(int cls, const KParams &kp, const ClassWork *w, int nw, const float *D, double *grad,
                             cudaStream_t st) {
   switch (cls) {
 #define SF_CASE(id, la, lb, lc, ld, t64, t32) \
-  case id: return run_grad32<la, lb, lc, ld>(kp, w, D, grad, st);
+  case id: return run_grad32<la, lb, lc, ld>(kp, w, nw, D, grad, st);
     SF_CLASS_LIST(SF_CASE)
 #undef SF_CASE
     default: return cudaErrorInvalidValue;

@@ -8,24 +8,23 @@
 namespace sf {
 
 template <int LA, int LB, int LC, int LD, int T>
-static cudaError_t run_jk_dd_wide(const KParams &kp, const ClassWork &w, const dd *D, double *Jh, double *Kh,
+static cudaError_t run_jk_dd_wide(const KParams &kp, const ClassWork *w, int nw, const dd *D, double *Jh, double *Kh,
                                   cudaStream_t st) {
-  const int64_t n = w.n;
-  if (n <= 0) return cudaSuccess;
-  const int P = w.psplit < 1 ? 1 : w.psplit, W = w.wsplit < 1 ? 1 : w.wsplit;
-  if (T * P > 32 || (P & (P - 1)) || W > kMaxWsplit) return cudaErrorInvalidValue;
-  const int G = kBlock / (T * P);
+  ClassMulti m;
+  m.n = 0;
+  for (int k = 0; k < nw; ++k)
+    if (w[k].n > 0 && !add_segment(m, w[k], T)) return cudaErrorInvalidValue;
+  if (m.n == 0) return cudaSuccess;
   constexpr size_t smem = grp_smem<LA, LB, LC, LD, dd, T>();
-  const int64_t grid = (n * W + G - 1) / G;
-  jk_kernel<LA, LB, LC, LD, dd, T><<<(unsigned)grid, kBlock, smem, st>>>(kp, w, D, Jh, Kh);
+  jk_kernel<LA, LB, LC, LD, dd, T><<<(unsigned)m.cta0[m.n], kBlock, smem, st>>>(kp, m, D, Jh, Kh);
   return cudaGetLastError();
 }
 
-cudaError_t launch_jk_dd_wide(int cls, const KParams &kp, const ClassWork &w, const dd *D, double *Jh, double *Kh,
+cudaError_t launch_jk_dd_wide(int cls, const KParams &kp, const ClassWork *w, int nw, const dd *D, double *Jh, double *Kh,
                               cudaStream_t st) {
   switch (cls) {
 #define SF_CASE(id, la, lb, lc, ld, t64, t32) \
-  case id: return run_jk_dd_wide<la, lb, lc, ld, tdd_wide(la, lb, lc, ld, t64)>(kp, w, D, Jh, Kh, st);
+  case id: return run_jk_dd_wide<la, lb, lc, ld, tdd_wide(la, lb, lc, ld, t64)>(kp, w, nw, D, Jh, Kh, st);
     SF_CLASS_LIST(SF_CASE)
 #undef SF_CASE
     default: return cudaErrorInvalidValue;

@@ -7,29 +7,27 @@
 namespace sf {
 
 template <int LA, int LB, int LC, int LD, int T>
-static cudaError_t run_jk32(const KParams &kp, const ClassWork &w, const float *D, double *Jh, double *Kh,
+static cudaError_t run_jk32(const KParams &kp, const ClassWork *w, int nw, const float *D, double *Jh, double *Kh,
                             cudaStream_t st) {
-  const int64_t n = w.n;
-  if (n <= 0) return cudaSuccess;
-  const int P = w.psplit < 1 ? 1 : w.psplit, W = w.wsplit < 1 ? 1 : w.wsplit;
-  if (T * P > 32 || (P & (P - 1)) || W > kMaxWsplit) return cudaErrorInvalidValue;
-  const int G = kBlock / (T * P);
+  // T == 1: Rys table block in shared memory, grid-stride over each list
+  const int64_t cap = T == 1 ? (int64_t)std::max(kp.nsm, 1) * 16 : 0;
+  ClassMulti m;
+  m.n = 0;
+  for (int k = 0; k < nw; ++k)
+    if (w[k].n > 0 && !add_segment(m, w[k], T, cap)) return cudaErrorInvalidValue;
+  if (m.n == 0) return cudaSuccess;
   auto kern = jk_kernel<LA, LB, LC, LD, float, T>;
-  int64_t grid = (n * W + G - 1) / G;
   size_t smem = grp_smem<LA, LB, LC, LD, float, T>();
-  if (T == 1) {   // Rys table block in shared memory, grid-stride over the list
-    smem = (size_t)kTabNint * QC<LA, LB, LC, LD>::NR * kTab32Row * sizeof(float);
-    grid = std::min<int64_t>(grid, (int64_t)std::max(kp.nsm, 1) * 16);
-  }
-  kern<<<(unsigned)grid, kBlock, smem, st>>>(kp, w, D, Jh, Kh);
+  if (T == 1) smem = (size_t)kTabNint * QC<LA, LB, LC, LD>::NR * kTab32Row * sizeof(float);
+  kern<<<(unsigned)m.cta0[m.n], kBlock, smem, st>>>(kp, m, D, Jh, Kh);
   return cudaGetLastError();
 }
 
-cudaError_t launch_jk_f32(int cls, const KParams &kp, const ClassWork &w, const float *D, double *Jh, double *Kh,
+cudaError_t launch_jk_f32(int cls, const KParams &kp, const ClassWork *w, int nw, const float *D, double *Jh, double *Kh,
                           cudaStream_t st) {
   switch (cls) {
 #define SF_CASE(id, la, lb, lc, ld, t64, t32) \
-  case id: return run_jk32<la, lb, lc, ld, t32>(kp, w, D, Jh, Kh, st);
+  case id: return run_jk32<la, lb, lc, ld, t32>(kp, w, nw, D, Jh, Kh, st);
     SF_CLASS_LIST(SF_CASE)
 #undef SF_CASE
     default: return cudaErrorInvalidValue;

@@ -3,15 +3,15 @@
 #include "quartet.cuh"
 
 namespace sf {
-// J/K digestion kernels of class cls (0..20) over one work slice
-cudaError_t launch_jk_f64(int cls, const KParams &kp, const ClassWork &w, const double *D, double *Jh, double *Kh,
+// J/K digestion kernels of class cls (0..20) over nw <= kMaxSegs segments, one launch
+cudaError_t launch_jk_f64(int cls, const KParams &kp, const ClassWork *w, int nw, const double *D, double *Jh, double *Kh,
                           cudaStream_t st);
-cudaError_t launch_jk_f32(int cls, const KParams &kp, const ClassWork &w, const float *D, double *Jh, double *Kh,
+cudaError_t launch_jk_f32(int cls, const KParams &kp, const ClassWork *w, int nw, const float *D, double *Jh, double *Kh,
                           cudaStream_t st);
-cudaError_t launch_jk_dd(int cls, const KParams &kp, const ClassWork &w, const dd *D, double *Jh, double *Kh,
+cudaError_t launch_jk_dd(int cls, const KParams &kp, const ClassWork *w, int nw, const dd *D, double *Jh, double *Kh,
                          cudaStream_t st);
 // the same with tdd_wide lanes per quartet (jk_dd_wide.cu)
-cudaError_t launch_jk_dd_wide(int cls, const KParams &kp, const ClassWork &w, const dd *D, double *Jh, double *Kh,
+cudaError_t launch_jk_dd_wide(int cls, const KParams &kp, const ClassWork *w, int nw, const dd *D, double *Jh, double *Kh,
                               cudaStream_t st);
 cudaError_t prepare_jk_dd_wide();
 // persistent multi-class FP32 J/K kernels (jk_persist.cu): one launch per
@@ -45,11 +45,11 @@ void md_tc_set_wait_limit(int iterations);
 // Schwarz bounds of pair class pc (0..5) over pairs [p0, p0+n)
 cudaError_t launch_schwarz(int pc, const KParams &kp, int p0, int n, double *qout, cudaStream_t st);
 
-cudaError_t launch_grad_f64(int cls, const KParams &kp, const ClassWork &w, const double *D, double *grad,
+cudaError_t launch_grad_f64(int cls, const KParams &kp, const ClassWork *w, int nw, const double *D, double *grad,
                             cudaStream_t st);
-cudaError_t launch_grad_f32(int cls, const KParams &kp, const ClassWork &w, const float *D, double *grad,
+cudaError_t launch_grad_f32(int cls, const KParams &kp, const ClassWork *w, int nw, const float *D, double *grad,
                             cudaStream_t st);
-cudaError_t launch_grad_dd(int cls, const KParams &kp, const ClassWork &w, const dd *D, double *grad,
+cudaError_t launch_grad_dd(int cls, const KParams &kp, const ClassWork *w, int nw, const dd *D, double *grad,
                            cudaStream_t st);
 cudaError_t prepare_grad_f64();
 cudaError_t prepare_grad_dd();

@@ -1304,6 +1304,41 @@ __device__ __forceinline__ int64_t work_count(const ClassWork &w) {
 constexpr int kBlock = 128;
 constexpr int kMaxWsplit = 64;
 
+// The lists of one launch: the segments of one class and arithmetic, each with
+// its own primitive split and its own range of CTAs, costliest first.  One
+// launch per segment made a build of a small molecule wait for the host:
+// (H2O)2 6-31G* had 194 launches of a few CTAs, issued in 0.9 ms, against 61
+// here (@MERGE@).
+constexpr int kMaxSegs = 12;
+struct ClassMulti {
+  ClassWork seg[kMaxSegs];
+  int cta0[kMaxSegs + 1];   // first CTA of each segment
+  int n;
+  __device__ __forceinline__ int find(int cta) const {
+    int s = 0;
+    while (s + 1 < n && cta >= cta0[s + 1]) ++s;
+    return s;
+  }
+};
+
+// host: append segment w whose kernel uses T lanes per quartet; cap > 0 limits
+// its CTAs (grid-stride kernels).  False: a bad split or too many CTAs.
+inline bool add_segment(ClassMulti &m, ClassWork w, int T, int64_t cap = 0) {
+  if (w.psplit < 1) w.psplit = 1;
+  if (w.wsplit < 1) w.wsplit = 1;
+  const int P = w.psplit, W = w.wsplit;
+  if (m.n >= kMaxSegs || T * P > 32 || (P & (P - 1)) || W > kMaxWsplit) return false;
+  const int G = kBlock / (T * P);
+  int64_t grid = (w.n * W + G - 1) / G;
+  if (cap > 0 && grid > cap) grid = cap;
+  if (m.n == 0) m.cta0[0] = 0;
+  if (m.cta0[m.n] + grid > 0x7fffffff) return false;
+  m.seg[m.n] = w;
+  m.cta0[m.n + 1] = m.cta0[m.n] + (int)grid;
+  ++m.n;
+  return true;
+}
+
 // One quartet group of the FP32 register path (one lane per quartet and
 // primitive sub-group): group gid of the list's W*P sub-groups per quartet,
 // Rys table rows read from the shared-memory copy tab_s of the class's root
@@ -1343,8 +1378,11 @@ __device__ __forceinline__ void load_tab32_block(const KParams &kp, int nr, floa
 }
 
 template <int LA, int LB, int LC, int LD, typename R, int T>
-__global__ void __launch_bounds__(kBlock) jk_kernel(KParams kp, ClassWork w, const R *__restrict__ D, double *Jh,
-                                                    double *Kh) {
+__global__ void __launch_bounds__(kBlock) jk_kernel(KParams kp, const __grid_constant__ ClassMulti m,
+                                                    const R *__restrict__ D, double *Jh, double *Kh) {
+  const int sg = m.find(blockIdx.x);
+  const ClassWork w = m.seg[sg];
+  const int64_t cta = (int)blockIdx.x - m.cta0[sg];   // among the segment's
   const int P = w.psplit, W = w.wsplit;
   const int TP = T * P;
   const int grp = threadIdx.x / TP, p = (threadIdx.x / T) % P, t = threadIdx.x % T;
@@ -1356,10 +1394,11 @@ __global__ void __launch_bounds__(kBlock) jk_kernel(KParams kp, ClassWork w, con
     __syncthreads();
     const float *tab_s = reinterpret_cast<const float *>(smem_raw);
     const int64_t nq = work_count(w);
-    for (int64_t gid = (int64_t)blockIdx.x * (kBlock / TP) + grp;; gid += (int64_t)gridDim.x * (kBlock / TP))
+    const int64_t stride = (int64_t)(m.cta0[sg + 1] - m.cta0[sg]) * (kBlock / TP);
+    for (int64_t gid = cta * (kBlock / TP) + grp;; gid += stride)
       if (!jk_f32_t1_step<LA, LB, LC, LD>(kp, w, gid, nq, tab_s, D, Jh, Kh)) return;
   }
-  const int64_t gid = (int64_t)blockIdx.x * (kBlock / TP) + grp;
+  const int64_t gid = cta * (kBlock / TP) + grp;
   const int64_t q = gid / W;
   const int sub = (int)(gid - q * W) * P + p;   // primitive sub-group of the W*P
   if (q >= work_count(w)) return;
