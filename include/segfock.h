@@ -365,9 +365,9 @@ int sf_fma_peak(int32_t precision, double *flops, float *ms, void *stream);
  * another component owns all device memory (a framework's memory pool, a
  * fixed memory budget) or a time-critical loop that must not enter the CUDA
  * allocator.  The scratch sf_fock_jk keeps in the handle (the half matrices
- * Jh, Kh and the single-precision copy of D) lives here in one static device
- * array of the library, sized for nao <= SF_NOALLOC_MAX_NAO (2.5 * 1024^2
- * doubles = 20 MiB, held on every GPU that loads the library until the
+ * Jh, Kh and the double-float and single-precision copies of D) lives here in one
+ * static device array of the library, sized for nao <= SF_NOALLOC_MAX_NAO (3.5 *
+ * 1024^2 doubles = 28 MiB, held on every GPU that loads the library until the
  * process exits).  Larger handles are rejected with SF_EINVAL.
  *
  * The call allocates nothing: no cudaMalloc, cudaFree or allocating library

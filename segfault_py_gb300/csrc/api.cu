@@ -340,6 +340,7 @@ struct sf_handle {
     int64_t quartets, prims;
     double flops;
     int64_t cost_hi;               // primitive cost of the segment's first quartet (tuning key)
+    int tail = 0;                  // the double-float part of an FP64 tier: its split is not tuned
     double est = 0.0;              // cost estimate (or tuned time) the stream assignment uses
   };
   // autotuned primitive splits S = P*W, keyed by (class, precision, cost_hi)
@@ -519,6 +520,20 @@ std::vector<int> lpt_streams(const std::vector<double> &cost_desc, int first = 0
 // number of primitive iterations; inside a cost bucket the (i, j) order of the
 // Schwarz-sorted pair lists is kept.  A partition (part, nparts) keeps every
 // nparts-th quartet of each sorted list, which balances cost across parts.
+// The FP64 kernels' quartets below this Schwarz bound run in double-float.  A
+// double-float quartet carries 2^-48 relative rounding instead of 2^-53, and a
+// quartet adds at most Q_ab Q_cd |D| to an element of J or K, so below 1e-3 of
+// the largest bounds (order one) its rounding lies under that of the large
+// quartets, which stay FP64: J and K of (H2O)16 6-31G* differ by 5e-15 of
+// their norm from the all-FP64 build, errors against 64-bit reference values are
+// the same to three digits; 68.0 -> 22.7 ms (everything in FP64: the pipe 88 % busy).
+constexpr double kDDTail = 1e-3;
+// ... when the class's part below it would hold the FP64 pipe for longer than
+// 20 us (estimated from its primitive quartets as in build_work at the measured
+// 1.25 TFLOP/s): a smaller one is hidden in the FP64 launch, and one more launch
+// per class costs (H2O)2 6-31G* 4 % of its 0.37 ms build
+constexpr double kDDTailMinFlops = 20e-6 * 1.25e12;
+
 // lanes per quartet of a launch of class ci in kind (0 FP64, 1 FP32, 2 dd)
 inline int kind_lanes(const ClassInfo &ci, int kind, int wide) {
   return kind == 1 ? ci.t32 : (kind == 2 && wide) ? tdd_wide(ci.la, ci.lb, ci.lc, ci.ld, ci.t64) : ci.t64;
@@ -538,7 +553,7 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     int x0, y0, same;
     int psplit, wsplit;
     int64_t cost_hi;
-    int wide;
+    int wide, tail;
   };
   std::vector<Pending> pend;
   h->st_q[0] = h->st_q[1] = h->st_pq[0] = h->st_pq[1] = 0;
@@ -553,7 +568,7 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     int64_t q = 0, pq = 0;
     double f = 0.0;
   };
-  std::vector<Part> parts(2 * kNumClass);
+  std::vector<Part> parts(3 * kNumClass);   // per class: accurate tier, FP32, double-float part of FP64
   std::vector<int64_t> totals(kNumClass, 0);
   auto build_class = [&](int cls, std::vector<int64_t> &hist) {
     const ClassInfo &ci = kClassInfo[cls];
@@ -564,7 +579,7 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     totals[cls] = same ? (int64_t)nX * (nX + 1) / 2 : (int64_t)nX * nY;
     if (nX == 0 || nY == 0) return;
     const double *qx = h->pq.data() + x0, *qy = h->pq.data() + y0;
-    std::vector<int64_t> m(nX), m64(nX);
+    std::vector<int64_t> m(nX), m64(nX), mdd(nX);   // ket prefix: all, accurate tier, its FP64 part
     for (int i = 0; i < nX; ++i) {
       int64_t mi = count_pass(qy, nY, qx[i], cut);
       if (same) mi = std::min<int64_t>(mi, i + 1);
@@ -573,19 +588,32 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
       else if (prec == SF_PREC_FP32) m6 = 0;
       else m6 = std::min<int64_t>(mi, count_pass(qy, nY, qx[i], std::max(cut32, cut)));
       m[i] = mi;
-      m64[i] = m6;
+      m64[i] = mdd[i] = m6;
     }
     const int nr = (ci.la + ci.lb + ci.lc + ci.ld) / 2 + 1;
     const double nabcd = (double)ncart(ci.la) * ncart(ci.lb) * ncart(ci.lc) * ncart(ci.ld);
     // launch kind of tier pr: 0 FP64, 1 FP32, 2 double-float
     const int hi_kind = (prec == SF_PREC_MIXED_DF || prec == SF_PREC_DF) ? 2 : 0;
-    for (int pr = 0; pr < 2; ++pr) {
-      const int kind = pr == 0 ? hi_kind : 1;
+    if (hi_kind == 0 && prec != SF_PREC_FP32) {
+      double tail = 0.0;
+      for (int i = 0; i < nX; ++i) {
+        mdd[i] = std::min<int64_t>(m64[i], count_pass(qy, nY, qx[i], std::max(kDDTail, cut)));
+        int64_t k = 0;
+        for (int64_t j = mdd[i]; j < m64[i]; ++j) k += h->pnp[y0 + j];
+        tail += (double)k * h->pnp[x0 + i];
+      }
+      if (tail * 2.0 * (nr * (nabcd + 30.0) + 40.0) < kDDTailMinFlops) mdd = m64;
+    }
+    for (int pr = 0; pr < 3; ++pr) {
+      const int kind = pr == 0 ? hi_kind : pr;
+      // ket range of bra i in this tier: [lo, hi) of the Q-sorted kets
+      const std::vector<int64_t> *from = pr == 0 ? nullptr : pr == 1 ? &m64 : &mdd;
+      const std::vector<int64_t> &upto = pr == 0 ? mdd : pr == 1 ? m : m64;
       // counting sort on (K_ab, K_cd)
       std::fill(hist.begin(), hist.end(), 0);
       int64_t n = 0;
       for (int i = 0; i < nX; ++i) {
-        const int64_t lo = pr == 0 ? 0 : m64[i], hi = pr == 0 ? m64[i] : m[i];
+        const int64_t lo = from ? (*from)[i] : 0, hi = upto[i];
         const int ka = h->pnp[x0 + i];
         for (int64_t j = lo; j < hi; ++j) ++hist[(size_t)ka * KB + h->pnp[y0 + j]];
         n += hi - lo;
@@ -607,13 +635,14 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
       }
       std::vector<int2> lst(n);
       for (int i = 0; i < nX; ++i) {
-        const int64_t lo = pr == 0 ? 0 : m64[i], hi = pr == 0 ? m64[i] : m[i];
+        const int64_t lo = from ? (*from)[i] : 0, hi = upto[i];
         const int ka = h->pnp[x0 + i];
         for (int64_t j = lo; j < hi; ++j) lst[pos[(size_t)ka * KB + h->pnp[y0 + j]]++] = make_int2(i, (int)j);
       }
       Pending p;
       // the double-float accurate tier of a mixed build runs its wide kernels
       p.wide = (kind == 2 && prec == SF_PREC_MIXED_DF) ? 1 : 0;
+      p.tail = pr == 2 ? 1 : 0;
       p.cost_hi = 0;
       p.psplit = 1;
       p.wsplit = 1;
@@ -632,7 +661,7 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
       p.n = (int64_t)lst.size();
       p.prims = (int64_t)(prims * frac);
       p.flops = ((double)prims * nr * 4.0 * nabcd + 12.0 * nabcd * (double)n) * frac;
-      Part &part = parts[2 * cls + pr];
+      Part &part = parts[3 * cls + pr];
       part.q = p.n;
       part.pq = p.prims;
       part.f = p.flops;
@@ -674,7 +703,7 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
         seg.cost_hi = cost_of(q0);
         int St = S;
         for (const sf_tune_entry &e : h->tune)
-          if (e.cls == cls && e.precision == kind && e.cost == seg.cost_hi) St = e.split;
+          if (!p.tail && e.cls == cls && e.precision == kind && e.cost == seg.cost_hi) St = e.split;
         seg.psplit = std::min(St, pmax);
         seg.wsplit = std::max(1, std::min(St / seg.psplit, kMaxWsplit));
         int64_t sp = 0;
@@ -702,16 +731,17 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
   }
   for (int cls = 0; cls < kNumClass; ++cls) {
     h->st_total += totals[cls];
-    for (int pr = 0; pr < 2; ++pr) {
-      Part &part = parts[2 * cls + pr];
+    for (int pr = 0; pr < 3; ++pr) {
+      Part &part = parts[3 * cls + pr];
+      const int acc = pr == 1 ? 1 : 0;   // accurate / FP32 counters
       for (Pending seg : part.segs) {
         seg.off += all.size();
         pend.push_back(seg);
       }
       all.insert(all.end(), part.lst.begin(), part.lst.end());
-      h->st_q[pr] += part.q;
-      h->st_pq[pr] += part.pq;
-      h->st_f[pr] += part.f;
+      h->st_q[acc] += part.q;
+      h->st_pq[acc] += part.pq;
+      h->st_f[acc] += part.f;
     }
   }
   SF_CK(h->d_list.upload(all));
@@ -726,7 +756,7 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     w.wsplit = p.wsplit;
     w.max_cost = (int)std::max<int64_t>(p.cost_hi, 1);
     w.wide = p.wide;
-    h->slices.push_back({p.cls, p.prec, w, p.n, p.prims, p.flops, p.cost_hi});
+    h->slices.push_back({p.cls, p.prec, w, p.n, p.prims, p.flops, p.cost_hi, p.tail});
   }
   // greedy longest-processing-time assignment of slices to side streams;
   // cost estimate: primitive quartets x roots x Cartesian outputs, FP64 work
@@ -749,7 +779,7 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
       const auto &sl = h->slices[k];
       bool found = false;
       for (const sf_tune_entry &e : h->tune)
-        if (e.cls == sl.cls && e.precision == sl.prec && e.cost == sl.cost_hi && e.ms_tuned > 0.f) {
+        if (!sl.tail && e.cls == sl.cls && e.precision == sl.prec && e.cost == sl.cost_hi && e.ms_tuned > 0.f) {
           timed[k] = e.ms_tuned;
           found = true;
         }
@@ -1025,8 +1055,8 @@ int profiling_events(sf_handle *h, cudaStream_t st);
 // one launch of the plan, nw segments of class cls: J/K digestion (Jh, Kh) or
 // gradient (g) kernels in the launch's arithmetic
 cudaError_t launch_one(sf_handle *h, int cls, int kind, const ClassWork *w, int nw, bool grad, const double *D,
-                       const float *D32, double *Jh, double *Kh, double *g, cudaStream_t st) {
-  const dd *Ddd = reinterpret_cast<const dd *>(h->d_Ddd.p);
+                       const float *D32, const float *Ddd_, double *Jh, double *Kh, double *g, cudaStream_t st) {
+  const dd *Ddd = reinterpret_cast<const dd *>(Ddd_);
   if (grad) {
     if (kind == 0) return launch_grad_f64(cls, h->kp, w, nw, D, g, st);
     if (kind == 1) return launch_grad_f32(cls, h->kp, w, nw, D32, g, st);
@@ -1041,13 +1071,13 @@ cudaError_t launch_one(sf_handle *h, int cls, int kind, const ClassWork *w, int 
 // merged launches (make_groups), or in the profiling modes every launch by
 // itself; profiling 1: events bracket each launch on its own stream;
 // profiling 2: the launches are serialised on st, each between two events.
-int run_plan(sf_handle *h, bool grad, const double *D, const float *D32, double *Jh, double *Kh, double *g,
-             cudaStream_t st, int profiling, int *launches) {
+int run_plan(sf_handle *h, bool grad, const double *D, const float *D32, const float *Ddd, double *Jh, double *Kh,
+             double *g, cudaStream_t st, int profiling, int *launches) {
   if (profiling == 2) {
     for (size_t k = 0; k < h->plan.size(); ++k) {
       SF_CK(cudaEventRecord(h->ev[2 * k], st));
       const auto &L = h->plan[k];
-      SF_CK(launch_one(h, h->slices[L.slice].cls, L.kind, &L.w, 1, grad, D, D32, Jh, Kh, g, st));
+      SF_CK(launch_one(h, h->slices[L.slice].cls, L.kind, &L.w, 1, grad, D, D32, Ddd, Jh, Kh, g, st));
       SF_CK(cudaEventRecord(h->ev[2 * k + 1], st));
       if (launches) ++*launches;
     }
@@ -1066,13 +1096,14 @@ int run_plan(sf_handle *h, bool grad, const double *D, const float *D32, double 
     const auto &L = h->plan[k];
     cudaStream_t ss = h->side[L.stream];
     SF_CK(cudaEventRecord(h->ev[2 * k], ss));
-    SF_CK(launch_one(h, h->slices[L.slice].cls, L.kind, &L.w, 1, grad, D, D32, Jh, Kh, g, ss));
+    SF_CK(launch_one(h, h->slices[L.slice].cls, L.kind, &L.w, 1, grad, D, D32, Ddd, Jh, Kh, g, ss));
     SF_CK(cudaEventRecord(h->ev[2 * k + 1], ss));
     if (launches) ++*launches;
   }
   for (size_t k = 0; !profiling && k < h->groups.size(); ++k) {
     const auto &G = h->groups[k];
-    SF_CK(launch_one(h, G.cls, G.kind, G.w.data(), (int)G.w.size(), grad, D, D32, Jh, Kh, g, h->side[G.stream]));
+    SF_CK(launch_one(h, G.cls, G.kind, G.w.data(), (int)G.w.size(), grad, D, D32, Ddd, Jh, Kh, g,
+                     h->side[G.stream]));
     if (launches) ++*launches;
   }
   // the persistent tier launches last: they take the SM slots the others leave
@@ -1091,8 +1122,8 @@ int run_plan(sf_handle *h, bool grad, const double *D, const float *D32, double 
 }
 
 // classification, plan and launches of one Fock build (Jh, Kh) or gradient (g)
-int run_call(sf_handle *h, bool grad, const double *D, const float *D32, double *Jh, double *Kh, double *g,
-             double cut, double cut32, cudaStream_t st, int profiling, int *launches) {
+int run_call(sf_handle *h, bool grad, const double *D, const float *D32, const float *Ddd, double *Jh, double *Kh,
+             double *g, double cut, double cut32, cudaStream_t st, int profiling, int *launches) {
   int active = 0;
   int rc = density_classify(h, D, grad, cut, cut32, st, launches, &active);
   if (rc) return rc;
@@ -1103,7 +1134,7 @@ int run_call(sf_handle *h, bool grad, const double *D, const float *D32, double 
     rc = profiling_events(h, st);
     if (rc) return rc;
   }
-  return run_plan(h, grad, D, D32, Jh, Kh, g, st, profiling, launches);
+  return run_plan(h, grad, D, D32, Ddd, Jh, Kh, g, st, profiling, launches);
 }
 
 // events of the profiling modes: two per launch plus the build's start,
@@ -1120,7 +1151,7 @@ int profiling_events(sf_handle *h, cudaStream_t st) {
 }
 
 // FP32 / double-float copies of D needed by the current launch list
-int convert_density(sf_handle *h, const double *D, float *D32, cudaStream_t st, int *launches) {
+int convert_density(sf_handle *h, const double *D, float *D32, float *Ddd, cudaStream_t st, int *launches) {
   const size_t nn = (size_t)h->nao * h->nao;
   bool need32 = false, needdd = false;
   for (const auto &s : h->slices) {
@@ -1133,8 +1164,7 @@ int convert_density(sf_handle *h, const double *D, float *D32, cudaStream_t st, 
     if (launches) ++*launches;
   }
   if (needdd) {
-    to_dd_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(D, reinterpret_cast<float2 *>(h->d_Ddd.p),
-                                                                (int64_t)nn);
+    to_dd_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(D, reinterpret_cast<float2 *>(Ddd), (int64_t)nn);
     SF_CK(cudaGetLastError());
     if (launches) ++*launches;
   }
@@ -1343,9 +1373,10 @@ int run_eri_plan(sf_eri_plan *pl, int precision, double *out, cudaStream_t st) {
 }  // namespace
 
 // Scratch of sf_fock_jk_noalloc: Jh and Kh (nao^2 doubles each) followed by
-// the single-precision copy of D (nao^2 floats), for nao <= SF_NOALLOC_MAX_NAO.
+// the double-float copy of D (nao^2 float pairs) and its single-precision copy
+// (nao^2 floats), for nao <= SF_NOALLOC_MAX_NAO.
 static constexpr size_t kNoAllocNN = (size_t)SF_NOALLOC_MAX_NAO * SF_NOALLOC_MAX_NAO;
-static __device__ __align__(256) double g_noalloc_scratch[2 * kNoAllocNN + (kNoAllocNN + 1) / 2];
+static __device__ __align__(256) double g_noalloc_scratch[3 * kNoAllocNN + (kNoAllocNN + 1) / 2];
 
 namespace {
 // device address of g_noalloc_scratch per device (host code cannot use the
@@ -1695,9 +1726,9 @@ int sf_fock_jk(sf_handle *h, const double *D, double *J, double *K, int32_t prec
   SF_CK(cudaMemsetAsync(h->d_Jh.p, 0, nn * sizeof(double), st));
   SF_CK(cudaMemsetAsync(h->d_Kh.p, 0, nn * sizeof(double), st));
   int launches = 0;
-  rc = convert_density(h, D, h->d_D32.p, st, &launches);
+  rc = convert_density(h, D, h->d_D32.p, h->d_Ddd.p, st, &launches);
   if (rc) return rc;
-  rc = run_call(h, false, D, h->d_D32.p, h->d_Jh.p, h->d_Kh.p, nullptr, cutoff, fp32_cutoff, st, h->profiling,
+  rc = run_call(h, false, D, h->d_D32.p, h->d_Ddd.p, h->d_Jh.p, h->d_Kh.p, nullptr, cutoff, fp32_cutoff, st, h->profiling,
                 &launches);
   if (rc) return rc;
   symmetrize_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(h->d_Jh.p, h->d_Kh.p, J, K, n);
@@ -1796,7 +1827,7 @@ int sf_autotune(sf_handle *h, const double *D, int32_t precision, double cutoff,
   cudaStream_t st = (cudaStream_t)stream;
   int rc = build_work(h, precision, cutoff, fp32_cutoff);
   if (rc) return rc;
-  rc = convert_density(h, D, h->d_D32.p, st, nullptr);
+  rc = convert_density(h, D, h->d_D32.p, h->d_Ddd.p, st, nullptr);
   if (rc) return rc;
   cudaEvent_t e0, e1;
   SF_CK(cudaEventCreate(&e0));
@@ -1823,12 +1854,12 @@ int sf_autotune(sf_handle *h, const double *D, int32_t precision, double cutoff,
   auto time_build = [&](float *ms) -> int {
     int r2 = build_work(h, precision, cutoff, fp32_cutoff);
     if (r2) return r2;
-    r2 = run_call(h, false, D, h->d_D32.p, h->d_Jh.p, h->d_Kh.p, nullptr, cutoff, fp32_cutoff, st, 0,
+    r2 = run_call(h, false, D, h->d_D32.p, h->d_Ddd.p, h->d_Jh.p, h->d_Kh.p, nullptr, cutoff, fp32_cutoff, st, 0,
                   nullptr);   // warm-up
     if (r2) return r2;
     SF_CK(cudaEventRecord(e0, st));
     for (int r = 0; r < reps; ++r) {
-      r2 = run_call(h, false, D, h->d_D32.p, h->d_Jh.p, h->d_Kh.p, nullptr, cutoff, fp32_cutoff, st, 0, nullptr);
+      r2 = run_call(h, false, D, h->d_D32.p, h->d_Ddd.p, h->d_Jh.p, h->d_Kh.p, nullptr, cutoff, fp32_cutoff, st, 0, nullptr);
       if (r2) return r2;
     }
     SF_CK(cudaEventRecord(e1, st));
@@ -1906,6 +1937,7 @@ int sf_autotune(sf_handle *h, const double *D, int32_t precision, double cutoff,
   // 2. per-launch splits, each launch timed alone
   int tuned = 0;
   for (auto &sl : h->slices) {
+    if (sl.tail) continue;
     const ClassInfo &ci = kClassInfo[sl.cls];
     const int pmax = 32 / kind_lanes(ci, sl.prec, sl.w.wide);
     const int S0 = sl.w.psplit * sl.w.wsplit;
@@ -2036,15 +2068,12 @@ int sf_fock_jk_noalloc(sf_handle *h, const double *D, double *J, double *K, int3
   const int n = h->nao;
   const size_t nn = (size_t)n * n;
   double *Jh = scratch, *Kh = scratch + nn;
-  float *D32 = reinterpret_cast<float *>(scratch + 2 * nn);
+  float *Ddd = reinterpret_cast<float *>(scratch + 2 * nn);   // nao^2 float pairs, then nao^2 floats
+  float *D32 = reinterpret_cast<float *>(scratch + 3 * nn);
   SF_CK(cudaMemsetAsync(scratch, 0, 2 * nn * sizeof(double), st));
-  bool need32 = false;
-  for (const auto &s : h->slices) need32 |= s.prec == 1;
-  if (need32) {
-    to_float_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(D, D32, (int64_t)nn);
-    SF_CK(cudaGetLastError());
-  }
-  int rc = run_call(h, false, D, D32, Jh, Kh, nullptr, cutoff, fp32_cutoff, st, 0, nullptr);
+  int rc = convert_density(h, D, D32, Ddd, st, nullptr);
+  if (rc) return rc;
+  rc = run_call(h, false, D, D32, Ddd, Jh, Kh, nullptr, cutoff, fp32_cutoff, st, 0, nullptr);
   if (rc) return rc;
   symmetrize_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(Jh, Kh, J, K, n);
   SF_CK(cudaGetLastError());
@@ -2062,10 +2091,10 @@ int sf_grad_jk(sf_handle *h, const double *D, double *grad, int32_t precision, d
   cudaStream_t st = (cudaStream_t)stream;
   int rc = build_work(h, precision, cutoff, fp32_cutoff);
   if (rc) return rc;
-  rc = convert_density(h, D, h->d_D32.p, st, nullptr);
+  rc = convert_density(h, D, h->d_D32.p, h->d_Ddd.p, st, nullptr);
   if (rc) return rc;
   // per-launch events in the profiling modes (serialised in mode 2), read by sf_get_slice_info
-  return run_call(h, true, D, h->d_D32.p, nullptr, nullptr, grad, cutoff, fp32_cutoff, st, h->profiling, nullptr);
+  return run_call(h, true, D, h->d_D32.p, h->d_Ddd.p, nullptr, nullptr, grad, cutoff, fp32_cutoff, st, h->profiling, nullptr);
 }
 
 int sf_grad_stats(sf_handle *h, sf_stats *stats, void *stream) {
