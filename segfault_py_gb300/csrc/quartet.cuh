@@ -44,6 +44,12 @@ struct KParams {
   // Rys table as dd rows (rys_tabdd_offset) and the asymptotic constants
   DevPrims<dd> pdd;
   const float4 *pair32;   // per canonical pair: (Ax,Ay,Az,ABx) (ABy,ABz,ao_a,ao_b) (poff,np,a,b), FP32 / int bits
+  // the same with the pair's full list of primitive pairs: the split FP32 lists
+  // keep it, so that a lane's share of the primitive loop, and with it the FP32
+  // rounding of J and K, does not depend on which pairs are negligible (a
+  // different share moved K of hexane 6-31G* by 1.5e-9 of its norm, an unsplit
+  // loop without them gives the same bits)
+  const float4 *pair32f;
   const dd *cxd, *cyd, *czd;
   const float4 *tabdd;
   dd asymdd_r[kMaxRoots + 1][kMaxRoots], asymdd_w[kMaxRoots + 1][kMaxRoots];
@@ -622,9 +628,10 @@ __device__ __forceinline__ QGeom<R> make_geom(const KParams &kp, int pab, int pc
 // FP32 geometry of a quartet from the packed pair records (three 16-byte
 // loads per pair instead of about twenty scattered loads of pair, shell and
 // centre arrays; the quartet set-up is a latency chain in the light classes)
-__device__ __forceinline__ QGeom<float> make_geom32(const KParams &kp, int pab, int pcd) {
+__device__ __forceinline__ QGeom<float> make_geom32(const KParams &kp, int pab, int pcd, bool full) {
   QGeom<float> g;
-  const float4 *pa = kp.pair32 + 3 * (size_t)pab, *pc = kp.pair32 + 3 * (size_t)pcd;
+  const float4 *tab = full ? kp.pair32f : kp.pair32;
+  const float4 *pa = tab + 3 * (size_t)pab, *pc = tab + 3 * (size_t)pcd;
   const float4 a0 = __ldg(pa), a1 = __ldg(pa + 1), a2 = __ldg(pa + 2);
   const float4 c0 = __ldg(pc), c1 = __ldg(pc + 1), c2 = __ldg(pc + 2);
   g.Ax = a0.x; g.Ay = a0.y; g.Az = a0.z; g.ABx = a0.w; g.ABy = a1.x; g.ABz = a1.y;
@@ -1355,7 +1362,7 @@ __device__ __forceinline__ bool jk_f32_t1_step(const KParams &kp, const ClassWor
   if (q >= nq) return false;
   const int sub = (int)(gid - q * W) * P + p;
   const int2 ij = __ldg(w.list + q);
-  const QGeom<R> g = make_geom32(kp, w.x0 + ij.x, w.y0 + ij.y);
+  const QGeom<R> g = make_geom32(kp, w.x0 + ij.x, w.y0 + ij.y, P * W > 1);
   R scale = (R)1;
   if (g.a == g.b) scale *= (R)0.5;
   if (g.c == g.d) scale *= (R)0.5;
@@ -1406,7 +1413,7 @@ __global__ void __launch_bounds__(kBlock) jk_kernel(KParams kp, const __grid_con
   const int i = ij.x, j = ij.y;
   const int pab = w.x0 + i, pcd = w.y0 + j;
   QGeom<R> g;
-  if constexpr (std::is_same<R, float>::value) g = make_geom32(kp, pab, pcd);
+  if constexpr (std::is_same<R, float>::value) g = make_geom32(kp, pab, pcd, P * W > 1);
   else g = make_geom<R>(kp, pab, pcd, false, false);
   R scale = (R)1;
   if (g.a == g.b) scale *= (R)0.5;

@@ -7,7 +7,8 @@
 //              sf_schwarz, sorted by Schwarz bound Q_ab descending inside each
 //              class.  A pair record holds a, b, the offset and count of its
 //              primitive pairs, and Q_ab.
-//   prims    : one 8-value record per primitive pair (alpha_i, beta_j):
+//   prims    : one 8-value record per kept primitive pair (alpha_i, beta_j),
+//              those negligible against the pair's largest left out:
 //              p = alpha+beta, P = (alpha A + beta B)/p, 0.5/p and
 //              K~ = c_i c_j exp(-alpha beta/p |AB|^2) sqrt(2) pi^(5/4) / p,
 //              in FP64 and FP32.  K~_ab K~_cd / sqrt(p+q) is the full
