@@ -472,8 +472,6 @@ void fill_kparams(sf_handle *h) {
 
 // tables of the one-electron kernels
 void one_params_tables(const sf_handle *h, OneParams *P) {
-  P->tab64 = h->kp.tab64;
-  P->asym = h->kp.asym;
   P->pr = h->kp.pr;
   P->rec = h->kp.p64.rec;
   P->boys = h->d_boys.p;
@@ -1599,6 +1597,7 @@ int sf_create(const sf_shell_desc *shells, int32_t nshell, sf_handle **out) {
   SF_CK(prepare_eri());
   SF_CK(prepare_eri_dd());
   SF_CK(prepare_md());
+  SF_CK(prepare_one_electron());
   SF_CK(prepare_md_tc());
   SF_CK(prepare_grad_f64());
   SF_CK(prepare_grad_f32());
@@ -2172,17 +2171,13 @@ int sf_grad_one_electron(sf_handle *h, const double *atom_xyz, const double *cha
   DeviceGuard g(h->device);
   OneParams P;
   P.sh = h->kp.sh;
-  P.exps = h->d_exps.p;
-  P.coefs = h->d_coefs.p;
-  P.poff = h->d_spoff.p;
-  P.nshell = h->nshell;
   P.nao = h->nao;
   P.atom_xyz = atom_xyz;
   P.charges = charges;
   P.natom = natom;
   P.S = P.T = P.V = nullptr;
   one_params_tables(h, &P);
-  SF_CK(launch_one_electron_grad(P, D, W, grad, (cudaStream_t)stream));
+  SF_CK(launch_one_electron_grad(P, D, W, grad, h->nsm, (cudaStream_t)stream));
   return SF_OK;
 }
 
@@ -2292,10 +2287,6 @@ int sf_one_electron(sf_handle *h, const double *atom_xyz, const double *charges,
   DeviceGuard g(h->device);
   OneParams P;
   P.sh = h->kp.sh;
-  P.exps = h->d_exps.p;
-  P.coefs = h->d_coefs.p;
-  P.poff = h->d_spoff.p;
-  P.nshell = h->nshell;
   P.nao = h->nao;
   P.atom_xyz = atom_xyz;
   P.charges = charges;

@@ -63,14 +63,10 @@ cudaError_t prepare_eri();
 // one-electron kernel parameters (oneint.cu)
 struct OneParams {
   DevShells sh;
-  const double *exps, *coefs;   // per shell primitives (shell prim offsets in poff)
-  const int *poff;
-  int nshell, nao;
+  int nao;
   const double *atom_xyz, *charges;
   int natom;
   double *S, *T, *V;
-  const double *tab64;          // FP64 Rys rule (Boys values of the gradient kernel)
-  RysAsym asym;
   DevPairs pr;                  // canonical shell pairs, class c at [cstart[c], cstart[c + 1])
   const double *rec;            // their primitive-pair records
   int cstart[kNumPairClass + 1];
@@ -80,8 +76,9 @@ struct OneParams {
 cudaError_t launch_one_electron(const OneParams &P, cudaStream_t st);
 // gradient of sum_ij D_ij (T+V)_ij - W_ij S_ij (derivatives of the basis
 // centres and, for V, of the nuclei), accumulated into grad[3*natom]
-cudaError_t launch_one_electron_grad(const OneParams &P, const double *D, const double *W, double *grad,
+cudaError_t launch_one_electron_grad(const OneParams &P, const double *D, const double *W, double *grad, int nsm,
                                      cudaStream_t st);
+cudaError_t prepare_one_electron();
 
 // smem bytes of a group kernel
 template <int LA, int LB, int LC, int LD, typename R, int T>

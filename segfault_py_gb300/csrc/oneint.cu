@@ -56,35 +56,8 @@ __device__ __forceinline__ void boys_table(const double *tab, double T, double (
   }
 }
 
-// E[i][j][t] for i <= LI, j <= LJ, t <= i+j along one direction
-template <int LI, int LJ>
-__device__ __forceinline__ void hermite_e(double p, double xpa, double xpb, double e0,
-                                          double (&E)[LI + 1][LJ + 1][LI + LJ + 1]) {
-#pragma unroll
-  for (int i = 0; i <= LI; ++i)
-#pragma unroll
-    for (int j = 0; j <= LJ; ++j)
-#pragma unroll
-      for (int t = 0; t <= LI + LJ; ++t) E[i][j][t] = 0.0;
-  const double h = 0.5 / p;
-  E[0][0][0] = e0;
-#pragma unroll
-  for (int i = 0; i < LI; ++i)
-#pragma unroll
-    for (int t = 0; t <= i + 1; ++t)
-      E[i + 1][0][t] = (t > 0 ? h * E[i][0][t - 1] : 0.0) + xpa * E[i][0][t] + (t + 1 <= i ? (t + 1) * E[i][0][t + 1] : 0.0);
-#pragma unroll
-  for (int i = 0; i <= LI; ++i)
-#pragma unroll
-    for (int j = 0; j < LJ; ++j)
-#pragma unroll
-      for (int t = 0; t <= i + j + 1; ++t)
-        E[i][j + 1][t] = (t > 0 ? h * E[i][j][t - 1] : 0.0) + xpb * E[i][j][t] +
-                         (t + 1 <= i + j ? (t + 1) * E[i][j][t + 1] : 0.0);
-}
-
-
-// the same from 1/(2p) with E^00_0 = 1 (the product Gaussian kept apart)
+// E[i][j][t] for i <= LI, j <= LJ, t <= i+j along one direction, from h = 1/(2p)
+// with E^00_0 = 1 (the product Gaussian kept apart)
 template <int LI, int LJ>
 __device__ __forceinline__ void hermite_e(double h, double xpa, double xpb, double (&E)[LI + 1][LJ + 1][LI + LJ + 1]) {
 #pragma unroll
@@ -361,306 +334,319 @@ cudaError_t launch_one_electron(const OneParams &P, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------------------
-// Gradient of E1 = sum_ij D_ij (T_ij + V_ij) - W_ij S_ij.  With D, W and the
-// operators symmetric, d/dR sum_ij D_ij O_ij = 2 sum_ij D_ij <d phi_i/dR|O|phi_j>
-// over ordered shell pairs; per canonical pair (a >= b) both the bra and the
-// ket derivative are taken, d phi/dA = 2 alpha phi_{+1} - a phi_{-1}:
-//  * S and T (two-centre): the ket derivative is minus the bra one;
-//  * V: the bra and ket derivative share R_tuv(p, P - C) of each nucleus C,
-//    which receives minus their sum (translational invariance of
-//    <a|1/r_C|b>).
-// CTA per canonical pair (a, b), 64 threads.  For every primitive pair whose
-// bound (product Gaussian x block max of |D|, |W| x derivative, kinetic and
-// attraction factors) is not below 1e-15:
-//  * E coefficients (bra to LA+1, ket to LB+2) into shared memory;
-//  * the S and T bra-derivative terms, one (i, j, direction) per thread;
-//  * the density-contracted Hermite coefficients of the bra and the ket
-//    derivative, M^d_tuv = 2pi/p c_i c_j sum_{i in a, j in b} D_ij sum_+- f
-//    E.. E.. E.. (nucleus independent), cooperatively into shared memory;
-//  * every thread takes nuclei C = t, t+64, ...: Boys values F_m(p |P-C|^2)
-//    = sum_i w_i u_i^m from the FP64 Rys rule of floor(L/2)+1 points (exact
-//    for m <= L), R_tuv by the Hermite Coulomb recursion, and
-//    dV/dX_d = -Z_C sum_tuv M^d_tuv R_tuv.
-constexpr int kOneGradThreads = 64;
-
-// shared-memory doubles of one_pair_grad2<LA, LB>: E coefficients, the bra and
-// ket Hermite coefficients MA, MB, the density block and the reduction rows
-template <int LA, int LB>
-constexpr int one_grad_smem() {
-  return 3 * (LA + 2) * (LB + 3) * (LA + LB + 4) + 6 * (LA + LB + 2) * (LA + LB + 2) * (LA + LB + 2) +
-         ncart(LA) * ncart(LB) + 6 * kOneGradThreads;
-}
-constexpr int kOneGradSmem = one_grad_smem<2, 2>();   // the largest
+// Gradient of E1 = sum_ij D_ij (T_ij + V_ij) - W_ij S_ij.  Per canonical pair
+// (a, b) and primitive pair, with P fixed or X = A - B fixed:
+//  * a derivative with respect to A is alpha/p d/dP + d/dX, to B
+//    beta/p d/dP - d/dX;
+//  * d/dP raises a Hermite function, so with H_tuv = sum_ij D_ij E E E the force
+//    on nucleus C is Z sum_tuv H_tuv R_{t+1,u,v} (x direction) and d/dP is minus
+//    the sum of these over the nuclei;
+//  * d/dX acts on the E coefficients, with dphi/dA = 2 alpha phi_{+1} - a phi_{-1}:
+//    dE_t/dX = 2 alpha E^{i+1,j}_t - i E^{i-1,j}_t - alpha/p E^{ij}_{t-1}, contracted
+//    with S_tuv = sum_C -Z_C R_tuv once per primitive pair;
+//  * S and T (two-centre): the bra derivative from one-dimensional overlap and
+//    kinetic tables and their derivatives, the ket one is minus it.
+// Lanes as in one_electron_kernel: groups of G lanes per primitive pair, lanes
+// over nuclei, then over the block's entries.  A warp strides over the pairs
+// and keeps the forces in its own shared-memory copy (one per group, so no
+// atomics), flushed once at the end: every pair adds to all 3 natom words.
+// Primitive pairs whose contributions all stay below 1e-15 are skipped (bounds
+// as in one_electron_kernel, times the block maximum of |D|, |W| and the growth
+// of a derivative, 2 max(alpha, beta) + L).
+// (H2O)16 6-31G*: the forces of (H2O)8, FP32 + double-float, 7.6 -> 6.4 ms; before (a CTA per pair, bra and ket Hermite
+// coefficients per primitive pair, one global atomic per nucleus and direction)
+// 3.9 ms.
+constexpr int kOneGradWarps = 2;
+constexpr int kOneGradAtoms = 128;   // larger molecules add to global memory directly
 
 template <int LA, int LB>
-__device__ void one_pair_grad2(const OneParams &P, const double *Dm, const double *Wm, double *grad, int a, int b,
-                               double *smem) {
-  constexpr int NA = ncart(LA), NB = ncart(LB);
-  constexpr int LE = LA + 1, L = LA + LB + 1, NH = (L + 1) * (L + 1) * (L + 1);
-  constexpr int NRT = L / 2 + 1;   // Rys points whose rule is exact for F_0 .. F_L
-  constexpr int EN = (LE + 1) * (LB + 3) * (LE + LB + 3);
-  const double pi = 3.14159265358979323846;
-  // carved from the kernel's one shared buffer (each instantiation declaring
-  // its own arrays made the kernel hold all nine sets, 79.5 KB)
-  using EArr = double[LE + 1][LB + 3][LE + LB + 3];
-  EArr *E = reinterpret_cast<EArr *>(smem);
-  double(*MA)[NH] = reinterpret_cast<double(*)[NH]>(smem + 3 * EN);
-  double(*MB)[NH] = MA + 3;
-  double(*Dab)[NB] = reinterpret_cast<double(*)[NB]>(smem + 3 * EN + 6 * NH);
-  double(*red)[6] = reinterpret_cast<double(*)[6]>(smem + 3 * EN + 6 * NH + NA * NB);
-  static_assert(3 * EN + 6 * NH + NA * NB + 6 * kOneGradThreads == one_grad_smem<LA, LB>(), "smem layout");
-  const int tid = threadIdx.x;
-  const bool two = a != b;   // canonical pair with a distinct ket: ket derivative too
+struct OneGrad {
+  static constexpr int L = LA + LB, IJ = (LA + 1) * (LB + 1);
+  static constexpr int NT = ntuv(L);
+  static constexpr int ES = IJ * (L + 1);                      // E_t of one direction
+  // doubles of a group: E, dE/dX (3 directions), s, k, ds, dk (3), S_tuv, H_tuv
+  static constexpr int GROUP = 6 * ES + 12 * IJ + 2 * NT;
+  static constexpr int WARP = 4 * GROUP + 2 * ncart(LA) * ncart(LB);   // four groups, D and W blocks
+};
+constexpr int kOneGradWarp = OneGrad<2, 2>::WARP;   // the largest
+
+template <int LA, int LB>
+__device__ __forceinline__ void one_pair_grad(const OneParams &P, const double *Dm, const double *Wm, double *frc,
+                                              int fstride, double *grad, int pair, double *smem, float zs, int lane) {
+  using O = OneGrad<LA, LB>;
+  constexpr int NA = ncart(LA), NB = ncart(LB), L = O::L, L1 = L + 1, IJ = O::IJ, NT = O::NT, ES = O::ES;
+  const int a = P.pr.a[pair], b = P.pr.b[pair], np = P.pr.np[pair];
+  const double *rec0 = P.rec + (size_t)P.pr.poff[pair] * kPrimRec;
+  const int G = np >= 3 ? 8 : np == 2 ? 16 : 32;
+  const int sub = lane / G, l = lane % G, ngrp = 32 / G;
+  double *E = smem + sub * O::GROUP, *X = E + 3 * ES, *s1 = X + 3 * ES, *k1 = s1 + 3 * IJ, *ds = k1 + 3 * IJ,
+         *dk = ds + 3 * IJ, *St = dk + 3 * IJ, *Ht = St + NT;
+  double *Db = smem + 4 * O::GROUP, *Wb = Db + NA * NB;
+#define SF_IJ(d, i, j) ((d) * IJ + (i) * (LB + 1) + (j))
+#define SF_ET(d, i, j, t) (SF_IJ(d, i, j) * (L + 1) + (t))
   const double A[3] = {P.sh.cx[a], P.sh.cy[a], P.sh.cz[a]};
   const double B[3] = {P.sh.cx[b], P.sh.cy[b], P.sh.cz[b]};
   const int a0 = P.sh.ao[a], b0 = P.sh.ao[b], n = P.nao;
-  // block maximum of |D| and |W| and the summed nuclear charge: the scale of
-  // everything this pair adds, for the primitive-pair screening below
-  double dw = 0.0, zs = 0.0;
-  for (int k = tid; k < NA * NB; k += blockDim.x) {
-    const int i = k / NB, j = k % NB;
-    const double nrm = cart_norm(LA, i) * cart_norm(LB, j);
-    Dab[i][j] = Dm[(a0 + i) * n + b0 + j] * nrm;
-    dw = fmax(dw, fmax(fabs(Dab[i][j]), fabs(Wm[(a0 + i) * n + b0 + j] * nrm)));
+  const double mult = a == b ? 1.0 : 2.0;   // (i, j) and (j, i)
+  float dw = 0.0f;
+  __syncwarp();
+  for (int k = lane; k < NA * NB; k += 32) {
+    const double nrm = mult * cart_norm(LA, k / NB) * cart_norm(LB, k % NB);
+    const size_t at = (size_t)(a0 + k / NB) * n + b0 + k % NB;
+    Db[k] = Dm[at] * nrm;
+    Wb[k] = Wm[at] * nrm;
+    dw = fmaxf(dw, fmaxf(fabsf((float)Db[k]), fabsf((float)Wb[k])));
   }
-  for (int k = tid; k < P.natom; k += blockDim.x) zs += fabs(P.charges[k]);
-  for (int off = 16; off > 0; off >>= 1) {
-    dw = fmax(dw, __shfl_xor_sync(0xffffffffu, dw, off));
-    zs += __shfl_xor_sync(0xffffffffu, zs, off);
-  }
-  if ((tid & 31) == 0) {
-    red[tid >> 5][0] = dw;
-    red[tid >> 5][1] = zs;
-  }
-  __syncthreads();
-  dw = 0.0;
-  zs = 0.0;
-  for (int w = 0; w < (int)blockDim.x / 32; ++w) {
-    dw = fmax(dw, red[w][0]);
-    zs += red[w][1];
-  }
-  __syncthreads();   // red is written again by the final reduction
-  double R2 = 0.0;
-  for (int d = 0; d < 3; ++d) R2 += (A[d] - B[d]) * (A[d] - B[d]);
-  double gST[3] = {0.0, 0.0, 0.0}, gVA[3] = {0.0, 0.0, 0.0}, gVB[3] = {0.0, 0.0, 0.0};
-  for (int ia = P.poff[a]; ia < P.poff[a + 1]; ++ia)
-    for (int ib = P.poff[b]; ib < P.poff[b + 1]; ++ib) {
-      const double al = P.exps[ia], be = P.exps[ib], p = al + be, mu = al * be / p;
-      const double cc = P.coefs[ia] * P.coefs[ib];
-      // primitive pairs whose contributions all stay below 1e-15 are skipped
-      // (the same on every thread, so the barriers below stay uniform): the
-      // product Gaussian c_i c_j exp(-mu |AB|^2) (pi/p)^3/2 bounds the
-      // overlap; E coefficients grow at most as (|AB| + 1/sqrt(p) + 1)^(L+1),
-      // derivatives as 2 max(alpha, beta) + L, kinetic terms as
-      // 3 beta (LB + 2), attraction as 2 sqrt(p/pi) times the summed charge
-      {
-        const double g = fabs(cc) * exp(-mu * R2) * pow(pi / p, 1.5) * dw;
-        const double e = pow(sqrt(R2) + rsqrt(p) + 1.0, (double)(L + 1));
-        const double f = (2.0 * fmax(al, be) + L) * (1.0 + 2.0 * sqrt(p / pi) * zs + 3.0 * fmax(al, be) * (LB + 2));
-        if (g * e * f < 1e-15) continue;
-      }
-      double Pc[3];
-      for (int d = 0; d < 3; ++d) Pc[d] = (al * A[d] + be * B[d]) / p;
-      __syncthreads();   // previous iteration done with E, M
-      if (tid < 3) {
-        const int d = tid;
-        const double X = A[d] - B[d];
-        double Et[LE + 1][LB + 3][LE + LB + 3];
-        hermite_e<LE, LB + 2>(p, Pc[d] - A[d], Pc[d] - B[d], exp(-mu * X * X), Et);
-        for (int i = 0; i <= LE; ++i)
-          for (int j = 0; j <= LB + 2; ++j)
-            for (int t = 0; t <= LE + LB + 2; ++t) E[d][i][j][t] = Et[i][j][t];
-      }
-      __syncthreads();
-      // overlap / kinetic bra derivatives (Pulay -W dS, D dT), one (i, j, d)
-      // per thread (gST is summed over the CTA at the end)
-      {
-        const double sp = pow(pi / p, 1.5);
-        for (int task = tid; task < NA * NB * 3; task += blockDim.x) {
-            const int i = task / (NB * 3), j = (task / 3) % NB, d = task % 3;
-            const double nrm = cart_norm(LA, i) * cart_norm(LB, j);
-            const double Dij = Dab[i][j], Wij = Wm[(a0 + i) * n + b0 + j] * nrm;
-            const int bx[3] = {cart_e(LB, j, 0), cart_e(LB, j, 1), cart_e(LB, j, 2)};
-            {
-              double dS = 0.0, dT = 0.0;
-              for (int sgn = 0; sgn < 2; ++sgn) {
-                int ax[3] = {cart_e(LA, i, 0), cart_e(LA, i, 1), cart_e(LA, i, 2)};
-                const int ad = ax[d];
-                if (sgn == 1 && ad == 0) continue;
-                ax[d] += sgn == 0 ? 1 : -1;
-                const double f = sgn == 0 ? 2.0 * al : -(double)ad;
-                const double sx = E[0][ax[0]][bx[0]][0], sy = E[1][ax[1]][bx[1]][0], sz = E[2][ax[2]][bx[2]][0];
-                const double s0 = sx * sy * sz * sp;
-                double t = be * (2 * (bx[0] + bx[1] + bx[2]) + 3) * s0;
-                t -= 2.0 * be * be * sp *
-                     (E[0][ax[0]][bx[0] + 2][0] * sy * sz + sx * E[1][ax[1]][bx[1] + 2][0] * sz +
-                      sx * sy * E[2][ax[2]][bx[2] + 2][0]);
-                if (bx[0] >= 2) t -= 0.5 * bx[0] * (bx[0] - 1) * sp * E[0][ax[0]][bx[0] - 2][0] * sy * sz;
-                if (bx[1] >= 2) t -= 0.5 * bx[1] * (bx[1] - 1) * sp * sx * E[1][ax[1]][bx[1] - 2][0] * sz;
-                if (bx[2] >= 2) t -= 0.5 * bx[2] * (bx[2] - 1) * sp * sx * sy * E[2][ax[2]][bx[2] - 2][0];
-                dS += f * s0;
-                dT += f * t;
-              }
-              gST[d] += cc * (Dij * dT - Wij * dS);
-            }
-          }
-      }
-      // density-contracted Hermite coefficients of the bra (MA) and ket (MB) derivatives
-      const double pre = 2.0 * pi / p * cc;
-      for (int k = tid; k < 3 * NH; k += blockDim.x) {
-        const int d = k / NH, h = k % NH;
-        const int t = h / ((L + 1) * (L + 1)), u = (h / (L + 1)) % (L + 1), v = h % (L + 1);
-        double ma = 0.0, mb = 0.0;
-        if (t + u + v <= L) {
-          for (int i = 0; i < NA; ++i)
-            for (int j = 0; j < NB; ++j) {
-              const int ax0[3] = {cart_e(LA, i, 0), cart_e(LA, i, 1), cart_e(LA, i, 2)};
-              const int bx0[3] = {cart_e(LB, j, 0), cart_e(LB, j, 1), cart_e(LB, j, 2)};
-              double acca = 0.0, accb = 0.0;
-              for (int sgn = 0; sgn < 2; ++sgn) {
-                {
-                  int ax[3] = {ax0[0], ax0[1], ax0[2]};
-                  const int ad = ax[d];
-                  if (!(sgn == 1 && ad == 0)) {
-                    ax[d] += sgn == 0 ? 1 : -1;
-                    if (t <= ax[0] + bx0[0] && u <= ax[1] + bx0[1] && v <= ax[2] + bx0[2]) {
-                      const double f = sgn == 0 ? 2.0 * al : -(double)ad;
-                      acca += f * E[0][ax[0]][bx0[0]][t] * E[1][ax[1]][bx0[1]][u] * E[2][ax[2]][bx0[2]][v];
-                    }
-                  }
-                }
-                if (two) {
-                  int bx[3] = {bx0[0], bx0[1], bx0[2]};
-                  const int bd = bx[d];
-                  if (!(sgn == 1 && bd == 0)) {
-                    bx[d] += sgn == 0 ? 1 : -1;
-                    if (t <= ax0[0] + bx[0] && u <= ax0[1] + bx[1] && v <= ax0[2] + bx[2]) {
-                      const double f = sgn == 0 ? 2.0 * be : -(double)bd;
-                      accb += f * E[0][ax0[0]][bx[0]][t] * E[1][ax0[1]][bx[1]][u] * E[2][ax0[2]][bx[2]][v];
-                    }
-                  }
-                }
-              }
-              ma += Dab[i][j] * acca;
-              mb += Dab[i][j] * accb;
-            }
+  for (int off = 16; off > 0; off >>= 1) dw = fmaxf(dw, __shfl_xor_sync(0xffffffffu, dw, off));
+  const float R1 = sqrtf((float)((A[0] - B[0]) * (A[0] - B[0]) + (A[1] - B[1]) * (A[1] - B[1]) +
+                                 (A[2] - B[2]) * (A[2] - B[2])));
+  double gst[3] = {0.0, 0.0, 0.0}, gva[3] = {0.0, 0.0, 0.0}, gvp[3] = {0.0, 0.0, 0.0};
+  for (int i0 = 0; i0 < np; i0 += ngrp) {
+    const int ip = i0 + sub;
+    bool on = ip < np;
+    const double *rec = rec0 + (size_t)(on ? ip : 0) * kPrimRec;
+    const double p = rec[0], Pc[3] = {rec[1], rec[2], rec[3]}, kt = rec[4], hp = rec[5], al = rec[6], be = rec[7];
+    {
+      const float pf = (float)p, g = fabsf((float)kt) * 0.9414f * rsqrtf(pf) * dw;
+      const float x = R1 + rsqrtf(pf) + 1.0f, mx = (float)fmax(al, be);
+      float e = x;
+#pragma unroll
+      for (int k = 0; k < L; ++k) e *= x;
+      const float f = (2.0f * mx + L1) * (1.0f + 1.1284f * sqrtf(pf) * zs + 3.0f * mx * (LB + 2));
+      if (!(g * e * f >= 1e-15f)) on = false;
+    }
+    if (!__any_sync(0xffffffffu, on)) continue;
+    __syncwarp();   // the previous pass is done with the tables
+    const double ap = 2.0 * al * hp;   // alpha / p
+    if (on && l < 3) {
+      const double pa = l == 0 ? Pc[0] - A[0] : l == 1 ? Pc[1] - A[1] : Pc[2] - A[2];
+      const double pb = l == 0 ? Pc[0] - B[0] : l == 1 ? Pc[1] - B[1] : Pc[2] - B[2];
+      double Et[LA + 2][LB + 3][LA + LB + 4];
+      hermite_e<LA + 1, LB + 2>(hp, pa, pb, Et);
+      double kin[LA + 2][LB + 1];   // one-dimensional kinetic energy
+#pragma unroll
+      for (int i = 0; i <= LA + 1; ++i)
+#pragma unroll
+        for (int j = 0; j <= LB; ++j) {
+          double t = be * ((2 * j + 1) * Et[i][j][0] - 2.0 * be * Et[i][j + 2][0]);
+          if (j >= 2) t -= 0.5 * j * (j - 1) * Et[i][j - 2][0];
+          kin[i][j] = t;
         }
-        MA[d][h] = pre * ma;
-        MB[d][h] = pre * mb;
-      }
-      __syncthreads();
-      for (int at = tid; at < P.natom; at += blockDim.x) {
-        const double pc[3] = {Pc[0] - P.atom_xyz[3 * at], Pc[1] - P.atom_xyz[3 * at + 1],
-                              Pc[2] - P.atom_xyz[3 * at + 2]};
-        double F[L + 1];
-        {
-          double ur[NRT], wr[NRT];
-          rys_roots_f64_tab<NRT>(P.tab64, P.asym, p * (pc[0] * pc[0] + pc[1] * pc[1] + pc[2] * pc[2]), ur, wr);
-          double pw[NRT];
 #pragma unroll
-          for (int r = 0; r < NRT; ++r) pw[r] = wr[r];
+      for (int i = 0; i <= LA; ++i)
 #pragma unroll
-          for (int m = 0; m <= L; ++m) {
-            double f = 0.0;
+        for (int j = 0; j <= LB; ++j) {
+          s1[SF_IJ(l, i, j)] = Et[i][j][0];
+          k1[SF_IJ(l, i, j)] = kin[i][j];
+          ds[SF_IJ(l, i, j)] = 2.0 * al * Et[i + 1][j][0] - (i > 0 ? i * Et[i - 1][j][0] : 0.0);
+          dk[SF_IJ(l, i, j)] = 2.0 * al * kin[i + 1][j] - (i > 0 ? i * kin[i - 1][j] : 0.0);
 #pragma unroll
-            for (int r = 0; r < NRT; ++r) {
-              f += pw[r];
-              pw[r] *= ur[r];
-            }
-            F[m] = f;
+          for (int t = 0; t <= L; ++t) {
+            E[SF_ET(l, i, j, t)] = Et[i][j][t];
+            X[SF_ET(l, i, j, t)] = 2.0 * al * Et[i + 1][j][t] - (i > 0 ? i * Et[i - 1][j][t] : 0.0) -
+                                   (t > 0 ? ap * Et[i][j][t - 1] : 0.0);
           }
         }
-        // R^m_tuv by the Hermite Coulomb recursion, in place: level m
-        // overwrites t+u+w = L-m .. 1 from the top down (each entry needs
-        // level m+1 at t+u+w-1 and -2, not yet overwritten), then R^m_000
-        double R[L + 1][L + 1][L + 1];
-        double fm2p[L + 1];
-        fm2p[0] = 1.0;
-#pragma unroll
-        for (int m = 1; m <= L; ++m) fm2p[m] = fm2p[m - 1] * (-2.0 * p);
-        R[0][0][0] = F[L] * fm2p[L];
-#pragma unroll
-        for (int m = L - 1; m >= 0; --m) {
-#pragma unroll
-          for (int sl = L - m; sl >= 1; --sl)
-#pragma unroll
-            for (int t = 0; t <= sl; ++t)
-#pragma unroll
-              for (int u = 0; u <= sl - t; ++u) {
-                const int w = sl - t - u;
-                double r;
-                if (t > 0) r = (t > 1 ? (t - 1) * R[t - 2][u][w] : 0.0) + pc[0] * R[t - 1][u][w];
-                else if (u > 0) r = (u > 1 ? (u - 1) * R[t][u - 2][w] : 0.0) + pc[1] * R[t][u - 1][w];
-                else r = (w > 1 ? (w - 1) * R[t][u][w - 2] : 0.0) + pc[2] * R[t][u][w - 1];
-                R[t][u][w] = r;
-              }
-          R[0][0][0] = F[m] * fm2p[m];
-        }
-        double da[3] = {0.0, 0.0, 0.0}, db[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-        for (int t = 0; t <= L; ++t)
-#pragma unroll
-          for (int u = 0; u <= L - t; ++u)
-#pragma unroll
-            for (int w = 0; w <= L - t - u; ++w) {
-              const int h = (t * (L + 1) + u) * (L + 1) + w;
-              const double rr = R[t][u][w];
-#pragma unroll
-              for (int d = 0; d < 3; ++d) {
-                da[d] += MA[d][h] * rr;
-                db[d] += MB[d][h] * rr;
-              }
+    }
+    __syncwarp();
+    const double sp = kt * 0.941396263776714813 * rsqrt_nr(p), vp = kt * 1.06225193202719693;
+    if (on) {
+      // density-contracted Hermite coefficients, Hermite triples over the lanes
+      int k = 0;
+#pragma unroll 1
+      for (int t = 0; t <= L; ++t)
+#pragma unroll 1
+        for (int u = 0; u <= L - t; ++u)
+#pragma unroll 1
+          for (int v = 0; v <= L - t - u; ++v, ++k) {
+            if (k % G != l) continue;
+            double h = 0.0;
+            for (int o = 0; o < NA * NB; ++o) {
+              const int i = o / NB, j = o % NB;
+              const int ax = cart_e(LA, i, 0), ay = cart_e(LA, i, 1), az = cart_e(LA, i, 2);
+              const int bx = cart_e(LB, j, 0), by = cart_e(LB, j, 1), bz = cart_e(LB, j, 2);
+              if (t <= ax + bx && u <= ay + by && v <= az + bz)
+                h += Db[o] * E[SF_ET(0, ax, bx, t)] * (E[SF_ET(1, ay, by, u)] * E[SF_ET(2, az, bz, v)]);
             }
-        const double z = -P.charges[at];
-        for (int d = 0; d < 3; ++d) {
-          gVA[d] += z * da[d];
-          gVB[d] += z * db[d];
-          atomicAdd(grad + 3 * at + d, -2.0 * z * (da[d] + db[d]));
-        }
+            Ht[k] = vp * h;
+          }
+      // overlap and kinetic bra derivatives, entries over the lanes
+      for (int o = l; o < NA * NB; o += G) {
+        const int i = o / NB, j = o % NB;
+        const int x = SF_IJ(0, cart_e(LA, i, 0), cart_e(LB, j, 0)), y = SF_IJ(1, cart_e(LA, i, 1), cart_e(LB, j, 1)),
+                  z = SF_IJ(2, cart_e(LA, i, 2), cart_e(LB, j, 2));
+        const double d = sp * Db[o], w = sp * Wb[o];
+        const double sx = s1[x], sy = s1[y], sz = s1[z], kx = k1[x], ky = k1[y], kz = k1[z];
+        // D (k' s s + s' k s + s' s k) - W s' s s
+        const double dx = ds[x], dy = ds[y], dz = ds[z];
+        gst[0] += d * (dk[x] * sy * sz + dx * (ky * sz + sy * kz)) - w * dx * sy * sz;
+        gst[1] += d * (dk[y] * sx * sz + dy * (kx * sz + sx * kz)) - w * dy * sx * sz;
+        gst[2] += d * (dk[z] * sx * sy + dz * (kx * sy + sx * ky)) - w * dz * sx * sy;
       }
     }
-  // reduce over the CTA, one atomic per centre and direction
-  for (int d = 0; d < 3; ++d) {
-    red[tid][d] = gVA[d] + gST[d];
-    red[tid][3 + d] = gVB[d] - gST[d];
+    __syncwarp();
+    double st[NT], gp[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < NT; ++k) st[k] = 0.0;
+    for (int at = on ? l : P.natom; at < P.natom; at += G) {
+      const double pc[3] = {Pc[0] - P.atom_xyz[3 * at], Pc[1] - P.atom_xyz[3 * at + 1], Pc[2] - P.atom_xyz[3 * at + 2]};
+      double F[L1 + 1];
+      boys_table<L1>(P.boys, p * (pc[0] * pc[0] + pc[1] * pc[1] + pc[2] * pc[2]), F);
+      double R[L1 + 1][L1 + 1][L1 + 1];
+      hermite_r<L1>(p, pc, F, R);
+      double q[3] = {0.0, 0.0, 0.0};
+      const double z = P.charges[at];
+#pragma unroll
+      for (int t = 0; t <= L; ++t)
+#pragma unroll
+        for (int u = 0; u <= L - t; ++u)
+#pragma unroll
+          for (int v = 0; v <= L - t - u; ++v) {
+            const int k = tuv_index(L, t, u, v);
+            const double h = Ht[k];
+            q[0] += h * R[t + 1][u][v];
+            q[1] += h * R[t][u + 1][v];
+            q[2] += h * R[t][u][v + 1];
+            st[k] -= z * R[t][u][v];
+          }
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        q[d] *= z;
+        gp[d] -= q[d];
+        if (frc) frc[sub * fstride + 3 * at + d] += q[d];
+        else atomicAdd(grad + 3 * at + d, q[d]);
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      gvp[d] += gp[d];
+      gva[d] += ap * gp[d];
+    }
+    for (int off = 1; off < G; off <<= 1) {
+#pragma unroll
+      for (int k = 0; k < NT; ++k) st[k] += __shfl_xor_sync(0xffffffffu, st[k], off);
+    }
+    if (l == 0) {
+#pragma unroll
+      for (int k = 0; k < NT; ++k) St[k] = vp * st[k];
+    }
+    __syncwarp();
+    if (on) {
+      for (int o = l; o < NA * NB; o += G) {
+        const int i = o / NB, j = o % NB;
+        const int ax = cart_e(LA, i, 0), ay = cart_e(LA, i, 1), az = cart_e(LA, i, 2);
+        const int bx = cart_e(LB, j, 0), by = cart_e(LB, j, 1), bz = cart_e(LB, j, 2);
+        const double *ex = E + SF_ET(0, ax, bx, 0), *ey = E + SF_ET(1, ay, by, 0), *ez = E + SF_ET(2, az, bz, 0);
+        const double *xx = X + SF_ET(0, ax, bx, 0), *xy = X + SF_ET(1, ay, by, 0), *xz = X + SF_ET(2, az, bz, 0);
+        double vx = 0.0, vy = 0.0, vz = 0.0;
+        for (int t = 0; t <= ax + bx; ++t) {
+          double e0 = 0.0, ey1 = 0.0, ez1 = 0.0;   // E_u E_v S, dE_u E_v S, E_u dE_v S
+          for (int u = 0; u <= ay + by; ++u) {
+            double c = 0.0, cz = 0.0;
+            for (int v = 0; v <= az + bz; ++v) {
+              const double sv = St[tuv_index(L, t, u, v)];
+              c += ez[v] * sv;
+              cz += xz[v] * sv;
+            }
+            e0 += ey[u] * c;
+            ey1 += xy[u] * c;
+            ez1 += ey[u] * cz;
+          }
+          vx += xx[t] * e0;
+          vy += ex[t] * ey1;
+          vz += ex[t] * ez1;
+        }
+        gva[0] += Db[o] * vx;
+        gva[1] += Db[o] * vy;
+        gva[2] += Db[o] * vz;
+      }
+    }
   }
+#undef SF_IJ
+#undef SF_ET
+  for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      gst[d] += __shfl_xor_sync(0xffffffffu, gst[d], off);
+      gva[d] += __shfl_xor_sync(0xffffffffu, gva[d], off);
+      gvp[d] += __shfl_xor_sync(0xffffffffu, gvp[d], off);
+    }
+  }
+  __syncwarp();
+  if (lane < 3) {
+    const double s = lane == 0 ? gst[0] : lane == 1 ? gst[1] : gst[2];
+    const double va = lane == 0 ? gva[0] : lane == 1 ? gva[1] : gva[2];
+    const double vp = lane == 0 ? gvp[0] : lane == 1 ? gvp[1] : gvp[2];
+    const int ia = 3 * P.sh.atom[a] + lane, ib = 3 * P.sh.atom[b] + lane;
+    if (frc) {
+      frc[ia] += s + va;
+      frc[ib] += vp - va - s;
+    } else {
+      atomicAdd(grad + ia, s + va);
+      atomicAdd(grad + ib, vp - va - s);
+    }
+  }
+  __syncwarp();
+}
+
+// warps stride over the pairs in the order dd, dp, ds, pp, ps, ss (the long
+// ones first)
+__global__ void __launch_bounds__(kOneGradWarps * 32, 4) one_electron_grad_kernel(OneParams P, const double *D,
+                                                                                 const double *W, double *grad) {
+  extern __shared__ __align__(16) double sm_grad[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double *tab = sm_grad + warp * kOneGradWarp;
+  const int fstride = 3 * P.natom;
+  double *frc = P.natom <= kOneGradAtoms ? sm_grad + kOneGradWarps * kOneGradWarp + warp * 4 * fstride : nullptr;
+  if (frc)
+    for (int k = lane; k < 4 * fstride; k += 32) frc[k] = 0.0;
+  float zs = 0.0f;
+  for (int k = lane; k < P.natom; k += 32) zs += fabsf((float)P.charges[k]);
+  for (int off = 16; off > 0; off >>= 1) zs += __shfl_xor_sync(0xffffffffu, zs, off);
+  __syncwarp();
+  const int npair = P.cstart[kNumPairClass];
+  for (int k = blockIdx.x * kOneGradWarps + warp; k < npair; k += gridDim.x * kOneGradWarps) {
+    const int pair = npair - 1 - k;
+    int cls = 0;
+    while (pair >= P.cstart[cls + 1]) ++cls;
+    switch (cls) {
+      case 0: one_pair_grad<0, 0>(P, D, W, frc, fstride, grad, pair, tab, zs, lane); break;
+      case 1: one_pair_grad<1, 0>(P, D, W, frc, fstride, grad, pair, tab, zs, lane); break;
+      case 2: one_pair_grad<1, 1>(P, D, W, frc, fstride, grad, pair, tab, zs, lane); break;
+      case 3: one_pair_grad<2, 0>(P, D, W, frc, fstride, grad, pair, tab, zs, lane); break;
+      case 4: one_pair_grad<2, 1>(P, D, W, frc, fstride, grad, pair, tab, zs, lane); break;
+      default: one_pair_grad<2, 2>(P, D, W, frc, fstride, grad, pair, tab, zs, lane); break;
+    }
+  }
+  if (!frc) return;
   __syncthreads();
-  if (tid < 6) {
-    double sacc = 0.0;
-    for (int k = 0; k < (int)blockDim.x; ++k) sacc += red[k][tid];
-    if (tid < 3) atomicAdd(grad + 3 * P.sh.atom[a] + tid, 2.0 * sacc);
-    else if (two) atomicAdd(grad + 3 * P.sh.atom[b] + tid - 3, 2.0 * sacc);
+  // the CTA's warps and groups, one atomic per word
+  const double *f = sm_grad + kOneGradWarps * kOneGradWarp;
+  for (int k = threadIdx.x; k < fstride; k += blockDim.x) {
+    double s = 0.0;
+#pragma unroll
+    for (int g = 0; g < 4 * kOneGradWarps; ++g) s += f[g * fstride + k];
+    if (s != 0.0) atomicAdd(grad + k, s);
   }
 }
 
-// one CTA per canonical pair (a >= b): block k = a (a + 1) / 2 + b
-__global__ void __launch_bounds__(kOneGradThreads) one_electron_grad_kernel(OneParams P, const double *D,
-                                                                            const double *W, double *grad) {
-  const int k = blockIdx.x;
-  int a = (int)((sqrt(8.0 * k + 1.0) - 1.0) * 0.5);
-  while (a * (a + 1) / 2 > k) --a;
-  while ((a + 1) * (a + 2) / 2 <= k) ++a;
-  const int b = k - a * (a + 1) / 2;
-  __shared__ __align__(16) double smem[kOneGradSmem];
-  switch (P.sh.l[a] * 3 + P.sh.l[b]) {
-    case 0: one_pair_grad2<0, 0>(P, D, W, grad, a, b, smem); break;
-    case 1: one_pair_grad2<0, 1>(P, D, W, grad, a, b, smem); break;
-    case 2: one_pair_grad2<0, 2>(P, D, W, grad, a, b, smem); break;
-    case 3: one_pair_grad2<1, 0>(P, D, W, grad, a, b, smem); break;
-    case 4: one_pair_grad2<1, 1>(P, D, W, grad, a, b, smem); break;
-    case 5: one_pair_grad2<1, 2>(P, D, W, grad, a, b, smem); break;
-    case 6: one_pair_grad2<2, 0>(P, D, W, grad, a, b, smem); break;
-    case 7: one_pair_grad2<2, 1>(P, D, W, grad, a, b, smem); break;
-    case 8: one_pair_grad2<2, 2>(P, D, W, grad, a, b, smem); break;
-    default: break;
-  }
+static size_t one_grad_smem(int natom) {
+  const size_t f = natom <= kOneGradAtoms ? (size_t)kOneGradWarps * 4 * 3 * natom : 0;
+  return (kOneGradWarps * (size_t)kOneGradWarp + f) * sizeof(double);
 }
 
-cudaError_t launch_one_electron_grad(const OneParams &P, const double *D, const double *W, double *grad,
+cudaError_t prepare_one_electron() {
+  return cudaFuncSetAttribute(one_electron_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)one_grad_smem(kOneGradAtoms));
+}
+
+cudaError_t launch_one_electron_grad(const OneParams &P, const double *D, const double *W, double *grad, int nsm,
                                      cudaStream_t st) {
-  const int n = P.nshell * (P.nshell + 1) / 2;
-  if (n == 0) return cudaSuccess;
-  one_electron_grad_kernel<<<n, kOneGradThreads, 0, st>>>(P, D, W, grad);
+  const int npair = P.cstart[kNumPairClass];
+  if (npair == 0) return cudaSuccess;
+  const int ctas = (npair + kOneGradWarps - 1) / kOneGradWarps, most = (nsm < 1 ? 1 : nsm) * 4;
+  one_electron_grad_kernel<<<ctas < most ? ctas : most, kOneGradWarps * 32, one_grad_smem(P.natom), st>>>(P, D, W, grad);
   return cudaGetLastError();
 }
 
