@@ -9,16 +9,16 @@ template <int LA, int LB, int LC, int LD, typename R, int T>
 static cudaError_t run_eri(const KParams &kp, const EriWork &w, cudaStream_t st) {
   if (w.n <= 0) return cudaSuccess;
   const int P = w.psplit < 1 ? 1 : w.psplit;
-  if (T * P > 32 || (P & (P - 1))) return cudaErrorInvalidValue;
+  const bool cta = w.csplit > 1;   // a CTA per quartet
+  if (T * P > 32 || (P & (P - 1)) || (cta && (T * P != 32 || w.csplit != kEriWarps))) return cudaErrorInvalidValue;
   EriWork w2 = w;
   w2.psplit = P;
-  const int G = kBlock / (T * P);
-  size_t smem = grp_smem<LA, LB, LC, LD, R, T>();
+  const int G = cta ? 1 : kBlock / (T * P);
+  size_t smem = grp_smem<LA, LB, LC, LD, R, T>() + eri_tab_smem<LA, LB, LC, LD, R, T>();
+  if (T == 1 && cta) smem += (size_t)kEriWarps * QC<LA, LB, LC, LD>::NABCD * sizeof(R);
   int64_t grid = (w.n + G - 1) / G;
-  if (T == 1 && std::is_same<R, float>::value) {   // Rys table block in shared memory, grid-stride
-    smem = (size_t)kTabNint * QC<LA, LB, LC, LD>::NR * kTab32Row * sizeof(float);
-    grid = std::min<int64_t>(grid, (int64_t)std::max(kp.nsm, 1) * 16);
-  }
+  // Rys table block in shared memory: grid-stride
+  if (T == 1 && std::is_same<R, float>::value) grid = std::min<int64_t>(grid, (int64_t)std::max(kp.nsm, 1) * 16);
   eri_kernel<LA, LB, LC, LD, R, T><<<(unsigned)grid, kBlock, smem, st>>>(kp, w2);
   return cudaGetLastError();
 }

@@ -9,11 +9,13 @@ template <int LA, int LB, int LC, int LD, int T>
 static cudaError_t run_eri_dd(const KParams &kp, const EriWork &w, cudaStream_t st) {
   if (w.n <= 0) return cudaSuccess;
   const int P = w.psplit < 1 ? 1 : w.psplit;
-  if (T * P > 32 || (P & (P - 1))) return cudaErrorInvalidValue;
+  const bool cta = w.csplit > 1;   // a CTA per quartet
+  if (T * P > 32 || (P & (P - 1)) || (cta && (T * P != 32 || w.csplit != kEriWarps))) return cudaErrorInvalidValue;
   EriWork w2 = w;
   w2.psplit = P;
-  const int G = kBlock / (T * P);
-  constexpr size_t smem = grp_smem<LA, LB, LC, LD, dd, T>();
+  const int G = cta ? 1 : kBlock / (T * P);
+  const size_t smem = grp_smem<LA, LB, LC, LD, dd, T>() +
+                      (T == 1 && cta ? (size_t)kEriWarps * QC<LA, LB, LC, LD>::NABCD * sizeof(dd) : 0);
   eri_kernel<LA, LB, LC, LD, dd, T><<<(unsigned)((w.n + G - 1) / G), kBlock, smem, st>>>(kp, w2);
   return cudaGetLastError();
 }

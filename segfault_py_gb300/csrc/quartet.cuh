@@ -1449,7 +1449,9 @@ struct EriWork {
   int64_t n;
   double *out;
   int psplit;                  // P primitive sub-groups per quartet (T*P <= 32)
+  int csplit = 1;              // kEriWarps: the four warps of a CTA share a quartet (T*P == 32), else 1
 };
+constexpr int kEriWarps = kBlock / 32;
 
 // one quartet of the one-lane (T == 1) raw-integral path: P lanes share it
 template <int LA, int LB, int LC, int LD, typename R>
@@ -1467,6 +1469,29 @@ __device__ __forceinline__ void eri_t1_quartet(const KParams &kp, const EriWork 
 #pragma unroll
   for (int o = 0; o < Q::NABCD; ++o)
     out[Q::ca(o) * s0 + Q::cb(o) * s1 + Q::cc(o) * s2 + Q::cd(o) * s3] = to_f64(acc[o] * (R)Q::norm(o));
+}
+
+// sum of a quartet's partial integrals over the CTA's warps (buf: warp c's
+// NABCD values at c * stride) and store
+template <int LA, int LB, int LC, int LD, typename R>
+__device__ __forceinline__ void eri_store_cta(const EriWork &w, int64_t q, const R *buf, int stride) {
+  using Q = QC<LA, LB, LC, LD>;
+  const int s0 = w.strides[4 * q], s1 = w.strides[4 * q + 1], s2 = w.strides[4 * q + 2], s3 = w.strides[4 * q + 3];
+  double *out = w.out + w.out_off[q];
+  for (int o = threadIdx.x; o < Q::NABCD; o += kBlock) {
+    R v = buf[o];
+#pragma unroll
+    for (int c = 1; c < kEriWarps; ++c) v += buf[c * stride + o];
+    out[Q::ca(o) * s0 + Q::cb(o) * s1 + Q::cc(o) * s2 + Q::cd(o) * s3] = to_f64(v * (R)Q::norm(o));
+  }
+}
+
+// dynamic shared memory: FP32 one-lane kernels the Rys table block, group
+// kernels the group buffers; then, one-lane kernels, the warps' partial sums
+template <int LA, int LB, int LC, int LD, typename R, int T>
+constexpr size_t eri_tab_smem() {
+  return T == 1 && std::is_same<R, float>::value ? (size_t)kTabNint * QC<LA, LB, LC, LD>::NR * kTab32Row * sizeof(float)
+                                                 : 0;
 }
 
 template <int LA, int LB, int LC, int LD, typename R, int T>
@@ -1488,11 +1513,31 @@ __global__ void __launch_bounds__(kBlock) eri_kernel(KParams kp, EriWork w) {
       __syncthreads();
       tab_s = reinterpret_cast<const float *>(smem_t);
     }
+    if (w.csplit > 1) {   // one quartet per CTA trip
+      extern __shared__ __align__(16) unsigned char smem_t[];
+      R *red = reinterpret_cast<R *>(smem_t + eri_tab_smem<LA, LB, LC, LD, R, T>());
+      for (int64_t q = blockIdx.x; q < w.n; q += gridDim.x) {
+        const int fl = w.flags[q];
+        const QGeom<R> g = make_geom<R>(kp, w.pab[q], w.pcd[q], fl & 1, fl & 2);
+        R acc[Q::NABCD];
+        eval_t1<LA, LB, LC, LD, R>(kp, g, acc, threadIdx.x, kBlock, tab_s);
+        reduce_psplit<R, Q::NABCD, 1>(acc, 32, 0xffffffffu);
+        if (lane == 0) {
+#pragma unroll
+          for (int o = 0; o < Q::NABCD; ++o) red[(threadIdx.x >> 5) * Q::NABCD + o] = acc[o];
+        }
+        __syncthreads();
+        eri_store_cta<LA, LB, LC, LD, R>(w, q, red, Q::NABCD);
+        __syncthreads();   // red is written again in the next trip
+      }
+      return;
+    }
     const int64_t stride = (int64_t)gridDim.x * (kBlock / TP);
     for (int64_t q = (int64_t)blockIdx.x * (kBlock / TP) + grp; q < w.n; q += stride)
       eri_t1_quartet<LA, LB, LC, LD, R>(kp, w, q, p, P, qmask, tab_s);
   } else {
-    const int64_t q = (int64_t)blockIdx.x * (kBlock / TP) + grp;
+    const int C = w.csplit;
+    const int64_t q = C > 1 ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * (kBlock / TP) + grp;
     if (q >= w.n) return;
     const int fl = w.flags[q];
     const QGeom<R> g = make_geom<R>(kp, w.pab[q], w.pcd[q], fl & 1, fl & 2);
@@ -1503,8 +1548,20 @@ __global__ void __launch_bounds__(kBlock) eri_kernel(KParams kp, EriWork w) {
     R *buf = reinterpret_cast<R *>(smem_raw) + (threadIdx.x / T) * GP::BUFN;
     const unsigned gmask = (T == 32) ? 0xffffffffu : (((1u << T) - 1u) << (lane & ~(T - 1)));
     R acc[GP::NPER];
-    eval_grp<LA, LB, LC, LD, R, T>(kp, g, buf, t, gmask, acc, p, P);
+    eval_grp<LA, LB, LC, LD, R, T>(kp, g, buf, t, gmask, acc, C > 1 ? grp * P + p : p, C * P);
     if (P > 1) reduce_psplit<R, GP::NPER, T>(acc, P, qmask);
+    if (C > 1) {   // the warps' sums through the buffers of their first groups
+      if (p == 0) {
+#pragma unroll
+        for (int k = 0; k < GP::NPER; ++k) {
+          const int o = GP::out(t, k);
+          if (o < Q::NABCD) buf[o] = acc[k];
+        }
+      }
+      __syncthreads();
+      eri_store_cta<LA, LB, LC, LD, R>(w, q, reinterpret_cast<const R *>(smem_raw), (32 / T) * GP::BUFN);
+      return;
+    }
     if (p != 0) return;
 #pragma unroll
     for (int k = 0; k < GP::NPER; ++k) {
