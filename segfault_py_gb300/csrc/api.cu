@@ -77,6 +77,8 @@ struct HostTables {
   std::vector<float> t32, t32v;   // t32v: the FP32 kernels' layout (sf_internal.h)
   std::vector<float4> tdd;         // the fine table as dd rows (sf_internal.h)
   std::vector<double> boys;        // Boys functions (sf_internal.h)
+  std::vector<uint2> gtab;         // gradient work tables (grad.cuh)
+  std::vector<int2> ghdr;
   RysAsym asym;
   RysAsym32 asym32;
 };
@@ -95,6 +97,7 @@ const HostTables &host_tables() {
     T.t32.assign(rys_tab_size(kTabDeg32), 0.0f);
     std::memset(&T.asym, 0, sizeof(T.asym));
     rys_build_tables(T.t64.data(), T.t32.data(), &T.asym);
+    grad_tables(T.gtab, T.ghdr);
     T.boys.assign(kBoysTab, 0.0);
     boys_build_table(T.boys.data());
     std::vector<double> fine(rys_fine_size());
@@ -343,6 +346,8 @@ struct sf_handle {
   DBuf<float> d_Ddd;               // density as dd (per build)
   DBuf<float> d_cx32, d_cy32, d_cz32;
   DBuf<double> d_tab64, d_boys;
+  DBuf<uint2> d_gtab;
+  DBuf<int2> d_ghdr;
   DBuf<float> d_tab32;
   DBuf<double> d_Jh, d_Kh;
   DBuf<float> d_D32;
@@ -452,6 +457,8 @@ void fill_kparams(sf_handle *h) {
   k.pdd = DevPrims<dd>{reinterpret_cast<const dd *>(h->d_ppdd.p)};
   k.pair32 = h->d_pair32.p;
   k.pair32f = h->d_pair32f.p;
+  k.grad_tab = h->d_gtab.p;
+  k.grad_hdr = h->d_ghdr.p;
   k.cxd = reinterpret_cast<const dd *>(h->d_cdd.p);
   k.cyd = k.cxd + h->nshell;
   k.czd = k.cyd + h->nshell;
@@ -1574,6 +1581,8 @@ int sf_create(const sf_shell_desc *shells, int32_t nshell, sf_handle **out) {
   const HostTables &T = host_tables();
   SF_CK(h->d_tab64.upload(T.t64));
   SF_CK(h->d_boys.upload(T.boys));
+  SF_CK(h->d_gtab.upload(T.gtab));
+  SF_CK(h->d_ghdr.upload(T.ghdr));
   SF_CK(h->d_tab32.upload(T.t32v));
   SF_CK(h->d_tabdd.upload(T.tdd));
   SF_CK(h->d_Ddd.alloc(2 * (size_t)nao * nao));

@@ -29,6 +29,24 @@ cudaError_t launch_grad_f32(int cls, const KParams &kp, const ClassWork *w, int 
   }
 }
 
+// work tables of every class for the FP64 / double-float and the FP32 lanes
+void grad_tables(std::vector<uint2> &tab, std::vector<int2> &hdr) {
+  tab.clear();
+  hdr.assign(2 * kNumClass * 3, make_int2(0, 0));
+#define SF_TAB(id, la, lb, lc, ld, t64, t32)                                     \
+  for (int f = 0; f < 2; ++f) {                                                  \
+    constexpr int N = QC<la, lb, lc, ld>::NABCD;                                 \
+    const int T = f ? tgrad_r<float>(N) : tgrad(N);                              \
+    int2 h[3];                                                                   \
+    if (T > 1) {                                                                 \
+      grad_table<la, lb, lc, ld>(T, tab, h);                                     \
+      for (int d = 0; d < 3; ++d) hdr[(2 * id + f) * 3 + d] = h[d];              \
+    }                                                                            \
+  }
+  SF_CLASS_LIST(SF_TAB)
+#undef SF_TAB
+}
+
 cudaError_t prepare_grad_f32() {
   cudaError_t e = cudaSuccess;
 #define SF_PREP(id, la, lb, lc, ld, t64, t32)                                                               \

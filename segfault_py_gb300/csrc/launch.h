@@ -1,5 +1,7 @@
 // launch.h -- host-side launchers implemented in the kernel translation units.
 #pragma once
+#include <vector>
+
 #include "quartet.cuh"
 
 namespace sf {
@@ -51,6 +53,7 @@ cudaError_t launch_grad_f32(int cls, const KParams &kp, const ClassWork *w, int 
                             cudaStream_t st);
 cudaError_t launch_grad_dd(int cls, const KParams &kp, const ClassWork *w, int nw, const dd *D, double *grad,
                            cudaStream_t st);
+void grad_tables(std::vector<uint2> &tab, std::vector<int2> &hdr);
 cudaError_t prepare_grad_f64();
 cudaError_t prepare_grad_dd();
 cudaError_t prepare_grad_f32();

@@ -53,6 +53,8 @@ struct KParams {
   const dd *cxd, *cyd, *czd;
   const float4 *tabdd;
   dd asymdd_r[kMaxRoots + 1][kMaxRoots], asymdd_w[kMaxRoots + 1][kMaxRoots];
+  const uint2 *grad_tab;   // work tables of the gradient's group kernels (grad.cuh)
+  const int2 *grad_hdr;
   int nao;
   int nsm;             // multiprocessors (grid sizing of the grid-stride kernels)
   int natom;           // atoms referenced by the shells (gradient length / 3)
