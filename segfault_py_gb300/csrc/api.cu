@@ -583,6 +583,7 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     int psplit, wsplit;
     int64_t cost_hi;
     int wide, tail;
+    float rel_load;
   };
   std::vector<Pending> pend;
   h->st_q[0] = h->st_q[1] = h->st_pq[0] = h->st_pq[1] = 0;
@@ -596,6 +597,8 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     std::vector<Pending> segs;
     int64_t q = 0, pq = 0;
     double f = 0.0;
+    Pending head{};             // the list as one segment, before it is split
+    double per_prim = 0.0, load = 0.0;   // estimated operations: of a primitive quartet, of the list
   };
   std::vector<Part> parts(3 * kNumClass);   // per class: accurate tier, FP32, double-float part of FP64
   std::vector<int64_t> totals(kNumClass, 0);
@@ -665,9 +668,11 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
       });
       std::vector<int64_t> pos((size_t)KB * KB, 0);
       int64_t run = 0;
+      double costs = 0.0;
       for (int k : keys) {
         pos[k] = run;
         run += hist[k];
+        costs += (double)hist[k] * (k / KB) * (k % KB);
       }
       std::vector<int2> lst(n);
       for (int i = 0; i < nX; ++i) {
@@ -701,57 +706,79 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
       part.q = p.n;
       part.pq = p.prims;
       part.f = p.flops;
-      // split the cost-sorted list into launches with P primitive sub-groups
-      // per quartet: heavy quartets (many primitive quartets) get more lanes
-      const int T = kind_lanes(ci, kind, p.wide);
-      const int pmax = 32 / T;
-      auto psplit = [&](int64_t cost) {
-        if (pmax > 1 && cost >= 4 * pmax) return pmax;
-        if (pmax > 8 && cost >= 32) return 8;
-        return 1;
-      };
-      // a list with fewer lanes than 8 resident warps per SM sub-partition
-      // leaves most of the GPU idle and runs at the latency of one warp's
-      // instruction stream (an FP64 instruction of one warp occupies its
-      // sub-partition's FP64 unit for 64 cycles): its quartets' primitive
-      // loops are split further, up to S_fill = P*W sub-groups per quartet,
-      // each sub-group keeping at least one primitive quartet
-      const int fx4 = (pr == 0 && h->fill_acc_x4[prec] >= 0) ? h->fill_acc_x4[prec] : h->fill_x4[prec];
-      const int64_t fill = (int64_t)std::max(h->nsm, 1) * 4 * 8 * 32 * fx4 / 4;
-      int sfill = 1;
-      while (p.n * T * sfill < fill && sfill < pmax * kMaxWsplit) sfill *= 2;
-      auto split_of = [&](int64_t cost) {
-        int sc = 1;
-        while (2 * sc <= cost && 2 * sc <= sfill) sc *= 2;
-        return std::max(psplit(cost), sc);
-      };
-      int64_t q0 = 0;
-      while (q0 < p.n) {
-        const auto cost_of = [&](int64_t q) {
-          return (int64_t)npair(x0 + lst[q].x) * npair(y0 + lst[q].y);
-        };
-        const int S = split_of(cost_of(q0));
-        int64_t q1 = q0 + 1;
-        while (q1 < p.n && split_of(cost_of(q1)) == S) ++q1;
-        Pending seg = p;
-        seg.off = q0;
-        seg.n = q1 - q0;
-        seg.cost_hi = cost_of(q0);
-        int St = S;
-        for (const sf_tune_entry &e : h->tune)
-          if (!p.tail && e.cls == cls && e.precision == kind && e.cost == seg.cost_hi) St = e.split;
-        seg.psplit = std::min(St, pmax);
-        seg.wsplit = std::max(1, std::min(St / seg.psplit, kMaxWsplit));
-        int64_t sp = 0;
-        for (int64_t q = q0; q < q1; ++q) sp += (int64_t)h->pair_full(x0 + lst[q].x) * h->pair_full(y0 + lst[q].y);
-        seg.prims = sp;
-        seg.flops = (double)sp * nr * 4.0 * nabcd + 12.0 * nabcd * (double)seg.n;
-        part.segs.push_back(seg);
-        q0 = q1;
-      }
+      part.head = p;
+      part.per_prim = nr * (nabcd + 30.0) + 40.0;
+      part.load = costs * frac * part.per_prim;
       part.lst = std::move(lst);
     }
+  };
+  // Cut the cost-sorted list of (class, tier) into segments with S = P*W
+  // primitive sub-groups per quartet.  Heavy quartets (many primitive quartets)
+  // get the lanes of a warp in any case (psplit).  Beyond that:
+  //  * accurate tiers: S grows until a sub-group's estimated work is at most the
+  //    average load of the lanes that fill the GPU (8 warps per SM sub-partition)
+  //    over all lists of the same arithmetic, each sub-group keeping at least
+  //    one primitive quartet.  Long quartets then end with the rest of the
+  //    build, and no list is split further than that (with 8 warps per
+  //    sub-partition from every list: hexane 6-31G* double-float 2.48 ms, 1.98
+  //    here; (H2O)4 FP64 1.23, 0.89; (H2O)8 FP32 + double-float 1.35, 1.21)
+  //  * FP32: S grows until the list by itself has 8 warps per sub-partition (its
+  //    rounding depends on S, so it keeps this rule).
+  auto segment = [&](int cls, int pr, const double *load) {
+    Part &part = parts[3 * cls + pr];
+    const Pending &p = part.head;
+    if (part.lst.empty()) return;
+    const std::vector<int2> &lst = part.lst;
+    const ClassInfo &ci = kClassInfo[cls];
+    const int x0 = p.x0, y0 = p.y0, kind = p.prec;
+    const int nr = (ci.la + ci.lb + ci.lc + ci.ld) / 2 + 1;
+    const double nabcd = (double)ncart(ci.la) * ncart(ci.lb) * ncart(ci.lc) * ncart(ci.ld);
+    auto npair = [&](int i) { return pr == 1 ? h->pair_full(i) : h->pnp[i]; };
+    const int T = kind_lanes(ci, kind, p.wide);
+    const int pmax = 32 / T;
+    auto psplit = [&](int64_t cost) {
+      if (pmax > 1 && cost >= 4 * pmax) return pmax;
+      if (pmax > 8 && cost >= 32) return 8;
+      return 1;
     };
+    const int fx4 = (pr == 0 && h->fill_acc_x4[prec] >= 0) ? h->fill_acc_x4[prec] : h->fill_x4[prec];
+    const double lanes = (double)std::max(h->nsm, 1) * 4 * 8 * 32 * fx4 / 4.0;
+    int sfill = pmax * kMaxWsplit;
+    double share = 0.0;   // work of a sub-group above which it is split further
+    if (pr == 1) {
+      for (sfill = 1; (double)p.n * T * sfill < lanes && sfill < pmax * kMaxWsplit;) sfill *= 2;
+    } else {
+      share = lanes > 0.0 ? load[kind] / lanes : 1e300;
+    }
+    auto split_of = [&](int64_t cost) {
+      int sc = 1;
+      while (2 * sc <= cost && 2 * sc <= sfill && (double)cost * part.per_prim / T > share * sc) sc *= 2;
+      return std::max(psplit(cost), sc);
+    };
+    const auto cost_of = [&](int64_t q) { return (int64_t)npair(x0 + lst[q].x) * npair(y0 + lst[q].y); };
+    int64_t q0 = 0;
+    while (q0 < p.n) {
+      const int S = split_of(cost_of(q0));
+      int64_t q1 = q0 + 1;
+      while (q1 < p.n && split_of(cost_of(q1)) == S) ++q1;
+      Pending seg = p;
+      seg.off = q0;
+      seg.n = q1 - q0;
+      seg.cost_hi = cost_of(q0);
+      seg.rel_load = load[kind] > 0.0 ? (float)(part.per_prim * lanes / load[kind]) : 0.0f;
+      int St = S;
+      for (const sf_tune_entry &e : h->tune)
+        if (!p.tail && e.cls == cls && e.precision == kind && e.cost == seg.cost_hi) St = e.split;
+      seg.psplit = std::min(St, pmax);
+      seg.wsplit = std::max(1, std::min(St / seg.psplit, kMaxWsplit));
+      int64_t sp = 0;
+      for (int64_t q = q0; q < q1; ++q) sp += (int64_t)h->pair_full(x0 + lst[q].x) * h->pair_full(y0 + lst[q].y);
+      seg.prims = sp;
+      seg.flops = (double)sp * nr * 4.0 * nabcd + 12.0 * nabcd * (double)seg.n;
+      part.segs.push_back(seg);
+      q0 = q1;
+    }
+  };
   {
     const unsigned hw = std::thread::hardware_concurrency();
     const int nthr = std::max(1, std::min<int>(kNumClass, hw ? (int)hw : 1));
@@ -763,6 +790,16 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     std::vector<std::thread> pool;
     for (int t = 1; t < nthr; ++t) pool.emplace_back(worker);
     worker();
+    for (auto &t : pool) t.join();
+    double load[3] = {0.0, 0.0, 0.0};   // per arithmetic
+    for (const Part &part : parts) load[part.head.prec] += part.load;
+    next = 0;
+    auto cut = [&]() {
+      for (int c = next++; c < 3 * kNumClass; c = next++) segment(c / 3, c % 3, load);
+    };
+    pool.clear();
+    for (int t = 1; t < nthr; ++t) pool.emplace_back(cut);
+    cut();
     for (auto &t : pool) t.join();
   }
   for (int cls = 0; cls < kNumClass; ++cls) {
@@ -792,6 +829,7 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     w.wsplit = p.wsplit;
     w.max_cost = (int)std::max<int64_t>(p.cost_hi, 1);
     w.wide = p.wide;
+    w.rel_load = p.rel_load;
     h->slices.push_back({p.cls, p.prec, w, p.n, p.prims, p.flops, p.cost_hi, p.tail});
   }
   // greedy longest-processing-time assignment of slices to side streams;

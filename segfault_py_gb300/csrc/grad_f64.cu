@@ -11,7 +11,7 @@ template <int LA, int LB, int LC, int LD>
 static cudaError_t run_grad64(const KParams &kp, const ClassWork *w, int nw, const double *D, double *grad, cudaStream_t st) {
   constexpr int T = tgrad(QC<LA, LB, LC, LD>::NABCD);
   ClassMulti m;
-  if (!grad_segments(m, w, nw, T, kp.nsm)) return cudaErrorInvalidValue;
+  if (!grad_segments(m, w, nw, T)) return cudaErrorInvalidValue;
   if (m.n == 0) return cudaSuccess;
   constexpr size_t smem = grad_smem<LA, LB, LC, LD, double>();
   grad_kernel<LA, LB, LC, LD, double, T><<<(unsigned)m.cta0[m.n], kBlock, smem, st>>>(kp, m, D, grad);
