@@ -223,7 +223,7 @@ void sf_fock_graph_destroy(sf_fock_graph *g);
 /* How a Fock build launches its class kernels (no counterpart in the
  * reference, whose scheduler is Pool(8).map over AO quartets, hf.py:45-47):
  *  - SF_LAUNCH_STREAMS (default): one launch per (class, precision, primitive
- *    split) slice, spread over 16 side streams forked from the caller's
+ *    split) slice, spread over up to 32 side streams forked from the caller's
  *    stream and joined back;
  *  - SF_LAUNCH_PERSISTENT: the FP32 register-path classes run as one
  *    persistent launch per register tier (four tiers of similar register

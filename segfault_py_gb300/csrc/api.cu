@@ -176,19 +176,23 @@ __global__ void symmetrize_kernel(const double *Jh, const double *Kh, double *J,
   K[idx] = Kh[idx] + Kh[t];
 }
 
-__global__ void to_float_kernel(const double *D, float *Df, int64_t n) {
+// What a Fock build needs before its class launches, in one launch (as two
+// memsets and two conversions it was a chain of four, 2 to 3 us each in front
+// of a small build: (H2O)3 STO-3G FP32 + double-float replayed 45 -> 41 us): zeroed half
+// matrices (Jh, Kh; null: none), D in FP32 (null: none) and as float pairs
+// (hi, lo) for the dd kernels (null: none)
+__global__ void prepare_kernel(const double *D, double *Jh, double *Kh, float *Df, float2 *Dd, int64_t n) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx < n) Df[idx] = (float)D[idx];
-}
-
-// D as float pairs (hi, lo) for the dd kernels
-__global__ void to_dd_kernel(const double *D, float2 *Dd, int64_t n) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx < n) {
-    const double d = D[idx];
-    const float hi = __double2float_rn(d);
-    Dd[idx] = make_float2(hi, __double2float_rn(d - (double)hi));
+  if (idx >= n) return;
+  if (Jh) {
+    Jh[idx] = 0.0;
+    Kh[idx] = 0.0;
   }
+  if (!Df && !Dd) return;
+  const double d = D[idx];
+  const float hi = __double2float_rn(d);
+  if (Df) Df[idx] = hi;
+  if (Dd) Dd[idx] = make_float2(hi, __double2float_rn(d - (double)hi));
 }
 
 // ---------------------------------------------------------------------------
@@ -374,8 +378,11 @@ struct sf_handle {
   // one hardware work queue per side stream needs CUDA_DEVICE_MAX_CONNECTIONS
   // >= kSideStreams when the context is created (default 8: streams then
   // share queues, and a launch waits behind another stream's launch)
-  static constexpr int kSideStreams = 16;
-  static constexpr int kHiStreams = 6;   // high-priority side streams (accurate tier of a mixed build)
+  static constexpr int kSideStreams = 32;
+  static constexpr int kHiStreams = 16;   // the first ones run at high priority (accurate tier of a mixed build)
+  // streams of the current lists in a mixed build: accurate-tier launches on
+  // [0, n_hi), FP32 launches on [kHiStreams, kHiStreams + n_lo) (build_work)
+  int n_hi = kHiStreams, n_lo = kSideStreams - kHiStreams;
   cudaStream_t side[kSideStreams] = {};
   cudaEvent_t fork_ev = nullptr, join_ev[kSideStreams] = {};
   std::vector<int> slice_stream;   // side stream of each slice (greedy by cost)
@@ -602,6 +609,7 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
   };
   std::vector<Part> parts(3 * kNumClass);   // per class: accurate tier, FP32, double-float part of FP64
   std::vector<int64_t> totals(kNumClass, 0);
+  double load32 = 0.0;          // estimated operations of the FP32 tier
   auto build_class = [&](int cls, std::vector<int64_t> &hist) {
     const ClassInfo &ci = kClassInfo[cls];
     const int X = pair_class_of(ci.la, ci.lb), Y = pair_class_of(ci.lc, ci.ld);
@@ -793,6 +801,7 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     for (auto &t : pool) t.join();
     double load[3] = {0.0, 0.0, 0.0};   // per arithmetic
     for (const Part &part : parts) load[part.head.prec] += part.load;
+    load32 = load[1];
     next = 0;
     auto cut = [&]() {
       for (int c = next++; c < 3 * kNumClass; c = next++) segment(c / 3, c % 3, load);
@@ -869,15 +878,26 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     }
     h->slices.swap(sorted);
     std::sort(cost.begin(), cost.end(), std::greater<double>());
-    bool has32 = false, hasacc = false;
+    bool has32 = false, hasacc = false, has64 = false;
     for (const auto &sl : h->slices) (sl.prec == 1 ? has32 : hasacc) = true;
+    for (const auto &sl : h->slices) has64 |= sl.prec == 0;
+    // A launch of a small or FP64 list lasts as long as its longest quartet, so
+    // each should have a stream of its own (16 + 16).  Where the FP32 tier keeps
+    // the GPU busy anyway (above 2e9 estimated operations), fewer streams leave
+    // the double-float launches, which go first, less in its way (6 + 10).
+    // FP32 + double-float 6-31G*, 6 + 10 / 16 + 16 streams: (H2O)3 0.37 / 0.22 ms,
+    // (H2O)6 0.61 / 0.62, (H2O)8 1.17 / 1.25; FP32 + FP64 at cutoff 1e-5: (H2O)3
+    // 0.55 / 0.42, (H2O)8 3.15 / 2.68.
+    const bool few = !has64 && load32 > 2e9;
+    h->n_hi = few ? 6 : sf_handle::kHiStreams;
+    h->n_lo = few ? 10 : sf_handle::kSideStreams - sf_handle::kHiStreams;
     if (has32 && hasacc) {
       // mixed build: accurate-tier launches on the high-priority streams,
       // FP32 launches on the others, each group balanced by LPT
       std::vector<double> ca, cf;
       for (size_t k = 0; k < h->slices.size(); ++k) (h->slices[k].prec == 1 ? cf : ca).push_back(cost[k]);
-      const std::vector<int> sa = lpt_streams(ca, 0, sf_handle::kHiStreams);
-      const std::vector<int> sf = lpt_streams(cf, sf_handle::kHiStreams, sf_handle::kSideStreams);
+      const std::vector<int> sa = lpt_streams(ca, 0, h->n_hi);
+      const std::vector<int> sf = lpt_streams(cf, sf_handle::kHiStreams, sf_handle::kHiStreams + h->n_lo);
       h->slice_stream.assign(h->slices.size(), 0);
       size_t ia = 0, ifp = 0;
       for (size_t k = 0; k < h->slices.size(); ++k)
@@ -1038,7 +1058,7 @@ int make_plan(sf_handle *h, bool grad, int active) {
     h->plan.push_back(L);
     if (cl && mixed && sl.prec != 1) {
       sf_handle::Launch Dm{(int)k, 1, sf_handle::kHiStreams + rr, 1, sl.w};
-      rr = (rr + 1) % (sf_handle::kSideStreams - sf_handle::kHiStreams);
+      rr = (rr + 1) % h->n_lo;
       Dm.w.list = h->d_dem.p + off;
       Dm.w.count = h->d_cnt.p + 4 * k + 1;
       const int S = std::max(1, sl.w.psplit) * std::max(1, sl.w.wsplit);
@@ -1090,8 +1110,9 @@ void make_groups(sf_handle *h) {
   const bool mixed = has32 && hasacc;
   std::vector<double> ca, cf;
   for (const auto &g : h->groups) (mixed && g.kind != 1 ? ca : cf).push_back(g.est);
-  const std::vector<int> sa = lpt_streams(ca, 0, sf_handle::kHiStreams);
-  const std::vector<int> sf = lpt_streams(cf, mixed ? sf_handle::kHiStreams : 0, sf_handle::kSideStreams);
+  const std::vector<int> sa = lpt_streams(ca, 0, h->n_hi);
+  const std::vector<int> sf = lpt_streams(cf, mixed ? sf_handle::kHiStreams : 0,
+                                          mixed ? sf_handle::kHiStreams + h->n_lo : sf_handle::kSideStreams);
   size_t ia = 0, ifp = 0;
   for (auto &g : h->groups) g.stream = mixed && g.kind != 1 ? sa[ia++] : sf[ifp++];
 }
@@ -1224,24 +1245,21 @@ int profiling_events(sf_handle *h, cudaStream_t st) {
   return SF_OK;
 }
 
-// FP32 / double-float copies of D needed by the current launch list
-int convert_density(sf_handle *h, const double *D, float *D32, float *Ddd, cudaStream_t st, int *launches) {
+// zero Jh and Kh (null for a gradient) and make the FP32 / double-float copies
+// of D that the current launch list needs
+int prepare_build(sf_handle *h, const double *D, double *Jh, double *Kh, float *D32, float *Ddd, cudaStream_t st,
+                  int *launches) {
   const size_t nn = (size_t)h->nao * h->nao;
   bool need32 = false, needdd = false;
   for (const auto &s : h->slices) {
     need32 |= s.prec == 1;
     needdd |= s.prec == 2;
   }
-  if (need32) {
-    to_float_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(D, D32, (int64_t)nn);
-    SF_CK(cudaGetLastError());
-    if (launches) ++*launches;
-  }
-  if (needdd) {
-    to_dd_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(D, reinterpret_cast<float2 *>(Ddd), (int64_t)nn);
-    SF_CK(cudaGetLastError());
-    if (launches) ++*launches;
-  }
+  if (!Jh && !need32 && !needdd) return SF_OK;
+  prepare_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(
+      D, Jh, Kh, need32 ? D32 : nullptr, needdd ? reinterpret_cast<float2 *>(Ddd) : nullptr, (int64_t)nn);
+  SF_CK(cudaGetLastError());
+  if (launches) ++*launches;
   return SF_OK;
 }
 
@@ -1828,10 +1846,8 @@ int sf_fock_jk(sf_handle *h, const double *D, double *J, double *K, int32_t prec
   if (rc) return rc;
   const int n = h->nao;
   const size_t nn = (size_t)n * n;
-  SF_CK(cudaMemsetAsync(h->d_Jh.p, 0, nn * sizeof(double), st));
-  SF_CK(cudaMemsetAsync(h->d_Kh.p, 0, nn * sizeof(double), st));
   int launches = 0;
-  rc = convert_density(h, D, h->d_D32.p, h->d_Ddd.p, st, &launches);
+  rc = prepare_build(h, D, h->d_Jh.p, h->d_Kh.p, h->d_D32.p, h->d_Ddd.p, st, &launches);
   if (rc) return rc;
   rc = run_call(h, false, D, h->d_D32.p, h->d_Ddd.p, h->d_Jh.p, h->d_Kh.p, nullptr, cutoff, fp32_cutoff, st, h->profiling,
                 &launches);
@@ -1932,7 +1948,7 @@ int sf_autotune(sf_handle *h, const double *D, int32_t precision, double cutoff,
   cudaStream_t st = (cudaStream_t)stream;
   int rc = build_work(h, precision, cutoff, fp32_cutoff);
   if (rc) return rc;
-  rc = convert_density(h, D, h->d_D32.p, h->d_Ddd.p, st, nullptr);
+  rc = prepare_build(h, D, nullptr, nullptr, h->d_D32.p, h->d_Ddd.p, st, nullptr);
   if (rc) return rc;
   cudaEvent_t e0, e1;
   SF_CK(cudaEventCreate(&e0));
@@ -2175,8 +2191,7 @@ int sf_fock_jk_noalloc(sf_handle *h, const double *D, double *J, double *K, int3
   double *Jh = scratch, *Kh = scratch + nn;
   float *Ddd = reinterpret_cast<float *>(scratch + 2 * nn);   // nao^2 float pairs, then nao^2 floats
   float *D32 = reinterpret_cast<float *>(scratch + 3 * nn);
-  SF_CK(cudaMemsetAsync(scratch, 0, 2 * nn * sizeof(double), st));
-  int rc = convert_density(h, D, D32, Ddd, st, nullptr);
+  int rc = prepare_build(h, D, Jh, Kh, D32, Ddd, st, nullptr);
   if (rc) return rc;
   rc = run_call(h, false, D, D32, Ddd, Jh, Kh, nullptr, cutoff, fp32_cutoff, st, 0, nullptr);
   if (rc) return rc;
@@ -2196,7 +2211,7 @@ int sf_grad_jk(sf_handle *h, const double *D, double *grad, int32_t precision, d
   cudaStream_t st = (cudaStream_t)stream;
   int rc = build_work(h, precision, cutoff, fp32_cutoff);
   if (rc) return rc;
-  rc = convert_density(h, D, h->d_D32.p, h->d_Ddd.p, st, nullptr);
+  rc = prepare_build(h, D, nullptr, nullptr, h->d_D32.p, h->d_Ddd.p, st, nullptr);
   if (rc) return rc;
   // per-launch events in the profiling modes (serialised in mode 2), read by sf_get_slice_info
   return run_call(h, true, D, h->d_D32.p, h->d_Ddd.p, nullptr, nullptr, grad, cutoff, fp32_cutoff, st, h->profiling, nullptr);

@@ -125,7 +125,7 @@ class FockBuilder:
 
     def set_launch_mode(self, mode: str = "streams", ctas_per_sm: int = 0):
         """How Fock builds launch their class kernels (sf_set_launch_mode):
-        "streams" (one launch per class slice on 16 side streams) or
+        "streams" (one launch per class and arithmetic on up to 32 side streams) or
         "persistent" (the FP32 register-path classes as one persistent launch
         per register tier, fed by a device work queue)."""
         m = {"streams": 0, "persistent": 1}[mode]
