@@ -1327,7 +1327,7 @@ struct sf_eri_plan {
   double flops = 0.0;
   std::vector<int64_t> offsets;
   struct Seg {
-    int cls, psplit, csplit;
+    int cls, psplit, csplit, cluster;
     int64_t n;
     size_t off;
   };
@@ -1390,6 +1390,14 @@ int build_eri_plan(sf_handle *h, const int32_t *hq, int64_t nq, const int64_t *h
     byc[x * (x + 1) / 2 + y].push_back(it);
   }
   pl->total = maxend;
+  double share = 0.0;   // estimated operations per lane with 8 warps per SM sub-partition
+  for (int cls = 0; cls < kNumClass; ++cls) {
+    const ClassInfo &ci = kClassInfo[cls];
+    const int nr = (ci.la + ci.lb + ci.lc + ci.ld) / 2 + 1;
+    const double nabcd = (double)ncart(ci.la) * ncart(ci.lb) * ncart(ci.lc) * ncart(ci.ld);
+    for (const Item &it : byc[cls]) share += it.cost * (nr * (nabcd + 30.0) + 40.0);
+  }
+  share /= (double)std::max(h->nsm, 1) * 4 * 8 * 32;
   std::vector<int> pab, pcd, fl, str;
   std::vector<int64_t> off;
   pab.reserve(nq); pcd.reserve(nq); fl.reserve(nq); off.reserve(nq); str.reserve(4 * nq);
@@ -1411,24 +1419,38 @@ int build_eri_plan(sf_handle *h, const int32_t *hq, int64_t nq, const int64_t *h
     for (int pr = 0; pr < 2; ++pr) {
       const int T = pr == 0 ? ci.t64 : ci.t32;
       const int pmax = 32 / T;
-      // {P, C}: lanes and warps that share a quartet.  The costliest quartets
-      // (hundreds of primitive quartets on one warp) set the end of a batch, so
-      // those that leave four primitive quartets to every sub-group of a whole
-      // CTA take one: 10 007 random quartets in FP64 10.7 -> 4.0 ms, 60 000 in
-      // double-float 11.0 -> 4.8 ms.
+      // lanes (P), warps (C) and CTAs (N) that share a quartet.  The costliest
+      // quartets (hundreds of primitive quartets on one warp) set the end of a
+      // batch, so those that leave four primitive quartets to every sub-group of
+      // a whole CTA take one (10 007 random quartets in FP64 10.7 -> 4.0 ms,
+      // 60 000 in double-float 11.0 -> 4.8 ms), and a cluster of two to eight
+      // where that leaves four to each and a lane's estimated work is still over
+      // four times the average over the lanes that fill the GPU (a batch that
+      // fills it loses 5 % to clusters): 500 quartets in FP64 2.0 -> 1.6 ms, in
+      // double-float 1.31 -> 0.76, 10 007 3.4 -> 2.6 and 1.95 -> 1.44, 60 000 unchanged.
+      const double per_prim = nr * (nabcd + 30.0) + 40.0;
+      struct Split {
+        int P, C, N;
+        bool operator==(const Split &o) const { return P == o.P && C == o.C && N == o.N; }
+      };
       auto split = [&](int64_t c) {
-        if (c >= 4 * (int64_t)pmax * kEriWarps) return std::make_pair(pmax, kEriWarps);
-        if (pmax > 1 && c >= 4 * pmax) return std::make_pair(pmax, 1);
-        if (pmax > 8 && c >= 32) return std::make_pair(8, 1);
-        return std::make_pair(1, 1);
+        const int64_t cta = 4 * (int64_t)pmax * kEriWarps;
+        if (c >= cta) {
+          int n = 1;
+          while (2 * n <= kEriCluster && c >= 2 * n * cta && (double)c * per_prim > 4.0 * share * kBlock * n) n *= 2;
+          return Split{pmax, kEriWarps, n};
+        }
+        if (pmax > 1 && c >= 4 * pmax) return Split{pmax, 1, 1};
+        if (pmax > 8 && c >= 32) return Split{8, 1, 1};
+        return Split{1, 1, 1};
       };
       size_t q0 = 0;
       while (q0 < v.size()) {
-        const std::pair<int, int> P = split(v[q0].cost);
+        const Split P = split(v[q0].cost);
         size_t q1 = q0 + 1;
         double c = v[q0].cost;
         while (q1 < v.size() && split(v[q1].cost) == P) c += v[q1++].cost;
-        pl->segs[pr].push_back({cls, P.first, P.second, (int64_t)(q1 - q0), base + q0});
+        pl->segs[pr].push_back({cls, P.P, P.C, P.N, (int64_t)(q1 - q0), base + q0});
         cost[pr].push_back(c * nr * (nabcd + 30.0));
         q0 = q1;
       }
@@ -1463,7 +1485,7 @@ int run_eri_plan(sf_eri_plan *pl, int precision, double *out, cudaStream_t st) {
   return fan_out_list(h, st, pl->seg_stream[pr], [&](size_t k, cudaStream_t ss) {
     const sf_eri_plan::Seg &sg = segs[k];
     EriWork w{pl->d_pab.p + sg.off, pl->d_pcd.p + sg.off, pl->d_fl.p + sg.off, pl->d_off.p + sg.off,
-              pl->d_str.p + 4 * sg.off, sg.n, out, sg.psplit, sg.csplit};
+              pl->d_str.p + 4 * sg.off, sg.n, out, sg.psplit, sg.csplit, sg.cluster};
     if (precision == SF_PREC_DF) return launch_eri_dd(sg.cls, h->kp, w, ss);
     return launch_eri(sg.cls, pr, h->kp, w, ss);
   });

@@ -10,7 +10,9 @@ static cudaError_t run_eri(const KParams &kp, const EriWork &w, cudaStream_t st)
   if (w.n <= 0) return cudaSuccess;
   const int P = w.psplit < 1 ? 1 : w.psplit;
   const bool cta = w.csplit > 1;   // a CTA per quartet
-  if (T * P > 32 || (P & (P - 1)) || (cta && (T * P != 32 || w.csplit != kEriWarps))) return cudaErrorInvalidValue;
+  if (T * P > 32 || (P & (P - 1)) || (cta && (T * P != 32 || w.csplit != kEriWarps)) ||
+      w.cluster < 1 || w.cluster > kEriCluster || (w.cluster > 1 && !cta))
+    return cudaErrorInvalidValue;
   EriWork w2 = w;
   w2.psplit = P;
   const int G = cta ? 1 : kBlock / (T * P);
@@ -19,8 +21,7 @@ static cudaError_t run_eri(const KParams &kp, const EriWork &w, cudaStream_t st)
   int64_t grid = (w.n + G - 1) / G;
   // Rys table block in shared memory: grid-stride
   if (T == 1 && std::is_same<R, float>::value) grid = std::min<int64_t>(grid, (int64_t)std::max(kp.nsm, 1) * 16);
-  eri_kernel<LA, LB, LC, LD, R, T><<<(unsigned)grid, kBlock, smem, st>>>(kp, w2);
-  return cudaGetLastError();
+  return launch_eri_kernel(eri_kernel<LA, LB, LC, LD, R, T>, grid, smem, kp, w2, st);
 }
 
 cudaError_t launch_eri(int cls, int fp32, const KParams &kp, const EriWork &w, cudaStream_t st) {

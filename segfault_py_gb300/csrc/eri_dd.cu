@@ -10,14 +10,15 @@ static cudaError_t run_eri_dd(const KParams &kp, const EriWork &w, cudaStream_t 
   if (w.n <= 0) return cudaSuccess;
   const int P = w.psplit < 1 ? 1 : w.psplit;
   const bool cta = w.csplit > 1;   // a CTA per quartet
-  if (T * P > 32 || (P & (P - 1)) || (cta && (T * P != 32 || w.csplit != kEriWarps))) return cudaErrorInvalidValue;
+  if (T * P > 32 || (P & (P - 1)) || (cta && (T * P != 32 || w.csplit != kEriWarps)) ||
+      w.cluster < 1 || w.cluster > kEriCluster || (w.cluster > 1 && !cta))
+    return cudaErrorInvalidValue;
   EriWork w2 = w;
   w2.psplit = P;
   const int G = cta ? 1 : kBlock / (T * P);
   const size_t smem = grp_smem<LA, LB, LC, LD, dd, T>() +
                       (T == 1 && cta ? (size_t)kEriWarps * QC<LA, LB, LC, LD>::NABCD * sizeof(dd) : 0);
-  eri_kernel<LA, LB, LC, LD, dd, T><<<(unsigned)((w.n + G - 1) / G), kBlock, smem, st>>>(kp, w2);
-  return cudaGetLastError();
+  return launch_eri_kernel(eri_kernel<LA, LB, LC, LD, dd, T>, (w.n + G - 1) / G, smem, kp, w2, st);
 }
 
 cudaError_t launch_eri_dd(int cls, const KParams &kp, const EriWork &w, cudaStream_t st) {

@@ -89,6 +89,24 @@ constexpr size_t grp_smem() {
   return T == 1 ? 0 : (size_t)(kBlock / T) * Grp<LA, LB, LC, LD, R, T>::BUFN * sizeof(R);
 }
 
+// a raw-integral launch of `quartets` CTA trips, w.cluster CTAs (one cluster) each
+template <typename K>
+inline cudaError_t launch_eri_kernel(K kern, int64_t quartets, size_t smem, const KParams &kp, const EriWork &w,
+                                     cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(quartets * w.cluster));
+  cfg.blockDim = dim3(kBlock);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)w.cluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = w.cluster > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, kp, w);
+}
+
 template <typename K>
 inline cudaError_t prep_smem(K kern, size_t smem) {
   if (smem > 48 * 1024) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

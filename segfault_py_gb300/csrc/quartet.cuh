@@ -24,6 +24,7 @@
 // Epilogues: J/K digestion (fock), store (eri batch), diagonal max (Schwarz).
 #pragma once
 #include <cstdint>
+#include <cstring>
 #include <type_traits>
 
 #include "dd.cuh"
@@ -1455,8 +1456,10 @@ struct EriWork {
   double *out;
   int psplit;                  // P primitive sub-groups per quartet (T*P <= 32)
   int csplit = 1;              // kEriWarps: the four warps of a CTA share a quartet (T*P == 32), else 1
+  int cluster = 1;             // CTAs (one cluster) that share a quartet; > 1 only with csplit
 };
 constexpr int kEriWarps = kBlock / 32;
+constexpr int kEriCluster = 8;   // the portable cluster size
 
 // one quartet of the one-lane (T == 1) raw-integral path: P lanes share it
 template <int LA, int LB, int LC, int LD, typename R>
@@ -1476,18 +1479,60 @@ __device__ __forceinline__ void eri_t1_quartet(const KParams &kp, const EriWork 
     out[Q::ca(o) * s0 + Q::cb(o) * s1 + Q::cc(o) * s2 + Q::cd(o) * s3] = to_f64(acc[o] * (R)Q::norm(o));
 }
 
+// CTA rank and size of the launch's clusters (1 without the launch attribute)
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// a 4-byte word at the same shared-memory address in CTA `rank` of the cluster
+__device__ __forceinline__ unsigned ld_cluster(const void *p, unsigned rank) {
+  unsigned a, v;
+  const unsigned local = (unsigned)__cvta_generic_to_shared(p);
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+template <typename R>
+__device__ __forceinline__ R ld_cluster_r(const R *p, unsigned rank) {
+  static_assert(sizeof(R) == 4 || sizeof(R) == 8, "");
+  R v;
+  unsigned w[sizeof(R) / 4];
+#pragma unroll
+  for (int k = 0; k < (int)(sizeof(R) / 4); ++k) w[k] = ld_cluster(reinterpret_cast<const unsigned *>(p) + k, rank);
+  memcpy(&v, w, sizeof(R));
+  return v;
+}
+
 // sum of a quartet's partial integrals over the CTA's warps (buf: warp c's
-// NABCD values at c * stride) and store
+// NABCD values at c * stride), then over the cluster's CTAs through distributed
+// shared memory (every CTA stores its share of the outputs)
 template <int LA, int LB, int LC, int LD, typename R>
-__device__ __forceinline__ void eri_store_cta(const EriWork &w, int64_t q, const R *buf, int stride) {
+__device__ __forceinline__ void eri_store_cta(const EriWork &w, int64_t q, R *buf, int stride) {
   using Q = QC<LA, LB, LC, LD>;
   const int s0 = w.strides[4 * q], s1 = w.strides[4 * q + 1], s2 = w.strides[4 * q + 2], s3 = w.strides[4 * q + 3];
   double *out = w.out + w.out_off[q];
+  auto store = [&](int o, R v) {
+    out[Q::ca(o) * s0 + Q::cb(o) * s1 + Q::cc(o) * s2 + Q::cd(o) * s3] = to_f64(v * (R)Q::norm(o));
+  };
   for (int o = threadIdx.x; o < Q::NABCD; o += kBlock) {
     R v = buf[o];
 #pragma unroll
     for (int c = 1; c < kEriWarps; ++c) v += buf[c * stride + o];
-    out[Q::ca(o) * s0 + Q::cb(o) * s1 + Q::cc(o) * s2 + Q::cd(o) * s3] = to_f64(v * (R)Q::norm(o));
+    if (w.cluster > 1) buf[o] = v;
+    else store(o, v);
+  }
+  if (w.cluster > 1) {
+    cluster_sync();
+    for (int o = (int)cluster_rank() * kBlock + threadIdx.x; o < Q::NABCD; o += w.cluster * kBlock) {
+      R v = ld_cluster_r(buf + o, 0);
+      for (int r = 1; r < w.cluster; ++r) v += ld_cluster_r(buf + o, r);
+      store(o, v);
+    }
+    cluster_sync();   // no CTA leaves, or writes buf again, while another reads it
   }
 }
 
@@ -1521,11 +1566,12 @@ __global__ void __launch_bounds__(kBlock) eri_kernel(KParams kp, EriWork w) {
     if (w.csplit > 1) {   // one quartet per CTA trip
       extern __shared__ __align__(16) unsigned char smem_t[];
       R *red = reinterpret_cast<R *>(smem_t + eri_tab_smem<LA, LB, LC, LD, R, T>());
-      for (int64_t q = blockIdx.x; q < w.n; q += gridDim.x) {
+      const int NC = w.cluster, rank = NC > 1 ? (int)cluster_rank() : 0;
+      for (int64_t q = blockIdx.x / NC; q < w.n; q += gridDim.x / NC) {
         const int fl = w.flags[q];
         const QGeom<R> g = make_geom<R>(kp, w.pab[q], w.pcd[q], fl & 1, fl & 2);
         R acc[Q::NABCD];
-        eval_t1<LA, LB, LC, LD, R>(kp, g, acc, threadIdx.x, kBlock, tab_s);
+        eval_t1<LA, LB, LC, LD, R>(kp, g, acc, rank * kBlock + threadIdx.x, NC * kBlock, tab_s);
         reduce_psplit<R, Q::NABCD, 1>(acc, 32, 0xffffffffu);
         if (lane == 0) {
 #pragma unroll
@@ -1541,8 +1587,8 @@ __global__ void __launch_bounds__(kBlock) eri_kernel(KParams kp, EriWork w) {
     for (int64_t q = (int64_t)blockIdx.x * (kBlock / TP) + grp; q < w.n; q += stride)
       eri_t1_quartet<LA, LB, LC, LD, R>(kp, w, q, p, P, qmask, tab_s);
   } else {
-    const int C = w.csplit;
-    const int64_t q = C > 1 ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * (kBlock / TP) + grp;
+    const int C = w.csplit, NC = w.cluster;
+    const int64_t q = C > 1 ? (int64_t)blockIdx.x / NC : (int64_t)blockIdx.x * (kBlock / TP) + grp;
     if (q >= w.n) return;
     const int fl = w.flags[q];
     const QGeom<R> g = make_geom<R>(kp, w.pab[q], w.pcd[q], fl & 1, fl & 2);
@@ -1553,7 +1599,7 @@ __global__ void __launch_bounds__(kBlock) eri_kernel(KParams kp, EriWork w) {
     R *buf = reinterpret_cast<R *>(smem_raw) + (threadIdx.x / T) * GP::BUFN;
     const unsigned gmask = (T == 32) ? 0xffffffffu : (((1u << T) - 1u) << (lane & ~(T - 1)));
     R acc[GP::NPER];
-    eval_grp<LA, LB, LC, LD, R, T>(kp, g, buf, t, gmask, acc, C > 1 ? grp * P + p : p, C * P);
+    eval_grp<LA, LB, LC, LD, R, T>(kp, g, buf, t, gmask, acc, C > 1 ? ((NC > 1 ? (int)cluster_rank() : 0) * C + grp) * P + p : p, NC * C * P);
     if (P > 1) reduce_psplit<R, GP::NPER, T>(acc, P, qmask);
     if (C > 1) {   // the warps' sums through the buffers of their first groups
       if (p == 0) {
@@ -1564,7 +1610,7 @@ __global__ void __launch_bounds__(kBlock) eri_kernel(KParams kp, EriWork w) {
         }
       }
       __syncthreads();
-      eri_store_cta<LA, LB, LC, LD, R>(w, q, reinterpret_cast<const R *>(smem_raw), (32 / T) * GP::BUFN);
+      eri_store_cta<LA, LB, LC, LD, R>(w, q, reinterpret_cast<R *>(smem_raw), (32 / T) * GP::BUFN);
       return;
     }
     if (p != 0) return;
