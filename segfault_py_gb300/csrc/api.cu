@@ -215,8 +215,11 @@ __global__ void prepare_kernel(const double *D, double *Jh, double *Kh, float *D
 //    exponent, is below the accurate cutoff: quartets of tight core shells
 //    stay accurate.
 // Every list is compacted into a "kept" and a "demoted" list at the same
-// offsets (d_keep, d_dem), order kept within each chunk of 1024 entries, with
-// device counts read by the kernels, so nothing synchronises with the host.
+// offsets (d_keep, d_dem), with device counts read by the kernels, so nothing
+// synchronises with the host.  Chunks of 1024 entries take their place in the
+// compacted list by an atomic counter (gradient: one pass, chunks in any order)
+// or, for a Fock build, in list order from the chunk counts of a first pass: the
+// FP32 sums over runs of equal bra pairs then round the same in every build.
 struct ClassifySlice {
   int64_t off, n;        // offset in the quartet-list buffer, length
   int x0, y0;            // first global pair of the bra / ket pair class
@@ -246,7 +249,8 @@ __global__ void shell_dmax_kernel(const double *D, int n, const int *l, const in
 __global__ void __launch_bounds__(kClsThreads) classify_kernel(
     const int2 *list, const ClassifySlice *sl, const int2 *blk, const int *pa, const int *pb, const int *pnp,
     const double *pq, const float *dm, const float *sqa, int ns, int grad_mode, double t_drop, double t_acc,
-    int2 *keep, int2 *dem, unsigned long long *cnt) {
+    int2 *keep, int2 *dem, unsigned long long *cnt, int2 *chunks, int pass) {
+  // pass 0: places by atomics; 1: this chunk's counts to chunks[]; 2: places from them
   const int2 bk = blk[blockIdx.x];
   const ClassifySlice S = sl[bk.x];
   const int64_t e0 = (int64_t)bk.y * kClsChunk + (int64_t)threadIdx.x * kClsPer;
@@ -295,10 +299,24 @@ __global__ void __launch_bounds__(kClsThreads) classify_kernel(
     sd += __shfl_xor_sync(0xffffffffu, sd, off);
   }
   if (lane == 31) { s_wk[warp] = ik; s_wd[warp] = id; }
-  if (lane == 0) {
+  if (lane == 0 && pass != 1) {
     if (sk) atomicAdd(cnt + 4 * bk.x + 2, sk);
     if (sd) atomicAdd(cnt + 4 * bk.x + 3, sd);
   }
+  int before_k = 0, before_d = 0;   // earlier chunks of the slice (blocks of a slice are consecutive)
+  if (pass == 2)
+    for (int c = threadIdx.x; c < bk.y; c += kClsThreads) {
+      const int2 n = chunks[(int)blockIdx.x - bk.y + c];
+      before_k += n.x;
+      before_d += n.y;
+    }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    before_k += __shfl_xor_sync(0xffffffffu, before_k, off);
+    before_d += __shfl_xor_sync(0xffffffffu, before_d, off);
+  }
+  __shared__ int s_bk[kClsThreads / 32], s_bd[kClsThreads / 32];
+  if (lane == 0) { s_bk[warp] = before_k; s_bd[warp] = before_d; }
   __syncthreads();
   if (threadIdx.x == 0) {
     int tk = 0, td = 0;
@@ -309,9 +327,21 @@ __global__ void __launch_bounds__(kClsThreads) classify_kernel(
       tk += a;
       td += b;
     }
-    s_base[0] = tk ? atomicAdd(cnt + 4 * bk.x, (unsigned long long)tk) : 0ull;
-    s_base[1] = td ? atomicAdd(cnt + 4 * bk.x + 1, (unsigned long long)td) : 0ull;
+    if (pass == 1) {
+      chunks[blockIdx.x] = make_int2(tk, td);
+    } else {
+      s_base[0] = tk ? atomicAdd(cnt + 4 * bk.x, (unsigned long long)tk) : 0ull;
+      s_base[1] = td ? atomicAdd(cnt + 4 * bk.x + 1, (unsigned long long)td) : 0ull;
+      if (pass == 2) {
+        s_base[0] = s_base[1] = 0ull;
+        for (int w = 0; w < kClsThreads / 32; ++w) {
+          s_base[0] += (unsigned long long)s_bk[w];
+          s_base[1] += (unsigned long long)s_bd[w];
+        }
+      }
+    }
   }
+  if (pass == 1) return;
   __syncthreads();
   int64_t ok = (int64_t)s_base[0] + s_wk[warp] + ik - nk, od = (int64_t)s_base[1] + s_wd[warp] + id - nd;
 #pragma unroll
@@ -410,6 +440,7 @@ struct sf_handle {
   DBuf<unsigned long long> d_cnt;          // per slice: kept, demoted quartets; kept, demoted primitive quartets
   DBuf<ClassifySlice> d_csl;
   DBuf<int2> d_blk_acc, d_blk_all;         // classification CTAs (slice, chunk): accurate-tier slices / all
+  DBuf<int2> d_chunks;                     // kept and demoted quartets of each accurate-tier chunk
   int nblk_acc = 0, nblk_all = 0;
   // the launches of the last Fock build or gradient: one per slice, plus one
   // FP32 launch per accurate-tier slice for its demoted quartets
@@ -923,6 +954,7 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     SF_CK(h->d_blk_all.upload(bl));
     h->nblk_acc = (int)ba.size();
     h->nblk_all = (int)bl.size();
+    SF_CK(h->d_chunks.alloc(ba.size()));
     SF_CK(h->d_keep.alloc(all.size()));
     SF_CK(h->d_dem.alloc(all.size()));
     SF_CK(h->d_cnt.alloc(4 * std::max<size_t>(h->slices.size(), 1)));
@@ -963,12 +995,15 @@ int density_classify(sf_handle *h, const double *D, bool grad, double cut, doubl
                                                                        h->d_dmax.p);
   SF_CK(cudaGetLastError());
   if (nb > 0) {
-    classify_kernel<<<(unsigned)nb, kClsThreads, 0, st>>>(
-        h->d_list.p, h->d_csl.p, grad ? h->d_blk_all.p : h->d_blk_acc.p, h->d_pa.p, h->d_pb.p, h->d_pfull.p, h->d_pq.p,
-        h->d_dmax.p, h->d_sqa.p, ns, grad ? 1 : 0, t_drop, t_acc, h->d_keep.p, h->d_dem.p, h->d_cnt.p);
-    SF_CK(cudaGetLastError());
+    for (int pass = grad ? 0 : 1; pass <= (grad ? 0 : 2); ++pass) {
+      classify_kernel<<<(unsigned)nb, kClsThreads, 0, st>>>(
+          h->d_list.p, h->d_csl.p, grad ? h->d_blk_all.p : h->d_blk_acc.p, h->d_pa.p, h->d_pb.p, h->d_pfull.p,
+          h->d_pq.p, h->d_dmax.p, h->d_sqa.p, ns, grad ? 1 : 0, t_drop, t_acc, h->d_keep.p, h->d_dem.p, h->d_cnt.p,
+          h->d_chunks.p, pass);
+      SF_CK(cudaGetLastError());
+    }
   }
-  if (launches) *launches += nb > 0 ? 2 : 1;
+  if (launches) *launches += nb == 0 ? 1 : grad ? 2 : 3;
   *active = 1;
   return SF_OK;
 }

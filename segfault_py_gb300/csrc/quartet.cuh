@@ -460,10 +460,10 @@ __device__ __forceinline__ void rys_2d_dd(dd g0, dd c00, dd c00p, dd b00, dd b10
                                           dd *__restrict__ I) {
   constexpr int LAB = LA + LB, LCD = LC + LD;
   dd G[LAB + 1][LCD + 1];
+  G[0][0] = g0;
   // x * G[i][k], and x * G[i][k] + y
   auto mul = [&](dd x, int i, int k) { return UNIT && i == 0 && k == 0 ? x : x * G[i][k]; };
   auto mad = [&](dd x, int i, int k, dd y) { return UNIT && i == 0 && k == 0 ? x + y : dd_fma(x, G[i][k], y); };
-  G[0][0] = g0;
   if (LAB > 0) G[1][0] = mul(c00, 0, 0);
 #pragma unroll
   for (int i = 1; i < LAB; ++i) G[i + 1][0] = dd_fma(c00, G[i][0], mul(dd_times(i, b10), i - 1, 0));
