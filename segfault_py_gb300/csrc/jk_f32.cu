@@ -18,7 +18,9 @@ static cudaError_t run_jk32(const KParams &kp, const ClassWork *w, int nw, const
   if (m.n == 0) return cudaSuccess;
   auto kern = jk_kernel<LA, LB, LC, LD, float, T>;
   size_t smem = grp_smem<LA, LB, LC, LD, float, T>();
-  if (T == 1) smem = (size_t)kTabNint * QC<LA, LB, LC, LD>::NR * kTab32Row * sizeof(float);
+  if (T == 1)   // Rys table block, then a stage per warp
+    smem = ((size_t)kTabNint * QC<LA, LB, LC, LD>::NR * kTab32Row + kBlock / 32 * digest_stage<LA, LB, LC, LD>()) *
+           sizeof(float);
   kern<<<(unsigned)m.cta0[m.n], kBlock, smem, st>>>(kp, m, D, Jh, Kh);
   return cudaGetLastError();
 }
