@@ -1142,10 +1142,13 @@ __device__ __forceinline__ void reduce_psplit(R (&acc)[N], int P, unsigned qmask
 // quartets is 32 sectors for L1 and L2 (with the K adds left out the FP32 builds
 // took 20 to 24 % less); a row of three or six doubles is one to three.
 // C20H42 6-31G** FP32 13.9 -> 12.9 ms ((20|10) 1.08 -> 0.71, (11|10) 1.27 -> 0.92).
-// ON: not for (00|00) and (10|00), whose few short rows do not pay for the stage.
+// ON: not for (00|00) and (10|00), whose few short rows do not pay for the stage
+// (2.62 -> 2.70 ms).
 template <int NR, int NC, typename R, bool ON>
 struct BlockOut {
-  static constexpr bool TR = NR > NC;                 // stored transposed: rows of NR
+  // stored transposed: rows of NR.  Without a stage the bra component stays the
+  // row, where lanes that share the bra pair meet in one row
+  static constexpr bool TR = ON && NR > NC;
   static constexpr int N = NR * NC, LEN = TR ? NR : NC;
   static constexpr bool STAGED = ON && std::is_same<R, float>::value && LEN > 1;
   static constexpr int PITCH = 33;                    // lanes of one quartet hit different banks
