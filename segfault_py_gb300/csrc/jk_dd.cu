@@ -15,7 +15,7 @@ static cudaError_t run_jk_dd(const KParams &kp, const ClassWork *w, int nw, cons
   for (int k = 0; k < nw; ++k)
     if (w[k].n > 0 && !add_segment(m, w[k], T)) return cudaErrorInvalidValue;
   if (m.n == 0) return cudaSuccess;
-  constexpr size_t smem = grp_smem<LA, LB, LC, LD, dd, T>();
+  constexpr size_t smem = jk_smem<LA, LB, LC, LD, dd, T>();
   jk_kernel<LA, LB, LC, LD, dd, T><<<(unsigned)m.cta0[m.n], kBlock, smem, st>>>(kp, m, D, Jh, Kh);
   return cudaGetLastError();
 }
@@ -37,7 +37,7 @@ cudaError_t launch_jk_dd(int cls, const KParams &kp, const ClassWork *w, int nw,
 cudaError_t prepare_jk_dd() {
   cudaError_t e = cudaSuccess;
 #define SF_PREP(id, la, lb, lc, ld, t64, t32)                                                           \
-  if (e == cudaSuccess) e = prep_smem(jk_kernel<la, lb, lc, ld, dd, t64>, grp_smem<la, lb, lc, ld, dd, t64>());
+  if (e == cudaSuccess) e = prep_smem(jk_kernel<la, lb, lc, ld, dd, t64>, jk_smem<la, lb, lc, ld, dd, t64>());
   SF_CLASS_LIST(SF_PREP)
 #undef SF_PREP
   if (e == cudaSuccess) e = prepare_jk_dd_wide();

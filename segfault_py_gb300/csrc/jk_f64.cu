@@ -12,7 +12,7 @@ static cudaError_t run_jk64(const KParams &kp, const ClassWork *w, int nw, const
   for (int k = 0; k < nw; ++k)
     if (w[k].n > 0 && !add_segment(m, w[k], T)) return cudaErrorInvalidValue;
   if (m.n == 0) return cudaSuccess;
-  constexpr size_t smem = grp_smem<LA, LB, LC, LD, double, T>();
+  constexpr size_t smem = jk_smem<LA, LB, LC, LD, double, T>();
   auto kern = jk_kernel<LA, LB, LC, LD, double, T>;
   kern<<<(unsigned)m.cta0[m.n], kBlock, smem, st>>>(kp, m, D, Jh, Kh);
   return cudaGetLastError();
@@ -35,7 +35,7 @@ cudaError_t prepare_jk_f64() {
   cudaError_t e = cudaSuccess;
 #define SF_PREP(id, la, lb, lc, ld, t64, t32)                                                      \
   if (e == cudaSuccess)                                                                            \
-    e = prep_smem(jk_kernel<la, lb, lc, ld, double, t64>, grp_smem<la, lb, lc, ld, double, t64>());
+    e = prep_smem(jk_kernel<la, lb, lc, ld, double, t64>, jk_smem<la, lb, lc, ld, double, t64>());
   SF_CLASS_LIST(SF_PREP)
 #undef SF_PREP
   return e;

@@ -89,6 +89,14 @@ constexpr size_t grp_smem() {
   return T == 1 ? 0 : (size_t)(kBlock / T) * Grp<LA, LB, LC, LD, R, T>::BUFN * sizeof(R);
 }
 
+// of an FP64 or double-float J/K kernel (one-lane classes: the integrals of the
+// quartets that kCoopLanes or more lanes digest)
+template <int LA, int LB, int LC, int LD, typename R, int T>
+constexpr size_t jk_smem() {
+  return T == 1 ? (size_t)(kBlock / kCoopLanes) * QC<LA, LB, LC, LD>::NABCD * sizeof(R)
+                : grp_smem<LA, LB, LC, LD, R, T>();
+}
+
 // a raw-integral launch of `quartets` CTA trips, w.cluster CTAs (one cluster) each
 template <typename K>
 inline cudaError_t launch_eri_kernel(K kern, int64_t quartets, size_t smem, const KParams &kp, const EriWork &w,

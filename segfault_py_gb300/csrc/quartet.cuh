@@ -1314,28 +1314,19 @@ __device__ __forceinline__ void digest_t1(const KParams &kp, const QGeom<R> &g, 
   kbd.flush();
 }
 
-// group version: normalised integrals are staged in buf (shared), then the
-// 6 blocks' entries are distributed over the T lanes
-template <int LA, int LB, int LC, int LD, typename R, int T>
-__device__ __forceinline__ void digest_grp(const KParams &kp, const QGeom<R> &g,
-                                           const R (&acc)[Grp<LA, LB, LC, LD, R, T>::NPER], R *buf, int t,
-                                           unsigned gmask, R scale, const R *__restrict__ D, double *Jh,
-                                           double *Kh) {
+// group version: the normalised integrals are in buf (shared); lane t of the nl
+// that digest the quartet takes the 6 blocks' entries t, t + nl, ...
+template <int LA, int LB, int LC, int LD, typename R>
+__device__ __forceinline__ void digest_grp(const KParams &kp, const QGeom<R> &g, const R *buf, int t, int nl, R scale,
+                                           const R *__restrict__ D, double *Jh, double *Kh) {
   using Q = QC<LA, LB, LC, LD>;
   constexpr int NA = Q::NA, NB = Q::NB, NC = Q::NC, ND = Q::ND;
   const int n = kp.nao;
   const int a0 = g.a0, b0 = g.b0, c0 = g.c0, d0 = g.d0;
-  __syncwarp(gmask);
-#pragma unroll
-  for (int k = 0; k < Grp<LA, LB, LC, LD, R, T>::NPER; ++k) {
-    const int o = Grp<LA, LB, LC, LD, R, T>::out(t, k);
-    if (o < Q::NABCD) buf[o] = acc[k] * (R)Q::norm(o);
-  }
-  __syncwarp(gmask);
   constexpr int E0 = NA * NB, E1 = E0 + NC * ND, E2 = E1 + NA * NC, E3 = E2 + NB * NC, E4 = E3 + NA * ND,
                 E5 = E4 + NB * ND;
 #define V4(ia, ib, ic, id) buf[(((ia) * NB + (ib)) * NC + (ic)) * ND + (id)]
-  for (int e = t; e < E5; e += T) {
+  for (int e = t; e < E5; e += nl) {
     R s = 0;
     if (e < E0) {
       const int ia = e / NB, ib = e % NB;
@@ -1479,9 +1470,42 @@ __device__ __forceinline__ void load_tab32_block(const KParams &kp, int nr, floa
   for (int k = threadIdx.x; k < ntab4; k += blockDim.x) tab4[k] = __ldg(src + k);
 }
 
+constexpr int kCoopLanes = 4;   // lanes from which a one-lane class digests a quartet with all of them
+
+// Digestion by all nl lanes that evaluated a quartet (nl <= 32: qmask; its integrals
+// in buf).  The four warps of a CTA that share one quartet (nl == 32 and W a multiple
+// of 4; FP64 and double-float, the FP32 integrals keep their order of summation)
+// first add their parts (warp c's at base + c wstride) and digest them once.  A
+// quartet split over W groups was digested W times by the T lanes of one primitive
+// sub-group each, two to four times the work of its integrals for short loops.
+template <int LA, int LB, int LC, int LD, typename R>
+__device__ __forceinline__ void digest_coop(const KParams &kp, const QGeom<R> &g, R *base, int wstride, R *buf, int nl,
+                                            int W, unsigned qmask, R scale, const R *__restrict__ D, double *Jh,
+                                            double *Kh) {
+  using Q = QC<LA, LB, LC, LD>;
+  if constexpr (!std::is_same<R, float>::value) {
+    if (nl == 32 && W % (kBlock / 32) == 0) {   // the same for the whole CTA
+      __syncthreads();
+      for (int o = threadIdx.x; o < Q::NABCD; o += kBlock) {
+        R v = base[o];
+#pragma unroll
+        for (int c = 1; c < kBlock / 32; ++c) v += base[c * wstride + o];
+        base[o] = v;
+      }
+      __syncthreads();
+      digest_grp<LA, LB, LC, LD, R>(kp, g, base, threadIdx.x, kBlock, scale, D, Jh, Kh);
+      return;
+    }
+  }
+  __syncwarp(qmask);
+  digest_grp<LA, LB, LC, LD, R>(kp, g, buf, (int)threadIdx.x % nl, nl, scale, D, Jh, Kh);
+}
+
 template <int LA, int LB, int LC, int LD, typename R, int T>
 __global__ void __launch_bounds__(kBlock) jk_kernel(KParams kp, const __grid_constant__ ClassMulti m,
                                                     const R *__restrict__ D, double *Jh, double *Kh) {
+  using Q = QC<LA, LB, LC, LD>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const int sg = m.find(blockIdx.x);
   const ClassWork w = m.seg[sg];
   const int64_t cta = (int)blockIdx.x - m.cta0[sg];   // among the segment's
@@ -1491,7 +1515,6 @@ __global__ void __launch_bounds__(kBlock) jk_kernel(KParams kp, const __grid_con
   if constexpr (T == 1 && std::is_same<R, float>::value) {
     // FP32 register path: the n-root block of the Rys table is copied to
     // shared memory once per CTA and the CTA strides over the list
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     load_tab32_block(kp, QC<LA, LB, LC, LD>::NR, reinterpret_cast<float4 *>(smem_raw));
     __syncthreads();
     const float *tab_s = reinterpret_cast<const float *>(smem_raw);
@@ -1519,19 +1542,38 @@ __global__ void __launch_bounds__(kBlock) jk_kernel(KParams kp, const __grid_con
   const int lane = threadIdx.x & 31;
   const unsigned qmask = (TP == 32) ? 0xffffffffu : (((1u << TP) - 1u) << (lane & ~(TP - 1)));
   if constexpr (T == 1) {
-    R acc[QC<LA, LB, LC, LD>::NABCD];
+    R acc[Q::NABCD];
     eval_t1<LA, LB, LC, LD, R>(kp, g, acc, sub, W * P);
-    if (P > 1) reduce_psplit<R, QC<LA, LB, LC, LD>::NABCD, 1>(acc, P, qmask);
-    if (p == 0) digest_t1<LA, LB, LC, LD, R>(kp, g, acc, scale, D, Jh, Kh, P == 1 ? i : -1);
+    if (P > 1) reduce_psplit<R, Q::NABCD, 1>(acc, P, qmask);
+    if (P < kCoopLanes) {
+      if (p == 0) digest_t1<LA, LB, LC, LD, R>(kp, g, acc, scale, D, Jh, Kh, P == 1 ? i : -1);
+      return;
+    }
+    R *buf = reinterpret_cast<R *>(smem_raw) + (threadIdx.x / P) * Q::NABCD;
+    if (p == 0) {
+#pragma unroll
+      for (int o = 0; o < Q::NABCD; ++o) buf[o] = acc[o] * (R)Q::norm(o);
+    }
+    digest_coop<LA, LB, LC, LD, R>(kp, g, reinterpret_cast<R *>(smem_raw), Q::NABCD, buf, P, W, qmask, scale, D, Jh,
+                                   Kh);
   } else {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     using GP = Grp<LA, LB, LC, LD, R, T>;
     R *buf = reinterpret_cast<R *>(smem_raw) + (threadIdx.x / T) * GP::BUFN;
     const unsigned gmask = (T == 32) ? 0xffffffffu : (((1u << T) - 1u) << (lane & ~(T - 1)));
     R acc[GP::NPER];
     eval_grp<LA, LB, LC, LD, R, T>(kp, g, buf, t, gmask, acc, sub, W * P);
     if (P > 1) reduce_psplit<R, GP::NPER, T>(acc, P, qmask);
-    if (p == 0) digest_grp<LA, LB, LC, LD, R, T>(kp, g, acc, buf, t, gmask, scale, D, Jh, Kh);
+    __syncwarp(qmask);
+    buf = reinterpret_cast<R *>(smem_raw) + (threadIdx.x / TP) * P * GP::BUFN;   // of the quartet's first group
+    if (p == 0) {
+#pragma unroll
+      for (int k = 0; k < GP::NPER; ++k) {
+        const int o = GP::out(t, k);
+        if (o < Q::NABCD) buf[o] = acc[k] * (R)Q::norm(o);
+      }
+    }
+    digest_coop<LA, LB, LC, LD, R>(kp, g, reinterpret_cast<R *>(smem_raw), (32 / T) * GP::BUFN, buf, TP, W, qmask,
+                                   scale, D, Jh, Kh);
   }
 }
 
