@@ -343,7 +343,7 @@ __device__ __forceinline__ void grad_quartet(const KParams &kp, const ClassWork 
     const int i = a0 + Q::ca(o), j = b0 + Q::cb(o), kk = c0 + Q::cc(o), l = d0 + Q::cd(o);
     const R Dij = ldg_r(D + i * n + j), Dkl = ldg_r(D + kk * n + l), Dik = ldg_r(D + i * n + kk);
     const R Djl = ldg_r(D + j * n + l), Dil = ldg_r(D + i * n + l), Djk = ldg_r(D + j * n + kk);
-    return scale * (R)Q::norm(o) * ((R)0.5 * Dij * Dkl - (R)0.125 * (Dik * Djl + Dil * Djk));
+    return scale * Q::template norm_r<R>(o) * ((R)0.5 * Dij * Dkl - (R)0.125 * (Dik * Djl + Dil * Djk));
   };
   R gA[3] = {0, 0, 0}, gB[3] = {0, 0, 0}, gC[3] = {0, 0, 0};
   if constexpr (T == 1) {

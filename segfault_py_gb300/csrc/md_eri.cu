@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(kBlock) md_eri_kernel(KParams kp, EriWork w) {
   double *out = w.out + w.out_off[q];
 #pragma unroll 1
   for (int o = 0; o < Q::NABCD; ++o)
-    out[Q::ca(o) * s0 + Q::cb(o) * s1 + Q::cc(o) * s2 + Q::cd(o) * s3] = to_f64(acc[o] * (R)Q::norm(o));
+    out[Q::ca(o) * s0 + Q::cb(o) * s1 + Q::cc(o) * s2 + Q::cd(o) * s3] = to_f64(acc[o] * Q::template norm_r<R>(o));
 }
 
 // host copy of the Hermite tables into constant memory (once per device)

@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kTcThreads) md_tc_kernel(KParams kp, EriWork w
       for (int c = 0; c < NCD; ++c) {
         const int ic = c / Q::ND, id = c % Q::ND;
         const int o = r * NCD + c;
-        out[ia * s0 + ib * s1 + ic * s2 + id * s3] = (double)(dv[c] * (float)Q::norm(o));
+        out[ia * s0 + ib * s1 + ic * s2 + id * s3] = (double)(dv[c] * Q::template norm_r<float>(o));
       }
     }
     tc_fence_before();

@@ -449,6 +449,36 @@ struct QC {
   __host__ __device__ static constexpr double norm(int o) {
     return cart_norm(LA, ca(o)) * cart_norm(LB, cb(o)) * cart_norm(LC, cc(o)) * cart_norm(LD, cd(o));
   }
+  // norm(o) in the kernel's arithmetic: sqrt(3) to the number of factors that have
+  // one.  Evaluated from o at run time (group kernels) the products above are
+  // three FP64 multiplications and conversions per output, on a pipe 64 times
+  // slower than the FP32 and double-float sums that they scale (C20H42 6-31G**:
+  // (22|20) FP32 0.202 -> 0.165 ms, double-float 0.88 -> 0.79, (21|21) 2.43 -> 2.10).
+  template <typename R>
+  __host__ __device__ static R norm_r(int o) {
+    constexpr double s = cart_norm(2, 1);
+    constexpr double p[5] = {1.0, s, s * s, s * s * s, s * s * s * s};
+    constexpr int D = (LA == 2) + (LB == 2) + (LC == 2) + (LD == 2);
+    const int m = (cart_norm(LA, ca(o)) != 1.0) + (cart_norm(LB, cb(o)) != 1.0) + (cart_norm(LC, cc(o)) != 1.0) +
+                  (cart_norm(LD, cd(o)) != 1.0);
+    if constexpr (std::is_same<R, dd>::value) {
+      constexpr float h[5] = {(float)p[0], (float)p[1], (float)p[2], (float)p[3], (float)p[4]};
+      constexpr float l[5] = {(float)(p[0] - (double)h[0]), (float)(p[1] - (double)h[1]), (float)(p[2] - (double)h[2]),
+                              (float)(p[3] - (double)h[3]), (float)(p[4] - (double)h[4])};
+      float vh = h[0], vl = l[0];
+#pragma unroll
+      for (int k = 1; k <= D; ++k) {
+        vh = m == k ? h[k] : vh;
+        vl = m == k ? l[k] : vl;
+      }
+      return dd(vh, vl);
+    } else {
+      R v = (R)p[0];
+#pragma unroll
+      for (int k = 1; k <= D; ++k) v = m == k ? (R)p[k] : v;
+      return v;
+    }
+  }
 };
 
 // The recurrences of rys_2d in double-float: every product that is added to
@@ -1219,7 +1249,7 @@ __device__ __forceinline__ void digest_t1(const KParams &kp, const QGeom<R> &g, 
   const int a0 = g.a0, b0 = g.b0, c0 = g.c0, d0 = g.d0;
   R v[Q::NABCD];
 #pragma unroll
-  for (int o = 0; o < Q::NABCD; ++o) v[o] = acc[o] * (R)Q::norm(o);
+  for (int o = 0; o < Q::NABCD; ++o) v[o] = acc[o] * Q::template norm_r<R>(o);
   // J_ab and K blocks need D of the other pairs.  J_ab: with one quartet per
   // lane (bra_key >= 0) the lanes sharing the bra pair add their J_ab first
   R sj[Q::NA * Q::NB];
@@ -1552,7 +1582,7 @@ __global__ void __launch_bounds__(kBlock) jk_kernel(KParams kp, const __grid_con
     R *buf = reinterpret_cast<R *>(smem_raw) + (threadIdx.x / P) * Q::NABCD;
     if (p == 0) {
 #pragma unroll
-      for (int o = 0; o < Q::NABCD; ++o) buf[o] = acc[o] * (R)Q::norm(o);
+      for (int o = 0; o < Q::NABCD; ++o) buf[o] = acc[o] * Q::template norm_r<R>(o);
     }
     digest_coop<LA, LB, LC, LD, R>(kp, g, reinterpret_cast<R *>(smem_raw), Q::NABCD, buf, P, W, qmask, scale, D, Jh,
                                    Kh);
@@ -1569,7 +1599,7 @@ __global__ void __launch_bounds__(kBlock) jk_kernel(KParams kp, const __grid_con
 #pragma unroll
       for (int k = 0; k < GP::NPER; ++k) {
         const int o = GP::out(t, k);
-        if (o < Q::NABCD) buf[o] = acc[k] * (R)Q::norm(o);
+        if (o < Q::NABCD) buf[o] = acc[k] * Q::template norm_r<R>(o);
       }
     }
     digest_coop<LA, LB, LC, LD, R>(kp, g, reinterpret_cast<R *>(smem_raw), (32 / T) * GP::BUFN, buf, TP, W, qmask,
@@ -1609,7 +1639,7 @@ __device__ __forceinline__ void eri_t1_quartet(const KParams &kp, const EriWork 
   double *out = w.out + w.out_off[q];
 #pragma unroll
   for (int o = 0; o < Q::NABCD; ++o)
-    out[Q::ca(o) * s0 + Q::cb(o) * s1 + Q::cc(o) * s2 + Q::cd(o) * s3] = to_f64(acc[o] * (R)Q::norm(o));
+    out[Q::ca(o) * s0 + Q::cb(o) * s1 + Q::cc(o) * s2 + Q::cd(o) * s3] = to_f64(acc[o] * Q::template norm_r<R>(o));
 }
 
 // CTA rank and size of the launch's clusters (1 without the launch attribute)
@@ -1649,7 +1679,7 @@ __device__ __forceinline__ void eri_store_cta(const EriWork &w, int64_t q, R *bu
   const int s0 = w.strides[4 * q], s1 = w.strides[4 * q + 1], s2 = w.strides[4 * q + 2], s3 = w.strides[4 * q + 3];
   double *out = w.out + w.out_off[q];
   auto store = [&](int o, R v) {
-    out[Q::ca(o) * s0 + Q::cb(o) * s1 + Q::cc(o) * s2 + Q::cd(o) * s3] = to_f64(v * (R)Q::norm(o));
+    out[Q::ca(o) * s0 + Q::cb(o) * s1 + Q::cc(o) * s2 + Q::cd(o) * s3] = to_f64(v * Q::template norm_r<R>(o));
   };
   for (int o = threadIdx.x; o < Q::NABCD; o += kBlock) {
     R v = buf[o];
@@ -1751,7 +1781,7 @@ __global__ void __launch_bounds__(kBlock) eri_kernel(KParams kp, EriWork w) {
     for (int k = 0; k < GP::NPER; ++k) {
       const int o = GP::out(t, k);
       if (o < Q::NABCD)
-        out[Q::ca(o) * s0 + Q::cb(o) * s1 + Q::cc(o) * s2 + Q::cd(o) * s3] = to_f64(acc[k] * (R)Q::norm(o));
+        out[Q::ca(o) * s0 + Q::cb(o) * s1 + Q::cc(o) * s2 + Q::cd(o) * s3] = to_f64(acc[k] * Q::template norm_r<R>(o));
     }
   }
 }
@@ -1772,7 +1802,7 @@ __global__ void __launch_bounds__(kBlock) schwarz_kernel(KParams kp, int p0, int
     eval_t1<LA, LB, LA, LB, R>(kp, g, acc);
 #pragma unroll
     for (int o = 0; o < Q::NABCD; ++o)
-      if (Q::ca(o) == Q::cc(o) && Q::cb(o) == Q::cd(o)) m = fmax(m, fabs((double)(acc[o] * (R)Q::norm(o))));
+      if (Q::ca(o) == Q::cc(o) && Q::cb(o) == Q::cd(o)) m = fmax(m, fabs((double)(acc[o] * Q::template norm_r<R>(o))));
   } else {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using GP = Grp<LA, LB, LA, LB, R, T>;
@@ -1784,7 +1814,7 @@ __global__ void __launch_bounds__(kBlock) schwarz_kernel(KParams kp, int p0, int
     for (int k = 0; k < GP::NPER; ++k) {
       const int o = GP::out(t, k);
       if (o < Q::NABCD && Q::ca(o) == Q::cc(o) && Q::cb(o) == Q::cd(o))
-        m = fmax(m, fabs((double)(acc[k] * (R)Q::norm(o))));
+        m = fmax(m, fabs((double)(acc[k] * Q::template norm_r<R>(o))));
     }
 #pragma unroll
     for (int sft = T / 2; sft > 0; sft >>= 1) m = fmax(m, __shfl_xor_sync(gmask, m, sft, T));
