@@ -1057,7 +1057,7 @@ struct Grp {
   static constexpr int BUFN = stride();
 };
 
-template <int LA, int LB, int LC, int LD, typename R, int T>
+template <int LA, int LB, int LC, int LD, typename R, int T, bool ROLL = false>
 __device__ __forceinline__ void eval_grp(const KParams &kp, const QGeom<R> &g, R *tab, int t, unsigned gmask,
                                          R (&acc)[Grp<LA, LB, LC, LD, R, T>::NPER], int p = 0, int P = 1) {
   using Q = QC<LA, LB, LC, LD>;
@@ -1127,6 +1127,32 @@ __device__ __forceinline__ void eval_grp(const KParams &kp, const QGeom<R> &g, R
       }
     }
     __syncwarp(gmask);
+    // ROLL (the J/K kernels): one root's products per trip.  All roots unrolled is
+    // up to 5 times the code for the same sums; a build runs many classes side by
+    // side on an SM, each through its instructions once or a few times.  Hexane
+    // 6-31G* double-float 1.83 -> 1.78 ms, FP64 4.32 -> 4.17; (H2O)8 FP32 +
+    // double-float 1.116 -> 1.086, FP64 3.91 -> 3.81.  The Schwarz kernel keeps its
+    // order of summation: the last bits of the bounds order equal pairs.
+    if constexpr (ROLL && INNER == 1) {
+#pragma unroll 1
+      for (int r = 0; r < NR; ++r) {
+        const R *tr = tab + r * SZ;
+#pragma unroll
+        for (int j = 0; j < RPER; ++j) {
+          if (t + j * T < GP::ROWS) {
+            const R x = tr[off[j] & 1023], y = tr[(off[j] >> 10) & 1023], z = tr[off[j] >> 20];
+            if constexpr (std::is_same<R, dd>::value) dd_acc(acc[j], dd_mul_raw(x, y), z);
+            else acc[j] += x * y * z;
+          }
+        }
+      }
+      if constexpr (std::is_same<R, dd>::value) {
+#pragma unroll
+        for (int j = 0; j < RPER; ++j) acc[j] = dd_norm(acc[j]);
+      }
+      __syncwarp(gmask);
+      continue;
+    }
 #pragma unroll
     for (int j = 0; j < RPER; ++j) {
       if (t + j * T < GP::ROWS) {
@@ -1591,7 +1617,7 @@ __global__ void __launch_bounds__(kBlock) jk_kernel(KParams kp, const __grid_con
     R *buf = reinterpret_cast<R *>(smem_raw) + (threadIdx.x / T) * GP::BUFN;
     const unsigned gmask = (T == 32) ? 0xffffffffu : (((1u << T) - 1u) << (lane & ~(T - 1)));
     R acc[GP::NPER];
-    eval_grp<LA, LB, LC, LD, R, T>(kp, g, buf, t, gmask, acc, sub, W * P);
+    eval_grp<LA, LB, LC, LD, R, T, true>(kp, g, buf, t, gmask, acc, sub, W * P);
     if (P > 1) reduce_psplit<R, GP::NPER, T>(acc, P, qmask);
     __syncwarp(qmask);
     buf = reinterpret_cast<R *>(smem_raw) + (threadIdx.x / TP) * P * GP::BUFN;   // of the quartet's first group
