@@ -277,6 +277,17 @@ __device__ __forceinline__ float acc_value(float v, float) { return v; }
 template <typename V>
 __device__ __forceinline__ double acc_value(V v, double) { return to_f64(v); }
 
+// one-lane classes: primitive sub-groups per quartet from which they share its G_o
+constexpr int kGradCoop = 4;
+// shared memory before the CTA's sums: the groups' buffers, or the G_o of the
+// quartets of a one-lane class with kGradCoop or more lanes each
+template <int LA, int LB, int LC, int LD, typename R, int T>
+__host__ __device__ constexpr size_t grad_buf_bytes() {
+  const size_t n = T == 1 ? (size_t)(kBlock / kGradCoop) * QC<LA, LB, LC, LD>::NABCD
+                          : (size_t)(kBlock / T) * GGrp<LA, LB, LC, LD, R, T>::BUFN;
+  return (n * sizeof(R) + 7) / 8 * 8;
+}
+
 template <int LA, int LB, int LC, int LD, typename R, int T>
 __global__ void __launch_bounds__(kBlock) grad_kernel(KParams kp, const __grid_constant__ ClassMulti m,
                                                       const R *__restrict__ D, double *grad) {
@@ -284,10 +295,9 @@ __global__ void __launch_bounds__(kBlock) grad_kernel(KParams kp, const __grid_c
   const ClassWork w = m.seg[sg];
   const int64_t cta = (int)blockIdx.x - m.cta0[sg];
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  using GP0 = GGrp<LA, LB, LC, LD, R, T>;
   using A = GradAcc<R>;
   const bool cta_sum = kp.natom <= kGradSmemAtoms;
-  A *sgrad = reinterpret_cast<A *>(smem_raw + (T == 1 ? 0 : (size_t)(kBlock / T) * GP0::BUFN * sizeof(R)));
+  A *sgrad = reinterpret_cast<A *>(smem_raw + grad_buf_bytes<LA, LB, LC, LD, R, T>());
   const int TP0 = T * w.psplit;
   const int64_t nq = work_count(w);
   const int64_t qfirst = (cta * (kBlock / TP0)) / w.wsplit;
@@ -335,8 +345,12 @@ __device__ __forceinline__ void grad_quartet(const KParams &kp, const ClassWork 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R *tab = reinterpret_cast<R *>(smem_raw) + (threadIdx.x / T) * GP::BUFN;
 
-  // G_o (normalised, permutation count folded in): in registers (T == 1) or,
-  // outputs t, t+T, ..., into the group's buffer
+  // G_o (normalised, permutation count folded in).  The primitive sub-groups of a
+  // quartet share them: each of the TP lanes evaluates outputs TP apart into the
+  // buffer of the first group (six density elements and nine operations each, per
+  // lane of every sub-group as much as one primitive quartet's contraction);
+  // T == 1 then keeps them in registers.  Forces of (H2O)4 6-31G* double-float
+  // 2.20 -> 2.17 ms.
   const int n = kp.nao;
   const int a0 = g.a0, b0 = g.b0, c0 = g.c0, d0 = g.d0;
   auto gamma = [&](int o) {
@@ -348,11 +362,21 @@ __device__ __forceinline__ void grad_quartet(const KParams &kp, const ClassWork 
   R gA[3] = {0, 0, 0}, gB[3] = {0, 0, 0}, gC[3] = {0, 0, 0};
   if constexpr (T == 1) {
     R gam[Q::NABCD];
+    if (P >= kGradCoop) {
+      R *sg = reinterpret_cast<R *>(smem_raw) + (threadIdx.x / P) * Q::NABCD;
+      for (int o = pl; o < Q::NABCD; o += P) sg[o] = gamma(o);
+      __syncwarp(qmask);
 #pragma unroll
-    for (int o = 0; o < Q::NABCD; ++o) gam[o] = gamma(o);
+      for (int o = 0; o < Q::NABCD; ++o) gam[o] = sg[o];
+    } else {
+#pragma unroll
+      for (int o = 0; o < Q::NABCD; ++o) gam[o] = gamma(o);
+    }
     grad_t1<LA, LB, LC, LD, R>(kp, g, gam, sub, W * P, gA, gB, gC);
   } else {
-  for (int o = t; o < Q::NABCD; o += T) tab[GP::GAM + o] = gamma(o);
+  R *gam = reinterpret_cast<R *>(smem_raw) + (threadIdx.x / TP) * P * GP::BUFN + GP::GAM;
+  for (int o = (int)threadIdx.x % TP; o < Q::NABCD; o += TP) gam[o] = gamma(o);
+  __syncwarp(qmask);
   const int2 *hdr = kp.grad_hdr + grad_tab_index<LA, LB, LC, LD, R>() * 3;   // {offset, steps} per direction
   const int nprim = g.ab_n * g.cd_n;
   int cur = -1;
@@ -414,7 +438,7 @@ __device__ __forceinline__ void grad_quartet(const KParams &kp, const ClassWork 
       for (int k = 0; k < h.y; ++k) {
         const uint2 e = __ldg(work + k * T);
         if (e.x == ~0u) break;
-        const R gm = tab[GP::GAM + (e.x & 2047u)];
+        const R gm = gam[e.x & 2047u];
         const R *p1 = t1 + ((e.x >> 11) & 255u), *p2 = t2 + ((e.x >> 19) & 255u);
 #pragma unroll
         for (int r = 0; r < NR; ++r) grad_acc(F[r], grad_mul(gm, p1[r * SZ]), p2[r * SZ]);
@@ -456,7 +480,45 @@ __device__ __forceinline__ void grad_quartet(const KParams &kp, const ClassWork 
     }
   }
   }
-  // sum over the T x P lanes of the quartet
+  // sum over the T x P lanes of the quartet.  Eight or more lanes halve the values
+  // with every exchange (12 -> 6 -> 3 -> 2 -> 1, a lane adds up the ones that it keeps: 13
+  // additions and 6 for centre D, instead of 45 and 6) and the lanes that hold
+  // the totals add them to the forces side by side.  Forces of (H2O)8 6-31G* FP32 +
+  // double-float 4.82 -> 4.67 ms, (H2O)2 FP64 1.14 -> 1.11.
+  if (TP >= 8) {
+    R v[12];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      v[d] = gA[d];
+      v[3 + d] = gB[d];
+      v[6 + d] = gC[d];
+      v[9 + d] = -(gA[d] + gB[d] + gC[d]);
+    }
+    const bool h1 = lane & 1, h2 = lane & 2, h4 = lane & 4, h8 = lane & 8;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) v[k] = (h1 ? v[6 + k] : v[k]) + shfl_xor_r(qmask, h1 ? v[k] : v[6 + k], 1);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[k] = (h2 ? v[3 + k] : v[k]) + shfl_xor_r(qmask, h2 ? v[k] : v[3 + k], 2);
+    const R x0 = shfl_xor_r(qmask, h4 ? v[0] : v[2], 4), x1 = shfl_xor_r(qmask, v[1], 4);
+    v[0] = (h4 ? v[2] : v[0]) + x0;   // values 0, 1 of three, or value 2
+    v[1] = v[1] + x1;
+    int i = (h1 ? 6 : 0) + (h2 ? 3 : 0) + (h4 ? 2 : 0), nv = h4 ? 1 : 2;
+    if (TP >= 16) {
+      const R x = shfl_xor_r(qmask, h8 ? v[0] : v[1], 8);
+      v[0] = (h8 ? v[1] : v[0]) + x;
+      nv = h8 && h4 ? 0 : 1;
+      i += h8;
+    }
+    if (TP == 32) {
+      v[0] = v[0] + shfl_xor_r(qmask, v[0], 16);
+      if (lane & 16) nv = 0;
+    }
+    for (int k = 0; k < nv; ++k, ++i) {
+      const int at = kp.sh.atom[i < 3 ? g.a : i < 6 ? g.b : i < 9 ? g.c : g.d];
+      atomicAdd(grad + 3 * at + i % 3, acc_value(k ? v[1] : v[0], A()));
+    }
+    return;
+  }
 #pragma unroll
   for (int d = 0; d < 3; ++d)
     for (int sft = 1; sft < TP; sft <<= 1) {
@@ -517,8 +579,7 @@ inline bool grad_segments(ClassMulti &m, const ClassWork *w, int nw, int T) {
 template <int LA, int LB, int LC, int LD, typename R>
 constexpr size_t grad_smem() {
   constexpr int T = tgrad_r<R>(QC<LA, LB, LC, LD>::NABCD);
-  return (T == 1 ? 0 : (size_t)(kBlock / T) * GGrp<LA, LB, LC, LD, R, T>::BUFN * sizeof(R)) +
-         3 * kGradSmemAtoms * sizeof(double);
+  return grad_buf_bytes<LA, LB, LC, LD, R, T>() + 3 * kGradSmemAtoms * sizeof(double);
 }
 
 }  // namespace sf
