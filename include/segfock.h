@@ -325,6 +325,13 @@ int sf_grad_stats(sf_handle *h, sf_stats *stats, void *stream);
 int sf_grad_one_electron(sf_handle *h, const double *atom_xyz, const double *charges, int32_t natom,
                          const double *D, const double *W, double *grad, void *stream);
 
+/* Both: sf_grad_one_electron beside sf_grad_jk (grad accumulated), the
+ * one-electron kernel on a stream of the handle's own that is forked from
+ * `stream` and joined back into it. */
+int sf_grad_rhf(sf_handle *h, const double *atom_xyz, const double *charges, int32_t natom,
+                const double *D, const double *W, double *grad, int32_t precision, double cutoff,
+                double fp32_cutoff, void *stream);
+
 /* Per-launch profiling of sf_fock_jk.  on = 1: every class kernel of a Fock
  * build is bracketed by CUDA events on the stream it runs on (class launches
  * run concurrently on streams forked from the caller's, so these times

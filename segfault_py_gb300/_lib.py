@@ -21,7 +21,7 @@ PRECISION = {"fp64": SF_PREC_FP64, "fp32": SF_PREC_FP32, "mixed": SF_PREC_MIXED,
 
 EXPORTS = ["sf_version", "sf_last_error", "sf_create", "sf_build_shells", "sf_destroy", "sf_nao", "sf_npairs",
            "sf_schwarz", "sf_fock_jk", "sf_set_partition", "sf_eri_batch", "sf_one_electron", "sf_rys_roots_host", "sf_set_profiling", "sf_slice_count", "sf_get_slice_info",
-           "sf_fma_peak", "sf_fock_jk_noalloc", "sf_grad_jk", "sf_grad_one_electron",
+           "sf_fma_peak", "sf_fock_jk_noalloc", "sf_grad_jk", "sf_grad_one_electron", "sf_grad_rhf",
            "sf_small_solve", "sf_eri_plan_create", "sf_eri_plan_info", "sf_eri_plan_offsets", "sf_eri_plan_run",
            "sf_eri_plan_destroy", "sf_autotune", "sf_tuning_count", "sf_get_tuning", "sf_set_tuning", "sf_eri_plan_run_md",
            "sf_set_density_screening", "sf_set_launch_mode", "sf_fock_jk_graph_create", "sf_fock_graph_launch",
@@ -109,6 +109,7 @@ def lib():
     L.sf_fock_jk_noalloc.argtypes = [p, p, p, p, i32, d, d, p]
     L.sf_grad_jk.argtypes = [p, p, p, i32, d, d, p]
     L.sf_grad_one_electron.argtypes = [p, p, p, i32, p, p, p, p]
+    L.sf_grad_rhf.argtypes = [p, p, p, i32, p, p, p, i32, d, d, p]
     L.sf_small_solve.argtypes = [i32, p, p, p, p, p]
     L.sf_eri_plan_create.argtypes = [p, p, i64, C.POINTER(p)]
     L.sf_eri_plan_info.argtypes = [p, p, p, p]

@@ -7,8 +7,8 @@ The reference computes energies only.  Here
     G_pqrs = 1/2 D_pq D_rs - 1/8 (D_pr D_qs + D_ps D_qr),
     W = 2 sum_occ e_i C_pi C_qi = (D F D)/2 at the converged density,
 
-with the derivative integrals contracted on the GPU (sf_grad_one_electron,
-sf_grad_jk) and the nuclear term on the host.  ``RHFEnergy`` wraps the SCF
+with the derivative integrals contracted on the GPU (sf_grad_rhf: the one-
+electron kernel beside the two-electron ones) and the nuclear term on the host.  ``RHFEnergy`` wraps the SCF
 energy as a torch.autograd.Function whose backward returns these forces.
 Coordinates are in bohr, gradients in Eh/bohr.
 """
@@ -57,16 +57,13 @@ def rhf_gradient(mol: Molecule, res: SCFResult, fb: FockBuilder, precision: str 
     xyz, Z = mol.atom_table()
     xyz_d = torch.as_tensor(xyz, device=dev)
     Z_d = torch.as_tensor(Z, device=dev)
-    g = torch.zeros(mol.natom * 3, dtype=torch.float64, device=dev)
+    g = torch.as_tensor(nuclear_repulsion_gradient(mol).ravel(), device=dev)   # the kernels add to it
     prec = _lib.PRECISION[precision or fb.precision]
     with torch.cuda.device(dev):
-        st = _stream_ptr()
-        _lib.check(L.sf_grad_one_electron(fb.handle, _ptr(xyz_d), _ptr(Z_d), mol.natom, _ptr(D), _ptr(W), _ptr(g),
-                                          st))
-        _lib.check(L.sf_grad_jk(fb.handle, _ptr(D), _ptr(g), prec, fb.cutoff if cutoff is None else cutoff,
-                                fb.fp32_cutoff if fp32_cutoff is None else fp32_cutoff, st))
-    g = g.view(mol.natom, 3) + torch.as_tensor(nuclear_repulsion_gradient(mol), device=dev)
-    return g
+        _lib.check(L.sf_grad_rhf(fb.handle, _ptr(xyz_d), _ptr(Z_d), mol.natom, _ptr(D), _ptr(W), _ptr(g), prec,
+                                 fb.cutoff if cutoff is None else cutoff,
+                                 fb.fp32_cutoff if fp32_cutoff is None else fp32_cutoff, _stream_ptr()))
+    return g.view(mol.natom, 3)
 
 
 class RHFEnergy(torch.autograd.Function):

@@ -96,6 +96,32 @@ def test_one_electron_gradient_layouts(cuda, nprim, extra):
         assert abs(fd - g[a, k]) <= 1e-6 * np.abs(g).max(), (a, k, fd, g[a, k])
 
 
+@pytest.mark.parametrize("profiling", [0, 2])
+@pytest.mark.parametrize("precision", ["fp64", "df"])
+def test_gradient_parts_side_by_side(cuda, precision, profiling):
+    """sf_grad_rhf adds what sf_grad_one_electron and sf_grad_jk add, in another order: fewer than 1e5
+    terms of at most the largest force each in FP64 (double-float: 2^-44 each), 1e-11 of the largest."""
+    from segfault_py_gb300 import _lib
+    from segfault_py_gb300.fock import FockBuilder, _ptr, _stream_ptr
+    ls = [0, 1, 2, 1, 0]
+    table = _table(ls, [2, 1, 1, 3, 2], 4, 2.0)
+    n = sum((l + 1) * (l + 2) // 2 for l in ls)
+    L = _lib.lib()
+    fb = FockBuilder(table, device=cuda, cutoff=0.0)
+    d = [torch.tensor(x, device=cuda) for x in (table["center"], np.arange(1.0, 6.0), _sym(n, 1), _sym(n, 2))]
+    p = [_ptr(x) for x in d]
+    apart, both = (torch.ones(15, dtype=torch.float64, device=cuda) for _ in range(2))
+    prec = _lib.PRECISION[precision]
+    _lib.check(L.sf_grad_one_electron(fb.handle, p[0], p[1], 5, p[2], p[3], _ptr(apart), _stream_ptr()))
+    _lib.check(L.sf_grad_jk(fb.handle, p[2], _ptr(apart), prec, 0.0, 0.0, _stream_ptr()))
+    fb.set_profiling(profiling)
+    _lib.check(L.sf_grad_rhf(fb.handle, p[0], p[1], 5, p[2], p[3], _ptr(both), prec, 0.0, 0.0, _stream_ptr()))
+    assert (both - apart).abs().max() <= 1e-11 * apart.abs().max()
+    with pytest.raises(Exception):   # the shells reference five nuclei
+        _lib.check(L.sf_grad_rhf(fb.handle, p[0], p[1], 4, p[2], p[3], _ptr(both), prec, 0.0, 0.0, _stream_ptr()))
+    fb.close()
+
+
 CLASSES = [(a, b, c, d) for a in range(3) for b in range(a + 1) for c in range(3) for d in range(c + 1)
            if (a * (a + 1) // 2 + b) >= (c * (c + 1) // 2 + d)]
 
