@@ -126,6 +126,28 @@ CLASSES = [(a, b, c, d) for a in range(3) for b in range(a + 1) for c in range(3
            if (a * (a + 1) // 2 + b) >= (c * (c + 1) // 2 + d)]
 
 
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-11), ("df", 1e-11), ("fp32", 3e-5)])
+@pytest.mark.parametrize("cls", CLASSES, ids=lambda c: "%d%d%d%d" % c)
+def test_fock_splits_by_class(cuda, cls, precision, tol):
+    """J and K of four shells of one class against the oracle, for primitive splits from one lane group to
+    more sub-groups than primitive quartets (digestion by one lane, all lanes of a quartet, whole CTAs).
+    D has random signs, so an element's 400 terms add their errors up to 20 times one: 2^-44 (double-float) or
+    less gives 2e-12 of the largest element, 3e-6 per FP32 integral 6e-5 of the largest term, a few of which
+    make an element: 1e-11 and 3e-5."""
+    from segfault_py_gb300.fock import FockBuilder
+    table = _table(list(cls), [3, 2, 2, 3], 40 + sum(3 ** i * l for i, l in enumerate(cls)), 2.0)
+    D = _sym(sum((l + 1) * (l + 2) // 2 for l in cls), 3)
+    J, K = O.jk_direct(_cgfs(table), D)
+    fb = FockBuilder(table, device=cuda, cutoff=0.0, precision=precision)
+    Dd = torch.tensor(D, device=cuda)
+    for split in (1, 2, 4, 8, 32, 128, 512):
+        fb.set_tuning([dict(cls=c, precision=k, cost=n, split=split, ms_default=0.0, ms_tuned=0.0)
+                       for c in range(21) for k in range(3) for n in range(1, 82)])
+        for got, ref in zip(fb.jk(Dd), (J, K)):
+            assert np.abs(got.cpu().numpy() - ref).max() <= tol * np.abs(ref).max(), split
+    fb.close()
+
+
 @pytest.mark.parametrize("precision,tol", [("fp64", 1e-6), ("df", 1e-6), ("fp32", 1e-4)])
 @pytest.mark.parametrize("cls", CLASSES, ids=lambda c: "%d%d%d%d" % c)
 def test_two_electron_gradient_by_class(cuda, cls, precision, tol):
