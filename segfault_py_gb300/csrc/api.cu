@@ -629,11 +629,16 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
   h->st_q[0] = h->st_q[1] = h->st_pq[0] = h->st_pq[1] = 0;
   h->st_f[0] = h->st_f[1] = 0.0;
   h->st_total = 0;
-  constexpr int KB = kMaxPrim * kMaxPrim + 1;   // primitive pairs per shell pair <= 256
+  int KB = 1;   // more than the primitive pairs of any shell pair
+  for (int i = 0; i < h->cstart[kNumPairClass]; ++i) KB = std::max(KB, h->pair_full(i) + 1);
   // every class's lists are cut independently, on host threads, then
   // concatenated in class order (the result does not depend on the threads)
+  struct Run {   // the quartets of equal (K_ab, K_cd) in a list
+    int64_t cost, end, prims;   // K_ab K_cd, one past the last, full primitive quartets
+  };
   struct Part {   // the list of one (class, tier), offsets relative to it
     std::vector<int2> lst;
+    std::vector<Run> runs;
     std::vector<Pending> segs;
     int64_t q = 0, pq = 0;
     double f = 0.0;
@@ -643,7 +648,7 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
   std::vector<Part> parts(3 * kNumClass);   // per class: accurate tier, FP32, double-float part of FP64
   std::vector<int64_t> totals(kNumClass, 0);
   double load32 = 0.0;          // estimated operations of the FP32 tier
-  auto build_class = [&](int cls, std::vector<int64_t> &hist) {
+  auto build_class = [&](int cls, std::vector<int64_t> &hist, std::vector<int64_t> &full) {
     const ClassInfo &ci = kClassInfo[cls];
     const int X = pair_class_of(ci.la, ci.lb), Y = pair_class_of(ci.lc, ci.ld);
     const int x0 = h->cstart[X], y0 = h->cstart[Y];
@@ -687,16 +692,16 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
       auto npair = [&](int i) { return pr == 1 ? h->pair_full(i) : h->pnp[i]; };
       // counting sort on (K_ab, K_cd); prims: the full count, for the statistics
       std::fill(hist.begin(), hist.end(), 0);
+      std::fill(full.begin(), full.end(), 0);
       int64_t n = 0, prims = 0;
       for (int i = 0; i < nX; ++i) {
         const int64_t lo = from ? (*from)[i] : 0, hi = upto[i];
-        const int ka = npair(x0 + i);
-        int64_t kf = 0;
+        const int64_t ka = npair(x0 + i), kf = h->pair_full(x0 + i);
         for (int64_t j = lo; j < hi; ++j) {
-          ++hist[(size_t)ka * KB + npair(y0 + (int)j)];
-          kf += h->pair_full(y0 + (int)j);
+          const size_t k = (size_t)ka * KB + npair(y0 + (int)j);
+          ++hist[k];
+          full[k] += kf * h->pair_full(y0 + (int)j);
         }
-        prims += kf * h->pair_full(x0 + i);
         n += hi - lo;
       }
       if (n == 0) continue;
@@ -708,12 +713,15 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
         return ca != cb ? ca > cb : a > b;
       });
       std::vector<int64_t> pos((size_t)KB * KB, 0);
+      std::vector<Run> runs;
       int64_t run = 0;
       double costs = 0.0;
       for (int k : keys) {
         pos[k] = run;
         run += hist[k];
+        prims += full[k];
         costs += (double)hist[k] * (k / KB) * (k % KB);
+        runs.push_back({(int64_t)(k / KB) * (k % KB), run, full[k]});
       }
       std::vector<int2> lst(n);
       for (int i = 0; i < nX; ++i) {
@@ -738,6 +746,12 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
         int64_t kept = 0;
         for (int64_t q = h->part; q < n; q += h->nparts) lst[kept++] = lst[q];
         lst.resize(kept);
+        int64_t q = 0;
+        for (Run &ru : runs) {
+          ru.end = ru.end > h->part ? (ru.end - 1 - h->part) / h->nparts + 1 : 0;
+          for (ru.prims = 0; q < ru.end; ++q)
+            ru.prims += (int64_t)h->pair_full(x0 + lst[q].x) * h->pair_full(y0 + lst[q].y);
+        }
       }
       const double frac = (double)lst.size() / (double)n;
       p.n = (int64_t)lst.size();
@@ -751,6 +765,7 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
       part.per_prim = nr * (nabcd + 30.0) + 40.0;
       part.load = costs * frac * part.per_prim;
       part.lst = std::move(lst);
+      part.runs = std::move(runs);
     }
   };
   // Cut the cost-sorted list of (class, tier) into segments with S = P*W
@@ -769,12 +784,10 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     Part &part = parts[3 * cls + pr];
     const Pending &p = part.head;
     if (part.lst.empty()) return;
-    const std::vector<int2> &lst = part.lst;
     const ClassInfo &ci = kClassInfo[cls];
-    const int x0 = p.x0, y0 = p.y0, kind = p.prec;
+    const int kind = p.prec;
     const int nr = (ci.la + ci.lb + ci.lc + ci.ld) / 2 + 1;
     const double nabcd = (double)ncart(ci.la) * ncart(ci.lb) * ncart(ci.lc) * ncart(ci.ld);
-    auto npair = [&](int i) { return pr == 1 ? h->pair_full(i) : h->pnp[i]; };
     const int T = kind_lanes(ci, kind, p.wide);
     const int pmax = 32 / T;
     auto psplit = [&](int64_t cost) {
@@ -796,24 +809,29 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
       while (2 * sc <= cost && 2 * sc <= sfill && (double)cost * part.per_prim / T > share * sc) sc *= 2;
       return std::max(psplit(cost), sc);
     };
-    const auto cost_of = [&](int64_t q) { return (int64_t)npair(x0 + lst[q].x) * npair(y0 + lst[q].y); };
     int64_t q0 = 0;
-    while (q0 < p.n) {
-      const int S = split_of(cost_of(q0));
-      int64_t q1 = q0 + 1;
-      while (q1 < p.n && split_of(cost_of(q1)) == S) ++q1;
+    for (size_t r = 0; r < part.runs.size();) {
+      const int64_t cost = part.runs[r].cost;
+      if (part.runs[r].end == q0) {   // none of its quartets in this partition
+        ++r;
+        continue;
+      }
+      const int S = split_of(cost);
+      int64_t q1 = q0, sp = 0;
+      for (; r < part.runs.size() && split_of(part.runs[r].cost) == S; ++r) {
+        q1 = part.runs[r].end;
+        sp += part.runs[r].prims;
+      }
       Pending seg = p;
       seg.off = q0;
       seg.n = q1 - q0;
-      seg.cost_hi = cost_of(q0);
+      seg.cost_hi = cost;
       seg.rel_load = load[kind] > 0.0 ? (float)(part.per_prim * lanes / load[kind]) : 0.0f;
       int St = S;
       for (const sf_tune_entry &e : h->tune)
         if (!p.tail && e.cls == cls && e.precision == kind && e.cost == seg.cost_hi) St = e.split;
       seg.psplit = std::min(St, pmax);
       seg.wsplit = std::max(1, std::min(St / seg.psplit, kMaxWsplit));
-      int64_t sp = 0;
-      for (int64_t q = q0; q < q1; ++q) sp += (int64_t)h->pair_full(x0 + lst[q].x) * h->pair_full(y0 + lst[q].y);
       seg.prims = sp;
       seg.flops = (double)sp * nr * 4.0 * nabcd + 12.0 * nabcd * (double)seg.n;
       part.segs.push_back(seg);
@@ -821,12 +839,14 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     }
   };
   {
+    // a thread costs 30 us to start: one for lists that take less to cut
     const unsigned hw = std::thread::hardware_concurrency();
-    const int nthr = std::max(1, std::min<int>(kNumClass, hw ? (int)hw : 1));
+    const double npairs = h->cstart[kNumPairClass];
+    const int nthr = npairs * npairs < 2e5 ? 1 : std::max(1, std::min<int>(kNumClass, hw ? (int)hw : 1));
     std::atomic<int> next{0};
     auto worker = [&]() {
-      std::vector<int64_t> hist((size_t)KB * KB);
-      for (int c = next++; c < kNumClass; c = next++) build_class(c, hist);
+      std::vector<int64_t> hist((size_t)KB * KB), full((size_t)KB * KB);
+      for (int c = next++; c < kNumClass; c = next++) build_class(c, hist, full);
     };
     std::vector<std::thread> pool;
     for (int t = 1; t < nthr; ++t) pool.emplace_back(worker);
@@ -835,14 +855,7 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     double load[3] = {0.0, 0.0, 0.0};   // per arithmetic
     for (const Part &part : parts) load[part.head.prec] += part.load;
     load32 = load[1];
-    next = 0;
-    auto cut = [&]() {
-      for (int c = next++; c < 3 * kNumClass; c = next++) segment(c / 3, c % 3, load);
-    };
-    pool.clear();
-    for (int t = 1; t < nthr; ++t) pool.emplace_back(cut);
-    cut();
-    for (auto &t : pool) t.join();
+    for (int c = 0; c < 3 * kNumClass; ++c) segment(c / 3, c % 3, load);
   }
   for (int cls = 0; cls < kNumClass; ++cls) {
     h->st_total += totals[cls];
