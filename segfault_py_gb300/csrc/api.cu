@@ -777,7 +777,11 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
   //    one primitive quartet.  Long quartets then end with the rest of the
   //    build, and no list is split further than that (with 8 warps per
   //    sub-partition from every list: hexane 6-31G* double-float 2.48 ms, 1.98
-  //    here; (H2O)4 FP64 1.23, 0.89; (H2O)8 FP32 + double-float 1.35, 1.21)
+  //    here; (H2O)4 FP64 1.23, 0.89; (H2O)8 FP32 + double-float 1.35, 1.21).
+  //    Where that leaves two primitive quartets to some sub-groups and one to others
+  //    (81 over 64), a last doubling gives every one its own if the sub-group is
+  //    far above the average (8 times: the GPU is nearly empty): H2O STO-3G FP64
+  //    39 -> 27 us replayed (from the average on: (H2O)2 FP32 + FP64 193 -> 198)
   //  * FP32: S grows until the list by itself has 8 warps per sub-partition (its
   //    rounding depends on S, so it keeps this rule).
   auto segment = [&](int cls, int pr, const double *load) {
@@ -806,7 +810,9 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     }
     auto split_of = [&](int64_t cost) {
       int sc = 1;
-      while (2 * sc <= cost && 2 * sc <= sfill && (double)cost * part.per_prim / T > share * sc) sc *= 2;
+      auto work = [&]() { return (double)cost * part.per_prim / T / sc; };   // of a sub-group
+      while ((2 * sc <= cost || (pr != 1 && sc < cost && work() > 8.0 * share)) && 2 * sc <= sfill && work() > share)
+        sc *= 2;
       return std::max(psplit(cost), sc);
     };
     int64_t q0 = 0;

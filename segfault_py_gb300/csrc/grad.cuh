@@ -553,13 +553,14 @@ __device__ __forceinline__ void grad_quartet(const KParams &kp, const ClassWork 
 // this kernel's T (as many sub-groups as fit in T*P <= 32 lanes, the rest as
 // separate groups), and doubled while a sub-group's estimated work is above a
 // quarter of the average load of the lanes that fill the GPU (rel_load: the Fock
-// kernels' estimate, a derivative quartet costs several times that), at least one
-// primitive quartet of the costliest quartet each.  Filling the GPU with every
+// kernels' estimate, a derivative quartet costs several times that), until the
+// costliest quartet has a sub-group per primitive quartet (with one to two each:
+// (H2O)2 6-31G* forces in FP64 0.99 ms against 0.93 here).  Filling the GPU with every
 // segment by itself instead: (H2O)8 6-31G* forces in FP64 17.3 ms against 15.2
 // here, FP32 + double-float 5.6 against 4.9, nonane 6-31G** 19.5 against 18.3.
 inline ClassWork grad_work(const ClassWork &w, int T) {
   int S = (w.psplit < 1 ? 1 : w.psplit) * (w.wsplit < 1 ? 1 : w.wsplit);
-  while (2 * S <= w.max_cost && 4.0f * (float)w.max_cost * w.rel_load > (float)S * T && 2 * S <= (32 / T) * kMaxWsplit) S *= 2;
+  while (S < w.max_cost && 4.0f * (float)w.max_cost * w.rel_load > (float)S * T && 2 * S <= (32 / T) * kMaxWsplit) S *= 2;
   int P = S;
   while (T * P > 32) P >>= 1;
   ClassWork w2 = w;
