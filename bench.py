@@ -22,7 +22,8 @@ Reported:
                register tier, fed by a device work queue)
 * e2e          same metric through the public API with host buffers: pinned D
                -> device, Fock build, J and K -> pinned host, every step
-* fp64         the all-FP64 build, same protocol (the plain FP64 GPU baseline)
+* fp64         the FP64 mode, same protocol (quartets with small Schwarz bounds in
+               double-float, as that mode runs)
 * mixed_fp32_fp64  the mixed build with native FP64 above the cutoff
 * roofline     dominant class kernel (the (class, precision) kernel with the
                most device time over its launches in one build): algorithmic
@@ -366,8 +367,8 @@ def run_ours(args):
         "fp64": {"value": world * steps / (ms_64 * 1e-3), "unit": "Fock builds/s", "ms_per_step": ms_64 / steps,
                  "quartets_per_s": st_64["quartets_fp64"] * steps / (ms_64 * 1e-3),
                  "flop_alg": st_64["flop_alg_fp64"],
-                 # algorithmic FLOPs per build over its time against the FP64 FMA peak (a lower
-                 # bound: ncu puts the FP64 pipe of its largest kernels at 88-89 % busy)
+                 # algorithmic FLOPs per build over its time against the FP64 FMA peak; the mode's
+                 # quartets with small Schwarz bounds run in double-float, on the FP32 pipe
                  "frac_of_fp64_peak": st_64["flop_alg_fp64"] / (ms_64 / steps * 1e-3) / (peaks["fp64"] * 1e12)},
         "mixed_speedup_vs_fp64": ms_64 / ms_eager,   # both issued eagerly
         "mixed_fp32_fp64": {"value": world * steps / (ms_mx * 1e-3), "unit": "Fock builds/s",
@@ -628,6 +629,8 @@ def eri_batch_config(nq, steps, warmup, flush, dev, peaks):
         res[p] = {"ms": ms, "quartets_per_s": nq / (ms * 1e-3), "prim_quartets_per_s": plan.prim_quartets / (ms * 1e-3),
                   "tflops_alg": plan.flop_alg / (ms * 1e-3) / 1e12,
                   "frac_of_fma_peak": plan.flop_alg / (ms * 1e-3) / 1e12 / peaks[p] if peaks.get(p) else None}
+    res["note"] = ("flop_alg and prim_quartets count the whole contractions; primitive pairs weighted below 1e-20 "
+                   "are left out of the evaluation")
     res["max_abs_diff_fp32_vs_fp64"] = diff
     res["max_abs_fp64"] = amax
     plan.close()

@@ -595,7 +595,8 @@ std::vector<int> lpt_streams(const std::vector<double> &cost_desc, int first = 0
 // the largest bounds (order one) its rounding lies under that of the large
 // quartets, which stay FP64: J and K of (H2O)16 6-31G* differ by 5e-15 of
 // their norm from the all-FP64 build, errors against 64-bit reference values are
-// the same to three digits; 68.0 -> 22.7 ms (everything in FP64: the pipe 88 % busy).
+// the same to three digits; 68.0 -> 22.7 ms when it came, 19.2 with the kernels as
+// they are now (everything in FP64: the pipe 88 % busy).
 constexpr double kDDTail = 1e-3;
 // ... when the class's part below it would hold the FP64 pipe for longer than
 // 20 us (estimated from its primitive quartets as in build_work at the measured
