@@ -604,6 +604,15 @@ constexpr double kDDTail = 1e-3;
 // per class costs (H2O)2 6-31G* 4 % of its 0.37 ms build
 constexpr double kDDTailMinFlops = 20e-6 * 1.25e12;
 
+// Estimated operations of an FP32 + double-float or double-float build below which
+// its double-float launches take the tdd_wide lanes: more lanes per quartet
+// shorten long quartets but repeat their set-up.  FP64 lanes / wide lanes, ms
+// (operations): FP32 + double-float 6-31G* (H2O)2 0.136 / 0.129 (5e7), (H2O)4 0.240 /
+// 0.237 (5e8), butane 0.619 / 0.607 (1e9), hexane 0.98 / 1.03 (3e9), (H2O)8 1.052 /
+// 1.063 (4e9), (H2O)16 4.68 / 4.76, decane 6-31G** 4.20 / 4.51, C20H42 17.95 / 19.28;
+// double-float butane 0.660 / 0.631 (8e8), hexane 1.78 / 1.93 (3e9), (H2O)8 2.60 / 2.90.
+constexpr double kWideMaxLoad = 1.5e9;
+
 // lanes per quartet of a launch of class ci in kind (0 FP64, 1 FP32, 2 dd)
 inline int kind_lanes(const ClassInfo &ci, int kind, int wide) {
   return kind == 1 ? ci.t32 : (kind == 2 && wide) ? tdd_wide(ci.la, ci.lb, ci.lc, ci.ld, ci.t64) : ci.t64;
@@ -731,8 +740,7 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
         for (int64_t j = lo; j < hi; ++j) lst[pos[(size_t)ka * KB + npair(y0 + (int)j)]++] = make_int2(i, (int)j);
       }
       Pending p;
-      // the double-float accurate tier of a mixed build runs its wide kernels
-      p.wide = (kind == 2 && prec == SF_PREC_MIXED_DF) ? 1 : 0;
+      p.wide = 0;
       p.tail = pr == 2 ? 1 : 0;
       p.cost_hi = 0;
       p.psplit = 1;
@@ -862,6 +870,8 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     double load[3] = {0.0, 0.0, 0.0};   // per arithmetic
     for (const Part &part : parts) load[part.head.prec] += part.load;
     load32 = load[1];
+    if (prec == SF_PREC_MIXED_DF || prec == SF_PREC_DF)
+      for (Part &part : parts) part.head.wide = part.head.prec == 2 && load[1] + load[2] < kWideMaxLoad;
     for (int c = 0; c < 3 * kNumClass; ++c) segment(c / 3, c % 3, load);
   }
   for (int cls = 0; cls < kNumClass; ++cls) {

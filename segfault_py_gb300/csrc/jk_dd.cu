@@ -1,7 +1,7 @@
 // jk_dd.cu -- double-float (dd) J/K kernels, per class: the accurate tier of
 // the SF_PREC_MIXED_DF / SF_PREC_DF modes.  Lanes per quartet as the FP64
 // kernels (same register footprint per value); the tdd_wide instantiations
-// for the accurate tier of a mixed build are in jk_dd_wide.cu.
+// for builds too small to fill the GPU are in jk_dd_wide.cu.
 #include "classes.h"
 #include "launch.h"
 
@@ -20,8 +20,8 @@ static cudaError_t run_jk_dd(const KParams &kp, const ClassWork *w, int nw, cons
   return cudaGetLastError();
 }
 
-// wide (the same for all segments) selects the tdd_wide lanes per quartet (the accurate tier of a mixed
-// build; compiled in jk_dd_wide.cu), else the FP64 lanes
+// wide (the same for all segments) selects the tdd_wide lanes per quartet
+// (compiled in jk_dd_wide.cu), else the FP64 lanes
 cudaError_t launch_jk_dd(int cls, const KParams &kp, const ClassWork *w, int nw, const dd *D, double *Jh, double *Kh,
                          cudaStream_t st) {
   if (nw > 0 && w[0].wide) return launch_jk_dd_wide(cls, kp, w, nw, D, Jh, Kh, st);

@@ -1,7 +1,7 @@
 // jk_dd_wide.cu -- double-float J/K kernels with tdd_wide lanes per quartet
-// (classes.h): the accurate tier of the SF_PREC_MIXED_DF mode, whose few long
-// quartets run latency-bound with the FP64 lane count.  Its own translation
-// unit so that the build compiles it beside jk_dd.cu.
+// (classes.h): builds too small to fill the GPU, whose long quartets run
+// latency-bound with the FP64 lane count.  Its own translation unit so that
+// the build compiles it beside jk_dd.cu.
 #include "classes.h"
 #include "launch.h"
 
