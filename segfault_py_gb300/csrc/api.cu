@@ -618,11 +618,7 @@ inline int kind_lanes(const ClassInfo &ci, int kind, int wide) {
   return kind == 1 ? ci.t32 : (kind == 2 && wide) ? tdd_wide(ci.la, ci.lb, ci.lc, ci.ld, ci.t64) : ci.t64;
 }
 
-int build_work(sf_handle *h, int prec, double cut, double cut32) {
-  if (h->c_prec == prec && h->c_cut == cut && h->c_cut32 == cut32 && h->c_part == h->part &&
-      h->c_nparts == h->nparts)
-    return SF_OK;
-  h->slices.clear();
+int cut_lists(sf_handle *h, int prec, double cut, double cut32) {
   std::vector<int2> all;
   struct Pending {
     int cls, prec;
@@ -991,6 +987,30 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     SF_CK(h->d_dem.alloc(all.size()));
     SF_CK(h->d_cnt.alloc(4 * std::max<size_t>(h->slices.size(), 1)));
     SF_CK(h->d_dmax.alloc((size_t)h->nshell * h->nshell));
+  }
+  return SF_OK;
+}
+
+// The lists of this mode, cut if the handle holds others.  A cut that fails (out of
+// memory) leaves none behind: half of them under the old key would be taken for the
+// old mode's by its next call.
+int build_work(sf_handle *h, int prec, double cut, double cut32) {
+  if (h->c_prec == prec && h->c_cut == cut && h->c_cut32 == cut32 && h->c_part == h->part &&
+      h->c_nparts == h->nparts)
+    return SF_OK;
+  auto clear = [h] {
+    h->c_prec = -1;
+    h->slices.clear();
+    h->slice_stream.clear();
+    h->plan.clear();     // refers to the slices
+    h->groups.clear();
+    h->pplan.clear();
+  };
+  clear();
+  const int rc = cut_lists(h, prec, cut, cut32);
+  if (rc) {
+    clear();
+    return rc;
   }
   ++h->lists_version;
   h->c_prec = prec;
