@@ -415,6 +415,7 @@ struct sf_handle {
   int n_hi = kHiStreams, n_lo = kSideStreams - kHiStreams;
   cudaStream_t side[kSideStreams] = {};
   cudaEvent_t fork_ev = nullptr, join_ev[kSideStreams] = {};
+  bool in_flight = false;          // launches since the last drain()
   cudaStream_t one_st = nullptr;   // sf_grad_rhf's one-electron kernel
   cudaEvent_t one_ev = nullptr;
   std::vector<int> slice_stream;   // side stream of each slice (greedy by cost)
@@ -991,10 +992,28 @@ int cut_lists(sf_handle *h, int prec, double cut, double cut32) {
   return SF_OK;
 }
 
+// Wait until no launch of an earlier call reads the handle's tables any more, before
+// they are overwritten: calls return before their kernels end, and a copy from host
+// memory goes to the legacy stream, which the non-blocking side streams (and a
+// caller's) do not wait for.  A stream that is being captured runs nothing.
+int drain(sf_handle *h, cudaStream_t st) {
+  if (!h->in_flight) return SF_OK;
+  auto wait = [](cudaStream_t s) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(s, &c);
+    return e != cudaSuccess || c != cudaStreamCaptureStatusNone ? e : cudaStreamSynchronize(s);
+  };
+  for (cudaStream_t s : h->side) SF_CK(wait(s));
+  SF_CK(wait(h->one_st));
+  SF_CK(wait(st));
+  h->in_flight = false;
+  return SF_OK;
+}
+
 // The lists of this mode, cut if the handle holds others.  A cut that fails (out of
 // memory) leaves none behind: half of them under the old key would be taken for the
 // old mode's by its next call.
-int build_work(sf_handle *h, int prec, double cut, double cut32) {
+int build_work(sf_handle *h, int prec, double cut, double cut32, cudaStream_t st) {
   if (h->c_prec == prec && h->c_cut == cut && h->c_cut32 == cut32 && h->c_part == h->part &&
       h->c_nparts == h->nparts)
     return SF_OK;
@@ -1007,7 +1026,8 @@ int build_work(sf_handle *h, int prec, double cut, double cut32) {
     h->pplan.clear();
   };
   clear();
-  const int rc = cut_lists(h, prec, cut, cut32);
+  int rc = drain(h, st);
+  if (!rc) rc = cut_lists(h, prec, cut, cut32);
   if (rc) {
     clear();
     return rc;
@@ -1208,6 +1228,7 @@ void make_groups(sf_handle *h) {
 // joined back into st).
 template <typename F>
 int fan_out_list(sf_handle *h, cudaStream_t st, const std::vector<int> &stream_of, F &&fn) {
+  h->in_flight = true;
   SF_CK(cudaEventRecord(h->fork_ev, st));
   bool used[sf_handle::kSideStreams] = {false};
   for (int j : stream_of) used[j] = true;
@@ -1255,6 +1276,7 @@ cudaError_t launch_one(sf_handle *h, int cls, int kind, const ClassWork *w, int 
 // profiling 2: the launches are serialised on st, each between two events.
 int run_plan(sf_handle *h, bool grad, const double *D, const float *D32, const float *Ddd, double *Jh, double *Kh,
              double *g, cudaStream_t st, int profiling, int *launches) {
+  h->in_flight = true;
   if (profiling == 2) {
     for (size_t k = 0; k < h->plan.size(); ++k) {
       SF_CK(cudaEventRecord(h->ev[2 * k], st));
@@ -1263,7 +1285,8 @@ int run_plan(sf_handle *h, bool grad, const double *D, const float *D32, const f
       SF_CK(cudaEventRecord(h->ev[2 * k + 1], st));
       if (launches) ++*launches;
     }
-    return SF_OK;
+    // drain() knows the handle's own streams: one of them follows the last launch
+    return fan_out_list(h, st, {0}, [](size_t, cudaStream_t) { return cudaSuccess; });
   }
   SF_CK(cudaEventRecord(h->fork_ev, st));
   bool used[sf_handle::kSideStreams] = {false};
@@ -1902,7 +1925,8 @@ int sf_schwarz(sf_handle *h, double *q_out, void *stream) {
     std::copy(n.begin(), n.end(), h->pnp.begin() + s0);
     std::copy(qq.begin(), qq.end(), h->pq.begin() + s0);
   }
-  int rc = upload_pairs(h);
+  int rc = drain(h, st);
+  if (!rc) rc = upload_pairs(h);
   if (rc) return rc;
   h->have_schwarz = true;
   h->c_prec = -1;   // invalidate quartet lists
@@ -1955,7 +1979,7 @@ int sf_fock_jk(sf_handle *h, const double *D, double *J, double *K, int32_t prec
   if (!h->have_schwarz) return fail(SF_ESTATE, "sf_fock_jk: call sf_schwarz first");
   DeviceGuard g(h->device);
   cudaStream_t st = (cudaStream_t)stream;
-  int rc = build_work(h, precision, cutoff, fp32_cutoff);
+  int rc = build_work(h, precision, cutoff, fp32_cutoff, st);
   if (rc) return rc;
   const int n = h->nao;
   const size_t nn = (size_t)n * n;
@@ -2059,7 +2083,7 @@ int sf_autotune(sf_handle *h, const double *D, int32_t precision, double cutoff,
   if (!h->have_schwarz) return fail(SF_ESTATE, "sf_autotune: call sf_schwarz first");
   DeviceGuard g(h->device);
   cudaStream_t st = (cudaStream_t)stream;
-  int rc = build_work(h, precision, cutoff, fp32_cutoff);
+  int rc = build_work(h, precision, cutoff, fp32_cutoff, st);
   if (rc) return rc;
   rc = prepare_build(h, D, nullptr, nullptr, h->d_D32.p, h->d_Ddd.p, st, nullptr);
   if (rc) return rc;
@@ -2086,7 +2110,7 @@ int sf_autotune(sf_handle *h, const double *D, int32_t precision, double cutoff,
   };
   // whole-build time of the current lists, launches concurrent as in a build
   auto time_build = [&](float *ms) -> int {
-    int r2 = build_work(h, precision, cutoff, fp32_cutoff);
+    int r2 = build_work(h, precision, cutoff, fp32_cutoff, st);
     if (r2) return r2;
     r2 = run_call(h, false, D, h->d_D32.p, h->d_Ddd.p, h->d_Jh.p, h->d_Kh.p, nullptr, cutoff, fp32_cutoff, st, 0,
                   nullptr);   // warm-up
@@ -2162,7 +2186,7 @@ int sf_autotune(sf_handle *h, const double *D, int32_t precision, double cutoff,
     h->fill_acc_x4[precision] = best_acc;
   }
   h->c_prec = -1;
-  rc = build_work(h, precision, cutoff, fp32_cutoff);
+  rc = build_work(h, precision, cutoff, fp32_cutoff, st);
   if (rc) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -2322,7 +2346,7 @@ int sf_grad_jk(sf_handle *h, const double *D, double *grad, int32_t precision, d
   if (!h->have_schwarz) return fail(SF_ESTATE, "sf_grad_jk: call sf_schwarz first");
   DeviceGuard g(h->device);
   cudaStream_t st = (cudaStream_t)stream;
-  int rc = build_work(h, precision, cutoff, fp32_cutoff);
+  int rc = build_work(h, precision, cutoff, fp32_cutoff, st);
   if (rc) return rc;
   rc = prepare_build(h, D, nullptr, nullptr, h->d_D32.p, h->d_Ddd.p, st, nullptr);
   if (rc) return rc;

@@ -35,3 +35,37 @@ def test_lists_of_a_failed_build_are_not_kept(fake):
         assert [(r.cls, r.kind, r.n, r.split) for r in fake.launches()] == good
     assert failed > 0
     fake.L.sf_destroy(h)
+
+
+@pytest.mark.parametrize("profiling", [0, 1, 2])
+@pytest.mark.parametrize("then", ["precision", "cutoff", "partition", "tuning", "schwarz", "forces"])
+def test_lists_in_use_are_not_overwritten(fake, then, profiling):
+    """Calls return before their kernels end: lists (and pair tables) that launched kernels read are overwritten
+    only after a wait for the streams those run on.  The copies do not order themselves behind such streams."""
+    h = fake.handle(_table())
+    fake.ok(fake.L.sf_set_profiling(h, profiling))
+    fake.ok(fake.fock(h, "fp64"))
+    first = fake.log()
+    assert not [r for r in first if r.what == fake_cuda.SYNC]   # nothing to wait for
+    last = {r.stream: i for i, r in enumerate(first) if r.what == fake_cuda.LAUNCH}   # of each stream
+    fake.ok(fake.fock(h, "fp64"))   # the same lists: no copy, no wait
+    assert not [r for r in fake.log() if r.what in (fake_cuda.SYNC, fake_cuda.MEMCPY)]
+    if then == "partition":
+        fake.ok(fake.L.sf_set_partition(h, 0, 2))
+    if then == "tuning":
+        fake.ok(fake.L.sf_set_tuning(h, None, 0))
+    if then == "schwarz":
+        fake.ok(fake.L.sf_schwarz(h, None, 0x55))
+    elif then == "forces":
+        fake.ok(fake.forces(h, "df"))
+    else:
+        fake.ok(fake.fock(h, "df" if then == "precision" else "fp64", cut=1e-9 if then == "cutoff" else 1e-12))
+    log = fake.log()
+    copy = min(i for i, r in enumerate(log) if r.what == fake_cuda.MEMCPY and (then != "schwarz" or r.stream == 0))
+    waited = {r.stream for r in log[:copy] if r.what == fake_cuda.SYNC}
+    for i, r in enumerate(first):   # a stream waited for may itself have waited for another one's event
+        if r.what == fake_cuda.WAIT and r.stream in waited:
+            waited |= {e.stream for j, e in enumerate(first[:i]) if e.what == fake_cuda.RECORD and e.list == r.list
+                       and j > last.get(e.stream, -1)}
+    assert set(last) <= waited
+    fake.L.sf_destroy(h)
