@@ -36,7 +36,7 @@ __device__ __forceinline__ double boys_horner(const double *row, double s) {
 template <int M>
 __device__ __forceinline__ void boys_table(const double *tab, double T, double (&F)[M + 1]) {
   static_assert(M <= kBoysMax, "orders in the table");
-  if (T >= kTabXmax) {
+  if (!(T < kTabXmax)) {   // NaN too: it has no table row
     const double y = rsqrt_nr(T), h = 0.5 * y * y;
     F[0] = 0.886226925452758014 * y;   // sqrt(pi) / 2
 #pragma unroll

@@ -338,7 +338,7 @@ template <int N>
 __device__ __forceinline__ void rys_roots_f64_tab(const double *tab64, const RysAsym &asym, double x,
                                                   double (&u)[N], double (&w)[N]) {
   using R = double;
-  if (x >= (R)kTabXmax) {
+  if (!(x < (R)kTabXmax)) {   // NaN too: it has no table row
     const R ix = (R)1 / x, isx = rsqrt_nr(x);
 #pragma unroll
     for (int i = 0; i < N; ++i) {
@@ -412,7 +412,7 @@ __device__ __forceinline__ void rys_root_one(const KParams &kp, R x, int r, R &u
 template <int N>
 __device__ __forceinline__ void rys_root_one_f64(const KParams &kp, double x, int r, double &u, double &w) {
   using R = double;
-  if (x >= (R)kTabXmax) {
+  if (!(x < (R)kTabXmax)) {
     u = (R)kp.asym.r[N][r] / x;
     w = (R)kp.asym.w[N][r] * rsqrt_nr(x);
     return;
