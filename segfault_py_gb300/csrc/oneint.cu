@@ -187,7 +187,7 @@ __device__ __forceinline__ void one_pair(const OneParams &P, int pair, double *s
 #pragma unroll
       for (int k = 0; k < L; ++k) e *= x;
       const float f = 1.0f + 1.1284f * sqrtf(pf) * (float)zs + 3.0f * (float)be * (LB + 2);
-      if (!(g * e * f >= 1e-17f)) on = false;
+      if (g * e * f < 1e-17f) on = false;   // not on NaN: it has to reach the matrix it belongs to
     }
     if (!__any_sync(0xffffffffu, on)) continue;
     __syncwarp();   // the previous pass is done with E and St
@@ -413,7 +413,7 @@ __device__ __forceinline__ void one_pair_grad(const OneParams &P, const double *
 #pragma unroll
       for (int k = 0; k < L; ++k) e *= x;
       const float f = (2.0f * mx + L1) * (1.0f + 1.1284f * sqrtf(pf) * zs + 3.0f * mx * (LB + 2));
-      if (!(g * e * f >= 1e-15f)) on = false;
+      if (g * e * f < 1e-15f) on = false;   // not on NaN: it has to reach the forces
     }
     if (!__any_sync(0xffffffffu, on)) continue;
     __syncwarp();   // the previous pass is done with the tables

@@ -46,3 +46,16 @@ def test_position_of_a_nucleus(cuda):
     assert torch.isnan(V2).all()
     g = _forces(cuda, xyz, Z).view(7, 3)
     assert torch.isnan(g[:6]).all() and torch.isfinite(g[6]).all()   # the shells' centres are atoms 0 to 4
+
+
+def test_charge_of_a_nucleus(cuda):
+    """A charge that is not a number makes V and the forces that it enters not numbers; S and T do not depend on
+    charges."""
+    xyz, Z = _geometry()
+    S, T, _ = _one_electron(cuda, xyz, Z)
+    Z[5] = float("nan")
+    S2, T2, V2 = _one_electron(cuda, xyz, Z)
+    assert torch.equal(S, S2) and torch.equal(T, T2)
+    assert torch.isnan(V2).all()
+    g = _forces(cuda, xyz, Z).view(7, 3)
+    assert torch.isnan(g[:6]).all() and torch.isfinite(g[6]).all()
