@@ -50,9 +50,12 @@ extern "C" {
 #define SF_MAX_PRIM 16
 
 /* precision modes of sf_fock_jk / sf_eri_batch */
-#define SF_PREC_FP64 0      /* every quartet in FP64                          */
+#define SF_PREC_FP64 0      /* FP64; in classes with enough work, quartets whose
+                               Schwarz bound Q_ab Q_cd is below 2e-4 of the
+                               largest run in double-float (no larger errors
+                               of J and K, measured in api.cu)                */
 #define SF_PREC_FP32 1      /* every quartet in FP32 (FP64 accumulation)      */
-#define SF_PREC_MIXED 2     /* FP64 above the FP32 cutoff, FP32 below it      */
+#define SF_PREC_MIXED 2     /* as FP64 above the FP32 cutoff, FP32 below it   */
 #define SF_PREC_MIXED_DF 3  /* double-float (FP32 pairs, ~2^-44 relative) above
                                the FP32 cutoff, FP32 below it                 */
 #define SF_PREC_DF 4        /* every quartet in double-float                  */
@@ -78,7 +81,8 @@ typedef struct {
 
 /* counters of the last sf_fock_jk call */
 typedef struct {
-    int64_t quartets_fp64;        /* canonical shell quartets done in FP64     */
+    int64_t quartets_fp64;        /* canonical shell quartets of the accurate
+                                     tier (FP64, double-float or both)         */
     int64_t quartets_fp32;        /* ... in FP32                               */
     int64_t quartets_total;       /* canonical shell quartets before screening */
     int64_t prim_quartets_fp64;
@@ -120,8 +124,8 @@ int sf_schwarz(sf_handle *h, double *q_out, void *stream);
  *   J_pq = sum_rs (pq|rs) D_rs,  K_pq = sum_rs (pr|qs) D_rs
  * (the two einsums of src/hf/hf.py:300), over the canonical shell quartets
  * with Q_ab Q_cd >= cutoff.  In SF_PREC_MIXED and SF_PREC_MIXED_DF, quartets
- * with Q_ab Q_cd < fp32_cutoff are evaluated in FP32, the others in FP64
- * (MIXED) or double-float (MIXED_DF); J and K are accumulated in FP64 in
+ * with Q_ab Q_cd < fp32_cutoff are evaluated in FP32, the others as in SF_PREC_FP64
+ * (MIXED) or in double-float (MIXED_DF); J and K are accumulated in FP64 in
  * every mode.  sf_stats counts the FP64 / double-float tier as "fp64".
  * J, K: device, nao*nao, overwritten.
  * stats (optional, host) receives counters.  Does not synchronise unless

@@ -365,6 +365,8 @@ struct sf_handle {
   std::vector<int> pa, pb, ppoff, pnp, ppoff32f;
   int pair_full(int i) const { return nprim[pa[i]] * nprim[pb[i]]; }
   std::vector<double> pq;
+  double qmax = 0.0;          // largest Schwarz bound of a pair
+  bool dd_range = true;       // every primitive record well inside FP32's range
   std::vector<int> pairmap;   // a*nshell+b -> pair index (a,b canonical)
   DBuf<int> d_l, d_nprim, d_ao, d_atom, d_spoff;
   DBuf<double> d_cx, d_cy, d_cz, d_exps, d_coefs;
@@ -590,15 +592,22 @@ std::vector<int> lpt_streams(const std::vector<double> &cost_desc, int first = 0
 // number of primitive iterations; inside a cost bucket the (i, j) order of the
 // Schwarz-sorted pair lists is kept.  A partition (part, nparts) keeps every
 // nparts-th quartet of each sorted list, which balances cost across parts.
-// The FP64 kernels' quartets below this Schwarz bound run in double-float.  A
-// double-float quartet carries 2^-48 relative rounding instead of 2^-53, and a
-// quartet adds at most Q_ab Q_cd |D| to an element of J or K, so below 1e-3 of
-// the largest bounds (order one) its rounding lies under that of the large
-// quartets, which stay FP64: J and K of (H2O)16 6-31G* differ by 5e-15 of
-// their norm from the all-FP64 build, errors against 64-bit reference values are
-// the same to three digits; 68.0 -> 22.7 ms when it came, 19.2 with the kernels as
-// they are now (everything in FP64: the pipe 88 % busy).
-constexpr double kDDTail = 1e-3;
+// The FP64 kernels' quartets with a Schwarz bound below this fraction of the square of
+// the largest Q run in double-float.  A double-float quartet carries 2^-48 relative
+// rounding instead of 2^-53, but its tables are the finer ones, and a quartet adds at
+// most Q_ab Q_cd |D| to an element of J or K, so below 2e-4 of the largest bounds its
+// rounding lies under that of the large quartets, which stay FP64.  Largest error and
+// norm of the error, of the largest element and the norm, against 64-bit-mantissa
+// McMurchie-Davidson values with no screening, everything in FP64 / with this part:
+// J of (H2O)16 6-31G* 7.1e-15, 3.0e-15 / 4.4e-15, 2.1e-15, K 7.4e-15, 5.5e-15 /
+// 3.6e-15, 3.3e-15; J of hexane 8.3e-15, 3.9e-15 / 8.4e-15, 4.1e-15, K 9.1e-15,
+// 1.4e-14 / 4.7e-15, 1.2e-14.  (An element of two functions
+// far apart, below 1e-6 of the largest, keeps fewer relative digits.)  (H2O)16
+// FP64 58.1 -> 19.9 ms.
+constexpr double kDDTail = 2e-4;
+// ... and for a largest Q whose square lies in this range, so that no integral that
+// counts comes near the ends of FP32's range
+constexpr double kDDTailQ2[2] = {1e-12, 1e12};
 // ... when the class's part below it would hold the FP64 pipe for longer than
 // 20 us (estimated from its primitive quartets as in build_work at the measured
 // 1.25 TFLOP/s): a smaller one is hidden in the FP64 launch, and one more launch
@@ -620,6 +629,8 @@ inline int kind_lanes(const ClassInfo &ci, int kind, int wide) {
 }
 
 int cut_lists(sf_handle *h, int prec, double cut, double cut32) {
+  const double q2 = h->qmax * h->qmax;
+  const double tail_cut = h->dd_range && q2 >= kDDTailQ2[0] && q2 <= kDDTailQ2[1] ? kDDTail * q2 : 0.0;
   std::vector<int2> all;
   struct Pending {
     int cls, prec;
@@ -679,10 +690,10 @@ int cut_lists(sf_handle *h, int prec, double cut, double cut32) {
     const double nabcd = (double)ncart(ci.la) * ncart(ci.lb) * ncart(ci.lc) * ncart(ci.ld);
     // launch kind of tier pr: 0 FP64, 1 FP32, 2 double-float
     const int hi_kind = (prec == SF_PREC_MIXED_DF || prec == SF_PREC_DF) ? 2 : 0;
-    if (hi_kind == 0 && prec != SF_PREC_FP32) {
+    if (hi_kind == 0 && prec != SF_PREC_FP32 && tail_cut > 0.0) {
       double tail = 0.0;
       for (int i = 0; i < nX; ++i) {
-        mdd[i] = std::min<int64_t>(m64[i], count_pass(qy, nY, qx[i], std::max(kDDTail, cut)));
+        mdd[i] = std::min<int64_t>(m64[i], count_pass(qy, nY, qx[i], std::max(tail_cut, cut)));
         int64_t k = 0;
         for (int64_t j = mdd[i]; j < m64[i]; ++j) k += h->pnp[y0 + j];
         tail += (double)k * h->pnp[x0 + i];
@@ -1723,6 +1734,11 @@ int sf_create(const sf_shell_desc *shells, int32_t nshell, sf_handle **out) {
     }
   }
   h->cstart[kNumPairClass] = (int)h->pa.size();
+  // sums and products of two records stay inside FP32's range with these
+  for (double v : h->exps) h->dd_range &= v >= 1e-9 && v <= 1e9;
+  for (const auto *c : {&h->cx, &h->cy, &h->cz})
+    for (double v : *c) h->dd_range &= std::fabs(v) <= 1e6;
+  for (size_t i = 0; i < rec.size(); i += kPrimRec) h->dd_range &= std::fabs(rec[i + 4]) <= 1e12;
   {
     SF_CK(h->d_pp64.upload(rec));
     // FP32: the kept records at the same offsets, then the full lists
@@ -1902,6 +1918,7 @@ int sf_schwarz(sf_handle *h, double *q_out, void *stream) {
   SF_CK(cudaStreamSynchronize(st));
   for (double v : q)
     if (!std::isfinite(v)) return fail(SF_EINVAL, "sf_schwarz: non-finite Schwarz bound (bad basis data?)");
+  h->qmax = q.empty() ? 0.0 : *std::max_element(q.begin(), q.end());
   // sort every pair class by Q descending (stable)
   for (int pc = 0; pc < kNumPairClass; ++pc) {
     const int s0 = h->cstart[pc], s1 = h->cstart[pc + 1];

@@ -69,3 +69,31 @@ def test_lists_in_use_are_not_overwritten(fake, then, profiling):
                        and j > last.get(e.stream, -1)}
     assert set(last) <= waited
     fake.L.sf_destroy(h)
+
+
+def _kinds(fake, table, scale=1.0, cut=1e-12):
+    h = fake.handle(table, q_scale=scale)
+    fake.ok(fake.fock(h, "fp64", cut=cut * scale * scale))
+    n = {}
+    for r in fake.launches():
+        n[r.cls, r.kind] = n.get((r.cls, r.kind), 0) + r.n
+    fake.L.sf_destroy(h)
+    return n
+
+
+def test_double_float_part_follows_the_largest_bound(fake):
+    """The FP64 mode's double-float part is what is small against the molecule's own largest quartets: scaling every
+    function moves no quartet, and bounds or primitives outside FP32's range leave everything in FP64."""
+    table = _table(6)
+    ref = _kinds(fake, table)
+    assert {k for _, k in ref} == {0, 2}
+    for s in (2.0 ** -10, 2.0 ** -3, 2.0 ** 4):
+        assert _kinds(fake, table, s) == ref
+    for s in (2.0 ** -40, 2.0 ** 40):
+        assert {k for _, k in _kinds(fake, table, s)} == {0}
+    for key, v in (("exps", 1e30), ("exps", 1e-30), ("coefs", 1e25)):
+        t = dict(table, **{key: table[key].copy()})
+        t[key][3] = v
+        assert {k for _, k in _kinds(fake, t)} == {0}, key
+    # no quartet of 2e-4 of the largest bound (1 here) or more is in it
+    assert {k for _, k in _kinds(fake, table, cut=2e-4)} == {0}
