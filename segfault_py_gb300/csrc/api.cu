@@ -1219,7 +1219,11 @@ void make_groups(sf_handle *h) {
       g = &h->groups.back();
     }
     g->w.push_back(L.w);
-    if (!L.demoted) g->est += sl.est;
+    // how many quartets are demoted is known on the device only: at most all of
+    // them, at FP32 cost (the ratios of cut_lists' estimate).  With no estimate they
+    // all went to the same stream: forces of (H2O)8 6-31G* FP32 + double-float 4.57 ->
+    // 4.22 ms, (H2O)2 0.70 -> 0.57, (H2O)4 FP32 + FP64 1.96 -> 1.74
+    g->est += !L.demoted ? sl.est : sl.est / (sl.prec == 0 ? 16.0 : 5.0);
   }
   for (auto &g : h->groups)
     std::stable_sort(g.w.begin(), g.w.end(), [](const ClassWork &a, const ClassWork &b) { return a.max_cost > b.max_cost; });

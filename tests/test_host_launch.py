@@ -97,3 +97,20 @@ def test_double_float_part_follows_the_largest_bound(fake):
         assert {k for _, k in _kinds(fake, t)} == {0}, key
     # no quartet of 2e-4 of the largest bound (1 here) or more is in it
     assert {k for _, k in _kinds(fake, table, cut=2e-4)} == {0}
+
+
+@pytest.mark.parametrize("precision,waters", [("mixed", 3), ("mixed_df", 3), ("mixed_df", 8)])
+def test_demoted_launches_share_the_streams(fake, precision, waters):
+    """The FP32 launches of demoted quartets are spread over the FP32 streams, by estimated cost: more of them than
+    streams, they use at least half of the streams."""
+    h = fake.handle(_table(waters))
+    fake.ok(fake.forces(h, precision, cut32=1e-2))
+    runs = {}
+    for r in fake.launches():
+        runs.setdefault((r.stream, r.cls, r.kind, r.count % 32), 0)   # the counts of a slice: kept, demoted, ...
+    base = min(c for _, _, k, c in runs if k != 1)
+    demoted = [s for s, _, k, c in runs if k == 1 and c == (base + 8) % 32]
+    low = {s for s, _, k, _ in runs if k == 1}
+    assert len(demoted) > len(low) > 1
+    assert 2 * len(set(demoted)) >= len(low)
+    fake.L.sf_destroy(h)
