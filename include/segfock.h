@@ -53,7 +53,8 @@ extern "C" {
 #define SF_PREC_FP64 0      /* FP64; in classes with enough work, quartets whose
                                Schwarz bound Q_ab Q_cd is below 2e-4 of the
                                largest run in double-float (no larger errors
-                               of J and K, measured in api.cu)                */
+                               of J and K, measured in api.cu), in gradients
+                               those whose derivatives are below it too       */
 #define SF_PREC_FP32 1      /* every quartet in FP32 (FP64 accumulation)      */
 #define SF_PREC_MIXED 2     /* as FP64 above the FP32 cutoff, FP32 below it   */
 #define SF_PREC_MIXED_DF 3  /* double-float (FP32 pairs, ~2^-44 relative) above

@@ -213,7 +213,10 @@ __global__ void prepare_kernel(const double *D, double *Jh, double *Kh, float *D
 //    one of the accurate tier runs in FP32 when
 //    Q_ab Q_cd G (s_a + s_b + s_c + s_d), s = sqrt of the shell's largest
 //    exponent, is below the accurate cutoff: quartets of tight core shells
-//    stay accurate.
+//    stay accurate;
+//  * gradient without an FP32 tier: a quartet of an FP64 tier's double-float part
+//    (kDDTail) stays there only while the bound times that factor is below t_tail
+//    times the square of the largest |D|; the others run in FP64.
 // Every list is compacted into a "kept" and a "demoted" list at the same
 // offsets (d_keep, d_dem), with device counts read by the kernels, so nothing
 // synchronises with the host.  Chunks of 1024 entries take their place in the
@@ -223,7 +226,7 @@ __global__ void prepare_kernel(const double *D, double *Jh, double *Kh, float *D
 struct ClassifySlice {
   int64_t off, n;        // offset in the quartet-list buffer, length
   int x0, y0;            // first global pair of the bra / ket pair class
-  int acc;               // accurate tier (FP64 or double-float launch)
+  int acc;               // accurate tier (FP64 or double-float launch); 2: the double-float part of FP64
   int pad;
 };
 constexpr int kClsThreads = 256, kClsPer = 4, kClsChunk = kClsThreads * kClsPer;
@@ -232,24 +235,40 @@ constexpr int kClsThreads = 256, kClsPer = 4, kClsChunk = kClsThreads * kClsPer;
 // gives 6.9e-8 / 4.5e-7 Eh/bohr, 1e-3 1.4e-7 / 1.05e-6, 1e-2 1.4e-6 / 9.8e-6
 // (the FP32 tier alone leaves 7e-8 / 3e-7)
 constexpr double kGradFp32Scale = 3e-2;
+// and the largest |D| for which a part of an FP64 gradient runs in double-float (what D
+// D times an integral may reach and keep a float pair's 48 bits)
+constexpr float kGradDDTailDMin = 1e-10f, kGradDDTailDMax = 1e10f;
 
-// M_xy = max |D| over the Cartesian block of shells x, y (FP32 is enough for a bound)
-__global__ void shell_dmax_kernel(const double *D, int n, const int *l, const int *ao, int ns, float *dm) {
+// M_xy = max |D| over the Cartesian block of shells x, y (FP32 is enough for a bound);
+// the largest of them to *top (zeroed before; as bits, whose order is that of the
+// values; not a number is above all)
+__global__ void shell_dmax_kernel(const double *D, int n, const int *l, const int *ao, int ns, float *dm,
+                                  unsigned *top) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= ns * ns) return;
-  const int a = idx / ns, b = idx % ns;
-  const int la = l[a], lb = l[b], a0 = ao[a], b0 = ao[b];
-  const int na = (la + 1) * (la + 2) / 2, nb = (lb + 1) * (lb + 2) / 2;
-  double m = 0.0;
-  for (int i = 0; i < na; ++i)
-    for (int j = 0; j < nb; ++j) m = fmax(m, fabs(D[(int64_t)(a0 + i) * n + b0 + j]));
-  dm[idx] = (float)m;
+  unsigned bits = 0;
+  if (idx < ns * ns) {
+    const int a = idx / ns, b = idx % ns;
+    const int la = l[a], lb = l[b], a0 = ao[a], b0 = ao[b];
+    const int na = (la + 1) * (la + 2) / 2, nb = (lb + 1) * (lb + 2) / 2;
+    double m = 0.0;
+    bool nan = false;
+    for (int i = 0; i < na; ++i)
+      for (int j = 0; j < nb; ++j) {
+        const double d = fabs(D[(int64_t)(a0 + i) * n + b0 + j]);
+        m = fmax(m, d);
+        nan |= d != d;
+      }
+    dm[idx] = (float)m;
+    bits = nan ? 0x7fffffffu : __float_as_uint((float)m);
+  }
+  bits = __reduce_max_sync(0xffffffffu, bits);
+  if ((threadIdx.x & 31) == 0) atomicMax(top, bits);
 }
 
 __global__ void __launch_bounds__(kClsThreads) classify_kernel(
     const int2 *list, const ClassifySlice *sl, const int2 *blk, const int *pa, const int *pb, const int *pnp,
     const double *pq, const float *dm, const float *sqa, int ns, int grad_mode, double t_drop, double t_acc,
-    int2 *keep, int2 *dem, unsigned long long *cnt, int2 *chunks, int pass) {
+    double t_tail, const unsigned *top, int2 *keep, int2 *dem, unsigned long long *cnt, int2 *chunks, int pass) {
   // pass 0: places by atomics; 1: this chunk's counts to chunks[]; 2: places from them
   const int2 bk = blk[blockIdx.x];
   const ClassifySlice S = sl[bk.x];
@@ -258,6 +277,12 @@ __global__ void __launch_bounds__(kClsThreads) classify_kernel(
   int where[kClsPer];   // 0 kept, 1 demoted, 2 left out
   int nk = 0, nd = 0;
   unsigned long long pk = 0, pd = 0;
+  const bool split_tail = S.acc == 2 && t_tail >= 0.0;
+  double tail = -1.0;   // bounds from here on (all for a density outside the range) in FP64
+  if (split_tail) {
+    const float m = __uint_as_float(*top);
+    if (m >= kGradDDTailDMin && m <= kGradDDTailDMax) tail = t_tail * m * m;
+  }
 #pragma unroll
   for (int k = 0; k < kClsPer; ++k) {
     where[k] = 2;
@@ -277,7 +302,7 @@ __global__ void __launch_bounds__(kClsThreads) classify_kernel(
       bound = q * (double)fmaxf(2.0f * fmaxf(mab, mcd), fmaxf(fmaxf(mac, mbd), fmaxf(mad, mbc)));
       bound_acc = bound;
     }
-    where[k] = bound < t_drop ? 2 : (S.acc && bound_acc < t_acc) ? 1 : 0;
+    where[k] = bound < t_drop ? 2 : split_tail ? !(bound_acc < tail) : (S.acc && bound_acc < t_acc) ? 1 : 0;
     const unsigned long long c0 = (unsigned long long)pnp[pab] * (unsigned long long)pnp[pcd];
     if (where[k] == 0) { ++nk; pk += c0; }
     if (where[k] == 1) { ++nd; pd += c0; }
@@ -442,7 +467,8 @@ struct sf_handle {
   DBuf<float> d_dmax;                      // nshell^2 block maxima of |D|
   DBuf<float> d_sqa;                       // per shell: sqrt of its largest primitive exponent
   DBuf<int2> d_keep, d_dem;                // compacted lists at the offsets of d_list
-  DBuf<unsigned long long> d_cnt;          // per slice: kept, demoted quartets; kept, demoted primitive quartets
+  // per slice: kept, demoted quartets; kept, demoted primitive quartets; then the largest |D| (shell_dmax_kernel)
+  DBuf<unsigned long long> d_cnt;
   DBuf<ClassifySlice> d_csl;
   DBuf<int2> d_blk_acc, d_blk_all;         // classification CTAs (slice, chunk): accurate-tier slices / all
   DBuf<int2> d_chunks;                     // kept and demoted quartets of each accurate-tier chunk
@@ -592,6 +618,7 @@ std::vector<int> lpt_streams(const std::vector<double> &cost_desc, int first = 0
 // number of primitive iterations; inside a cost bucket the (i, j) order of the
 // Schwarz-sorted pair lists is kept.  A partition (part, nparts) keeps every
 // nparts-th quartet of each sorted list, which balances cost across parts.
+
 // The FP64 kernels' quartets with a Schwarz bound below this fraction of the square of
 // the largest Q run in double-float.  A double-float quartet carries 2^-48 relative
 // rounding instead of 2^-53, but its tables are the finer ones, and a quartet adds at
@@ -600,10 +627,18 @@ std::vector<int> lpt_streams(const std::vector<double> &cost_desc, int first = 0
 // norm of the error, of the largest element and the norm, against 64-bit-mantissa
 // McMurchie-Davidson values with no screening, everything in FP64 / with this part:
 // J of (H2O)16 6-31G* 7.1e-15, 3.0e-15 / 4.4e-15, 2.1e-15, K 7.4e-15, 5.5e-15 /
-// 3.6e-15, 3.3e-15; J of hexane 8.3e-15, 3.9e-15 / 8.4e-15, 4.1e-15, K 9.1e-15,
-// 1.4e-14 / 4.7e-15, 1.2e-14.  (An element of two functions
+// 3.6e-15, 3.3e-15; J of hexane 8.3e-15, 3.9e-15 / 9.9e-15, 3.8e-15, K 9.1e-15,
+// 1.4e-14 / 5.0e-15, 1.2e-14 (the largest errors vary by a fifth from run to run).  (An element of two functions
 // far apart, below 1e-6 of the largest, keeps fewer relative digits.)  (H2O)16
 // FP64 58.1 -> 19.9 ms.
+// Gradients: the derivatives of a quartet outgrow its bound by about the square roots of
+// its exponents (classify_kernel), so bounds with that factor, weighted by the density,
+// decide, against the same threshold.  Largest error of the forces against 64-bit-mantissa
+// values, no screening, everything in FP64 / with the whole part / with what is sorted
+// out: butane 6-31G** 1.3-1.5e-12 / 2.2e-12 / 1.2-2.1e-12, (H2O)8 6-31G* 2.4-3.6e-13 /
+// 5.8e-13 / 3.8-4.4e-13 (ranges over runs of the same build).  FP64 forces of (H2O)4
+// 6-31G* 3.88 -> 4.06 ms, pentane 6-31G** 20.1 -> 20.7, (H2O)8 14.4 against 24.9
+// with everything in FP64; ten or a hundred times the threshold takes as long.
 constexpr double kDDTail = 2e-4;
 // ... and for a largest Q whose square lies in this range, so that no integral that
 // counts comes near the ends of FP32's range
@@ -983,7 +1018,8 @@ int cut_lists(sf_handle *h, int prec, double cut, double cut32) {
     std::vector<int2> ba, bl;
     for (size_t k = 0; k < h->slices.size(); ++k) {
       const auto &sl = h->slices[k];
-      csl[k] = ClassifySlice{(int64_t)(sl.w.list - h->d_list.p), sl.w.n, sl.w.x0, sl.w.y0, sl.prec != 1 ? 1 : 0, 0};
+      csl[k] = ClassifySlice{(int64_t)(sl.w.list - h->d_list.p), sl.w.n, sl.w.x0, sl.w.y0,
+                             sl.prec == 1 ? 0 : sl.tail ? 2 : 1, 0};
       for (int64_t c = 0; c * kClsChunk < sl.w.n; ++c) {
         bl.push_back(make_int2((int)k, (int)c));
         if (sl.prec != 1) ba.push_back(make_int2((int)k, (int)c));
@@ -997,7 +1033,7 @@ int cut_lists(sf_handle *h, int prec, double cut, double cut32) {
     SF_CK(h->d_chunks.alloc(ba.size()));
     SF_CK(h->d_keep.alloc(all.size()));
     SF_CK(h->d_dem.alloc(all.size()));
-    SF_CK(h->d_cnt.alloc(4 * std::max<size_t>(h->slices.size(), 1)));
+    SF_CK(h->d_cnt.alloc(4 * h->slices.size() + 1));
     SF_CK(h->d_dmax.alloc((size_t)h->nshell * h->nshell));
   }
   return SF_OK;
@@ -1071,18 +1107,20 @@ int density_classify(sf_handle *h, const double *D, bool grad, double cut, doubl
                        : grad ? (h->dens_grad_acc >= 0.0 ? h->dens_grad_acc : cut32 * kGradFp32Scale)
                               : (h->dens_fock_acc >= 0.0 ? h->dens_fock_acc : cut32);
   const double t_drop = grad ? (h->dens_grad_drop >= 0.0 ? h->dens_grad_drop : cut) : -1.0;
+  const double t_tail = grad && !mixed ? kDDTail * h->qmax * h->qmax : -1.0;
   const int nb = grad ? h->nblk_all : h->nblk_acc;
   const int ns = h->nshell;
-  SF_CK(cudaMemsetAsync(h->d_cnt.p, 0, 4 * h->slices.size() * sizeof(unsigned long long), st));
+  unsigned *top = reinterpret_cast<unsigned *>(h->d_cnt.p + 4 * h->slices.size());
+  SF_CK(cudaMemsetAsync(h->d_cnt.p, 0, (4 * h->slices.size() + 1) * sizeof(unsigned long long), st));
   shell_dmax_kernel<<<(unsigned)((ns * ns + 255) / 256), 256, 0, st>>>(D, h->nao, h->d_l.p, h->d_ao.p, ns,
-                                                                       h->d_dmax.p);
+                                                                       h->d_dmax.p, top);
   SF_CK(cudaGetLastError());
   if (nb > 0) {
     for (int pass = grad ? 0 : 1; pass <= (grad ? 0 : 2); ++pass) {
       classify_kernel<<<(unsigned)nb, kClsThreads, 0, st>>>(
           h->d_list.p, h->d_csl.p, grad ? h->d_blk_all.p : h->d_blk_acc.p, h->d_pa.p, h->d_pb.p, h->d_pfull.p,
-          h->d_pq.p, h->d_dmax.p, h->d_sqa.p, ns, grad ? 1 : 0, t_drop, t_acc, h->d_keep.p, h->d_dem.p, h->d_cnt.p,
-          h->d_chunks.p, pass);
+          h->d_pq.p, h->d_dmax.p, h->d_sqa.p, ns, grad ? 1 : 0, t_drop, t_acc, t_tail, top, h->d_keep.p, h->d_dem.p,
+          h->d_cnt.p, h->d_chunks.p, pass);
       SF_CK(cudaGetLastError());
     }
   }
@@ -1145,9 +1183,10 @@ int build_persist(sf_handle *h) {
 }
 
 // The launches of one call: one per slice (reading its compacted list when
-// the classification ran for it) and, for a classified accurate-tier slice of
-// a mixed mode, one FP32 launch of its demoted quartets on the next FP32
-// stream.  In the persistent launch mode (Fock builds, profiling off) the
+// the classification ran for it), for a classified accurate-tier slice of
+// a mixed mode one FP32 launch of its demoted quartets on the next FP32
+// stream, and for the double-float part of an FP64 gradient one FP64 launch of
+// the quartets that the classification took out of it.  In the persistent launch mode (Fock builds, profiling off) the
 // slices of the register tiers are marked covered and one launch per tier
 // runs them, on the FP32 streams.
 int make_plan(sf_handle *h, bool grad, int active) {
@@ -1168,12 +1207,21 @@ int make_plan(sf_handle *h, bool grad, int active) {
     const auto &sl = h->slices[k];
     const bool cl = active && (grad || sl.prec != 1);
     const int64_t off = sl.w.list - h->d_list.p;
-    sf_handle::Launch L{(int)k, sl.prec, h->slice_stream[k], 0, sl.w};
+    // a gradient runs an FP64 tier's double-float part in FP64 where nothing sorts
+    // out the quartets whose derivatives are large (kDDTail)
+    const bool split_tail = grad && sl.tail && active && !mixed;
+    sf_handle::Launch L{(int)k, grad && sl.tail && !split_tail ? 0 : sl.prec, h->slice_stream[k], 0, sl.w};
     if (cl) {
       L.w.list = h->d_keep.p + off;
       L.w.count = h->d_cnt.p + 4 * k;
     }
     h->plan.push_back(L);
+    if (split_tail) {
+      sf_handle::Launch P{(int)k, 0, h->slice_stream[k], 1, sl.w};
+      P.w.list = h->d_dem.p + off;
+      P.w.count = h->d_cnt.p + 4 * k + 1;
+      h->plan.push_back(P);
+    }
     if (cl && mixed && sl.prec != 1) {
       sf_handle::Launch Dm{(int)k, 1, sf_handle::kHiStreams + rr, 1, sl.w};
       rr = (rr + 1) % h->n_lo;
@@ -1222,8 +1270,9 @@ void make_groups(sf_handle *h) {
     // how many quartets are demoted is known on the device only: at most all of
     // them, at FP32 cost (the ratios of cut_lists' estimate).  With no estimate they
     // all went to the same stream: forces of (H2O)8 6-31G* FP32 + double-float 4.57 ->
-    // 4.22 ms, (H2O)2 0.70 -> 0.57, (H2O)4 FP32 + FP64 1.96 -> 1.74
-    g->est += !L.demoted ? sl.est : sl.est / (sl.prec == 0 ? 16.0 : 5.0);
+    // 4.22 ms, (H2O)2 0.70 -> 0.57, (H2O)4 FP32 + FP64 1.96 -> 1.74.  (FP64 quartets
+    // out of a double-float part: a fifth of it, at FP64 cost.)
+    g->est += !L.demoted ? sl.est : L.kind == 0 ? 0.2 * 16.0 / 5.0 * sl.est : sl.est / (sl.prec == 0 ? 16.0 : 5.0);
   }
   for (auto &g : h->groups)
     std::stable_sort(g.w.begin(), g.w.end(), [](const ClassWork &a, const ClassWork &b) { return a.max_cost > b.max_cost; });

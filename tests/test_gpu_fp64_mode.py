@@ -1,0 +1,88 @@
+"""What the FP64 mode runs in double-float."""
+import numpy as np
+import pytest
+import torch
+
+from test_gpu_kernel_edges import _sym
+
+pytestmark = pytest.mark.gpu
+
+CUT, TAIL = 1e-9, 2e-4
+
+
+@pytest.fixture(scope="module")
+def water(cuda):
+    from segfault_py_gb300 import geometry as G
+    from segfault_py_gb300.fock import FockBuilder
+    from segfault_py_gb300.molecule import Molecule
+    mol = Molecule.from_geometry(*G.water_cluster(5, seed=4), "6-31g*")
+    fb = FockBuilder(mol, device=cuda, cutoff=CUT, precision="fp64")
+    fb.set_density_screening(grad=True, grad_drop_cutoff=0.0)
+    yield fb, torch.tensor(_sym(mol.nao, 5), device=cuda)
+    fb.close()
+
+
+def _forces(fb, D):
+    """The two-electron forces and (class, kind) -> quartets of the launches."""
+    from segfault_py_gb300 import _lib
+    from segfault_py_gb300.fock import _ptr, _stream_ptr
+    g = torch.zeros(3 * fb.mol.natom, dtype=torch.float64, device=D.device)
+    _lib.check(_lib.lib().sf_grad_jk(fb.handle, _ptr(D), _ptr(g), _lib.PRECISION["fp64"], CUT, 0.0, _stream_ptr()))
+    n = {}
+    for s in fb.slice_info():
+        n[s["cls"], s["precision"]] = n.get((s["cls"], s["precision"]), 0) + s["quartets"]
+    return g, n
+
+
+def test_gradient_part_by_derivative_bound(water):
+    """A quartet's gradient stays in double-float while its density-weighted bound, times the square roots of its
+    largest exponents, is below the threshold: counted here from the Schwarz bounds."""
+    fb, D = water
+    fb.jk(D)
+    part = {s["cls"] for s in fb.slice_info() if s["precision"] == 2}
+    assert part
+    _, n = _forces(fb, D)
+    t, l = fb.table, fb.l
+    off = np.append(fb.ao_offset, fb.nao)
+    M = D.abs().cpu().numpy()
+    M = np.array([[M[off[a]:off[a + 1], off[b]:off[b + 1]].max() for b in range(fb.nshell)] for a in range(fb.nshell)])
+    s = np.sqrt([t["exps"][o:o + k].max() for o, k in zip(t["prim_offset"], t["nprim"])])
+    pairs = [np.array([(a, b) for a in range(fb.nshell) for b in range(fb.nshell)
+                       if (l[a], l[b]) == x and (l[a] > l[b] or a >= b)]) for x in
+             [(0, 0), (1, 0), (1, 1), (2, 0), (2, 1), (2, 2)]]
+    top = fb.q.max() ** 2
+    for cls in part:
+        x = next(k for k in range(6) if k * (k + 1) // 2 <= cls < (k + 1) * (k + 2) // 2)
+        y = cls - x * (x + 1) // 2
+        A, B = pairs[x], pairs[y]
+        q = fb.q[A[:, 0], A[:, 1]][:, None] * fb.q[B[:, 0], B[:, 1]]
+        a, b, c, d = A[:, :1], A[:, 1:], B[:, 0], B[:, 1]
+        bound = q * (0.5 * M[a, b] * M[c, d] + 0.125 * (M[a, c] * M[b, d] + M[a, d] * M[b, c]))
+        low = (q >= CUT) & (q < TAIL * top) & (bound * (s[a] + s[b] + s[c] + s[d]) < TAIL * top * M.max() ** 2)
+        if x == y:   # unordered pairs of pairs: the matrix is symmetric
+            count = (low.sum() + np.diag(low).sum()) / 2
+        else:
+            count = low.sum()
+        assert abs(n[cls, 2] - count) <= 1e-4 * count + 2, cls   # FP32 rounding of the bounds at the threshold
+
+
+def test_gradient_part_follows_the_density(water):
+    """The threshold scales with the density; a density near the ends of FP32's range, or not a number, leaves
+    everything in FP64 and the forces are what FP64 makes of it."""
+    fb, D = water
+    g, n = _forces(fb, D)
+    assert any(k == 2 for _, k in n)
+    for e in (-20, 20):
+        g2, n2 = _forces(fb, D * 2.0 ** e)
+        assert n2 == n
+        # equal quartets and roundings, FP64 sums of fewer than 1e5 terms in another order
+        assert float((g2 * 2.0 ** (-2 * e) - g).abs().max()) <= 1e-11 * float(g.abs().max())
+    for e in (-40, 40):
+        g2, n2 = _forces(fb, D * 2.0 ** e)
+        assert not any(v for (_, k), v in n2.items() if k == 2)
+        # against the double-float part's 2^-44: fewer than 1e5 terms
+        assert float((g2 * 2.0 ** (-2 * e) - g).abs().max()) <= 1e-10 * float(g.abs().max())
+    bad = D.clone()
+    bad[3, 4] = bad[4, 3] = float("nan")
+    g2, n2 = _forces(fb, bad)
+    assert not any(v for (_, k), v in n2.items() if k == 2) and torch.isnan(g2).any()

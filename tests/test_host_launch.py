@@ -114,3 +114,22 @@ def test_demoted_launches_share_the_streams(fake, precision, waters):
     assert len(demoted) > len(low) > 1
     assert 2 * len(set(demoted)) >= len(low)
     fake.L.sf_destroy(h)
+
+
+def test_gradient_launches_of_the_double_float_part(fake):
+    """Gradients keep in double-float only what the classification leaves there: every such launch has an FP64 one
+    of what it takes out, and with the classification off or an FP32 tier beside it the whole part is FP64."""
+    h = fake.handle(_table(6))
+    fake.ok(fake.fock(h, "fp64"))
+    assert {r.kind for r in fake.launches()} == {0, 2}
+    fake.ok(fake.forces(h, "fp64"))
+    runs = fake.launches()
+    dd = {(r.cls, r.count + 8) for r in runs if r.kind == 2}   # the counts of a slice: kept, taken out, ...
+    assert dd and dd <= {(r.cls, r.count) for r in runs if r.kind == 0}
+    fake.ok(fake.L.sf_set_density_screening(h, 0, -1.0, -1.0, -1.0))
+    fake.ok(fake.forces(h, "fp64"))
+    assert {r.kind for r in fake.launches()} == {0}
+    fake.ok(fake.L.sf_set_density_screening(h, 2, -1.0, -1.0, -1.0))
+    fake.ok(fake.forces(h, "mixed"))
+    assert {r.kind for r in fake.launches()} == {0, 1}
+    fake.L.sf_destroy(h)
