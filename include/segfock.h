@@ -376,11 +376,10 @@ int sf_fma_peak(int32_t precision, double *flops, float *ms, void *stream);
  * cannot call cudaMalloc when they build a Fock matrix: code that runs where
  * another component owns all device memory (a framework's memory pool, a
  * fixed memory budget) or a time-critical loop that must not enter the CUDA
- * allocator.  The scratch sf_fock_jk keeps in the handle (the half matrices
- * Jh, Kh and the double-float and single-precision copies of D) lives here in one
- * static device array of the library, sized for nao <= SF_NOALLOC_MAX_NAO (3.5 *
- * 1024^2 doubles = 28 MiB, held on every GPU that loads the library until the
- * process exits).  Larger handles are rejected with SF_EINVAL.
+ * allocator.  The half matrices that sf_fock_jk keeps in the handle are summed in
+ * J and K here, and the copies of D live in one static device array of the
+ * library, sized for nao <= SF_NOALLOC_MAX_NAO (2.5 * 1024^2 doubles = 20 MiB,
+ * held on every GPU that loads the library until the process exits).  Larger handles are rejected with SF_EINVAL.
  *
  * The call allocates nothing: no cudaMalloc, cudaFree or allocating library
  * routine.  Set-up that does allocate must happen before it: sf_create,
@@ -396,7 +395,7 @@ int sf_fma_peak(int32_t precision, double *flops, float *ms, void *stream);
  * assumes the device's primary context is never reset (cudaDeviceReset) while
  * the library is loaded.  Every call shares the one array: calls that overlap on
  * the GPU (other streams, other threads, other handles) race and must be
- * serialised by the caller.  The array is cleared by each call before use. */
+ * serialised by the caller.  Each call writes what it uses of the array first. */
 #define SF_NOALLOC_MAX_NAO 1024
 int sf_fock_jk_noalloc(sf_handle *h, const double *D, double *J, double *K, int32_t precision,
                        double cutoff, double fp32_cutoff, void *stream);

@@ -167,29 +167,82 @@ struct DeviceGuard {
   }
 };
 
-__global__ void symmetrize_kernel(const double *Jh, const double *Kh, double *J, double *K, int n) {
+// scale (null: one): 2^e of density_scale_kernel
+__global__ void symmetrize_kernel(const double *Jh, const double *Kh, double *J, double *K, int n,
+                                  const double *scale) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (int64_t)n * n) return;
   const int i = (int)(idx / n), j = (int)(idx % n);
   const int64_t t = (int64_t)j * n + i;
-  J[idx] = Jh[idx] + Jh[t];
-  K[idx] = Kh[idx] + Kh[t];
+  const double s = scale ? scale[1] : 1.0;
+  J[idx] = (Jh[idx] + Jh[t]) * s;
+  K[idx] = (Kh[idx] + Kh[t]) * s;
+}
+
+// the same in place: one thread per pair of elements
+__global__ void symmetrize_in_place_kernel(double *J, double *K, int n, const double *scale) {
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= (int64_t)n * n) return;
+  const int i = (int)(idx / n), j = (int)(idx % n);
+  if (i > j) return;
+  const int64_t t = (int64_t)j * n + i;
+  const double s = scale ? scale[1] : 1.0;
+  J[idx] = J[t] = (J[idx] + J[t]) * s;
+  K[idx] = K[t] = (K[idx] + K[t]) * s;
+}
+
+// scale[0] = 2^-e, scale[1] = 2^e for a build whose FP64 tier has a double-float part:
+// float pairs lose digits of densities near the ends of FP32's range, which an FP64
+// build takes, so a density whose largest element is outside 2^-20 .. 2^20 is brought
+// to one first (J and K are linear in it; powers of two change no digits).  One that is
+// not finite makes all of J and K not a number (the double-float kernels' conversion to
+// FP64 has no such values).  One CTA: 92 000 elements take 32 us.
+__global__ void __launch_bounds__(1024) density_scale_kernel(const double *D, int64_t nn, double *scale) {
+  // eight loads in flight per thread; the largest bit pattern of |d| is that of the
+  // largest value, of an infinity or above it not a number
+  unsigned long long top = 0;
+  auto take = [&](double d) { top = max(top, (unsigned long long)__double_as_longlong(fabs(d))); };
+  int64_t k = threadIdx.x;
+  for (; k + 7 * 1024 < nn; k += 8 * 1024) {
+    double d[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) d[i] = D[k + i * 1024];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) take(d[i]);
+  }
+  for (; k < nn; k += 1024) take(D[k]);
+  double m = __longlong_as_double((long long)top);
+  const bool finite = __syncthreads_and(top < 0x7ff0000000000000ull);
+  __shared__ double s_m[32];
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
+  if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x) return;
+  for (int w = 1; w < 32; ++w) m = fmax(m, s_m[w]);
+  double up = 1.0;
+  if (m > 0.0 && (m < 0x1p-20 || m > 0x1p20)) up = scalbn(1.0, max(-1000, min(1000, ilogb(m))));
+  scale[0] = finite ? 1.0 / up : 1.0;
+  scale[1] = finite ? up : (double)NAN;
 }
 
 // What a Fock build needs before its class launches, in one launch (as two
 // memsets and two conversions it was a chain of four, 2 to 3 us each in front
 // of a small build: (H2O)3 STO-3G FP32 + double-float replayed 45 -> 41 us): zeroed half
 // matrices (Jh, Kh; null: none), D in FP32 (null: none) and as float pairs
-// (hi, lo) for the dd kernels (null: none)
-__global__ void prepare_kernel(const double *D, double *Jh, double *Kh, float *Df, float2 *Dd, int64_t n) {
+// (hi, lo) for the dd kernels (null: none), D in FP64 (null: none), all of them
+// times scale[0] (null: one).  D may be Jh or Kh where it is copied.
+__global__ void prepare_kernel(const double *D, double *Jh, double *Kh, float *Df, float2 *Dd, double *Dc,
+                               const double *scale, int64_t n) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n) return;
+  const double d = Df || Dd || Dc ? (scale ? D[idx] * scale[0] : D[idx]) : 0.0;
   if (Jh) {
     Jh[idx] = 0.0;
     Kh[idx] = 0.0;
   }
+  if (Dc) Dc[idx] = d;
   if (!Df && !Dd) return;
-  const double d = D[idx];
   const float hi = __double2float_rn(d);
   if (Df) Df[idx] = hi;
   if (Dd) Dd[idx] = make_float2(hi, __double2float_rn(d - (double)hi));
@@ -405,6 +458,7 @@ struct sf_handle {
   DBuf<float4> d_pair32, d_pair32f;   // packed FP32 pair geometry (KParams::pair32, pair32f)
   DBuf<int> d_pfull;               // pair_full per pair
   DBuf<float> d_Ddd;               // density as dd (per build)
+  DBuf<double> d_Ds, d_scale;      // scaled density and its scale (density_scale_kernel)
   DBuf<float> d_cx32, d_cy32, d_cz32;
   DBuf<double> d_tab64, d_boys;
   DBuf<uint2> d_gtab;
@@ -1035,6 +1089,8 @@ int cut_lists(sf_handle *h, int prec, double cut, double cut32) {
     SF_CK(h->d_dem.alloc(all.size()));
     SF_CK(h->d_cnt.alloc(4 * h->slices.size() + 1));
     SF_CK(h->d_dmax.alloc((size_t)h->nshell * h->nshell));
+    for (const auto &sl : h->slices)
+      if (sl.tail) SF_CK(h->d_Ds.alloc((size_t)h->nao * h->nao));
   }
   return SF_OK;
 }
@@ -1189,7 +1245,7 @@ int build_persist(sf_handle *h) {
 // the quartets that the classification took out of it.  In the persistent launch mode (Fock builds, profiling off) the
 // slices of the register tiers are marked covered and one launch per tier
 // runs them, on the FP32 streams.
-int make_plan(sf_handle *h, bool grad, int active) {
+int make_plan(sf_handle *h, bool grad, int active, bool no_dd) {
   h->plan.clear();
   h->pplan.clear();
   h->plan_grad = grad;
@@ -1210,7 +1266,8 @@ int make_plan(sf_handle *h, bool grad, int active) {
     // a gradient runs an FP64 tier's double-float part in FP64 where nothing sorts
     // out the quartets whose derivatives are large (kDDTail)
     const bool split_tail = grad && sl.tail && active && !mixed;
-    sf_handle::Launch L{(int)k, grad && sl.tail && !split_tail ? 0 : sl.prec, h->slice_stream[k], 0, sl.w};
+    const bool fp64_tail = sl.tail && (grad ? !split_tail : no_dd);
+    sf_handle::Launch L{(int)k, fp64_tail ? 0 : sl.prec, h->slice_stream[k], 0, sl.w};
     if (cl) {
       L.w.list = h->d_keep.p + off;
       L.w.count = h->d_cnt.p + 4 * k;
@@ -1390,20 +1447,78 @@ int run_plan(sf_handle *h, bool grad, const double *D, const float *D32, const f
   return SF_OK;
 }
 
-// classification, plan and launches of one Fock build (Jh, Kh) or gradient (g)
-int run_call(sf_handle *h, bool grad, const double *D, const float *D32, const float *Ddd, double *Jh, double *Kh,
-             double *g, double cut, double cut32, cudaStream_t st, int profiling, int *launches) {
+// what a call works on: half matrices (a gradient's: null), copies of D, its scale
+struct CallBufs {
+  double *Jh = nullptr, *Kh = nullptr;
+  float *D32 = nullptr, *Ddd = nullptr;
+  double *Ds = nullptr, *scale = nullptr;
+  bool copy = false;          // the kernels read Ds, not the caller's D
+  bool no_dd = false;         // the double-float part of an FP64 tier in FP64: no Ddd, Ds
+  bool scaled = false;        // set by prepare_build: J and K are to be multiplied by scale[1]
+};
+
+CallBufs handle_bufs(sf_handle *h, bool grad) {
+  CallBufs b;
+  if (!grad) {
+    b.Jh = h->d_Jh.p;
+    b.Kh = h->d_Kh.p;
+  }
+  b.D32 = h->d_D32.p;
+  b.Ddd = h->d_Ddd.p;
+  b.Ds = h->d_Ds.p;
+  b.scale = h->d_scale.p;
+  return b;
+}
+
+// zero Jh and Kh (if asked) and make the copies of D that the current launch list
+// needs; *D becomes the FP64 one where there is one.  A Fock build with a double-float
+// part in its FP64 tier gets a scaled copy (density_scale_kernel), a gradient's
+// classification leaves that part to FP64 for densities out of range.
+int prepare_build(sf_handle *h, bool grad, const double **D, CallBufs &b, bool zero, cudaStream_t st, int *launches) {
+  const int64_t nn = (int64_t)h->nao * h->nao;
+  bool need32 = false, needdd = false, tail = false;
+  for (const auto &s : h->slices) {
+    need32 |= s.prec == 1;
+    if (s.tail && b.no_dd) continue;
+    needdd |= s.prec == 2;
+    tail |= s.tail != 0;
+  }
+  b.scaled = tail && !grad;
+  const bool copy = b.copy || b.scaled;
+  if (!zero && !need32 && !needdd && !copy) return SF_OK;
+  if (b.scaled) {
+    density_scale_kernel<<<1, 1024, 0, st>>>(*D, nn, b.scale);
+    SF_CK(cudaGetLastError());
+    if (launches) ++*launches;
+  }
+  prepare_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(
+      *D, zero ? b.Jh : nullptr, zero ? b.Kh : nullptr, need32 ? b.D32 : nullptr,
+      needdd ? reinterpret_cast<float2 *>(b.Ddd) : nullptr, copy ? b.Ds : nullptr, b.scaled ? b.scale : nullptr, nn);
+  SF_CK(cudaGetLastError());
+  if (launches) ++*launches;
+  if (copy) *D = b.Ds;
+  return SF_OK;
+}
+
+// classification, preparation (prepared: done before, D as that left it), plan and
+// launches of one Fock build (b.Jh, b.Kh) or gradient (g)
+int run_call(sf_handle *h, bool grad, const double *D, CallBufs &b, double *g, double cut, double cut32,
+             cudaStream_t st, int profiling, int *launches, bool prepared = false) {
   int active = 0;
   int rc = density_classify(h, D, grad, cut, cut32, st, launches, &active);
   if (rc) return rc;
-  rc = make_plan(h, grad, active);
+  if (!prepared) {
+    rc = prepare_build(h, grad, &D, b, !grad, st, launches);
+    if (rc) return rc;
+  }
+  rc = make_plan(h, grad, active, b.no_dd);
   if (rc) return rc;
   if (!profiling) make_groups(h);
   if (profiling) {
     rc = profiling_events(h, st);
     if (rc) return rc;
   }
-  return run_plan(h, grad, D, D32, Ddd, Jh, Kh, g, st, profiling, launches);
+  return run_plan(h, grad, D, b.D32, b.Ddd, b.Jh, b.Kh, g, st, profiling, launches);
 }
 
 // events of the profiling modes: two per launch plus the build's start,
@@ -1416,24 +1531,6 @@ int profiling_events(sf_handle *h, cudaStream_t st) {
   }
   if (!h->prof_t0) SF_CK(cudaEventCreate(&h->prof_t0));
   SF_CK(cudaEventRecord(h->prof_t0, st));
-  return SF_OK;
-}
-
-// zero Jh and Kh (null for a gradient) and make the FP32 / double-float copies
-// of D that the current launch list needs
-int prepare_build(sf_handle *h, const double *D, double *Jh, double *Kh, float *D32, float *Ddd, cudaStream_t st,
-                  int *launches) {
-  const size_t nn = (size_t)h->nao * h->nao;
-  bool need32 = false, needdd = false;
-  for (const auto &s : h->slices) {
-    need32 |= s.prec == 1;
-    needdd |= s.prec == 2;
-  }
-  if (!Jh && !need32 && !needdd) return SF_OK;
-  prepare_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(
-      D, Jh, Kh, need32 ? D32 : nullptr, needdd ? reinterpret_cast<float2 *>(Ddd) : nullptr, (int64_t)nn);
-  SF_CK(cudaGetLastError());
-  if (launches) ++*launches;
   return SF_OK;
 }
 
@@ -1667,11 +1764,12 @@ int run_eri_plan(sf_eri_plan *pl, int precision, double *out, cudaStream_t st) {
 
 }  // namespace
 
-// Scratch of sf_fock_jk_noalloc: Jh and Kh (nao^2 doubles each) followed by
-// the double-float copy of D (nao^2 float pairs) and its single-precision copy
-// (nao^2 floats), for nao <= SF_NOALLOC_MAX_NAO.
+// Scratch of sf_fock_jk_noalloc: D (nao^2 doubles) and its double-float copy (nao^2
+// float pairs), or the half matrices; its single-precision copy (nao^2 floats), for
+// nao <= SF_NOALLOC_MAX_NAO; then D's scale.
 static constexpr size_t kNoAllocNN = (size_t)SF_NOALLOC_MAX_NAO * SF_NOALLOC_MAX_NAO;
-static __device__ __align__(256) double g_noalloc_scratch[3 * kNoAllocNN + (kNoAllocNN + 1) / 2];
+static constexpr size_t kNoAllocScale = 2 * kNoAllocNN + (kNoAllocNN + 1) / 2;
+static __device__ __align__(256) double g_noalloc_scratch[kNoAllocScale + 2];
 
 namespace {
 // device address of g_noalloc_scratch per device (host code cannot use the
@@ -1843,6 +1941,7 @@ int sf_create(const sf_shell_desc *shells, int32_t nshell, sf_handle **out) {
   SF_CK(h->d_tab32.upload(T.t32v));
   SF_CK(h->d_tabdd.upload(T.tdd));
   SF_CK(h->d_Ddd.alloc(2 * (size_t)nao * nao));
+  SF_CK(h->d_scale.alloc(2));
   SF_CK(h->d_Jh.alloc((size_t)nao * nao));
   SF_CK(h->d_Kh.alloc((size_t)nao * nao));
   SF_CK(h->d_D32.alloc((size_t)nao * nao));
@@ -2054,12 +2153,10 @@ int sf_fock_jk(sf_handle *h, const double *D, double *J, double *K, int32_t prec
   const int n = h->nao;
   const size_t nn = (size_t)n * n;
   int launches = 0;
-  rc = prepare_build(h, D, h->d_Jh.p, h->d_Kh.p, h->d_D32.p, h->d_Ddd.p, st, &launches);
+  CallBufs b = handle_bufs(h, false);
+  rc = run_call(h, false, D, b, nullptr, cutoff, fp32_cutoff, st, h->profiling, &launches);
   if (rc) return rc;
-  rc = run_call(h, false, D, h->d_D32.p, h->d_Ddd.p, h->d_Jh.p, h->d_Kh.p, nullptr, cutoff, fp32_cutoff, st, h->profiling,
-                &launches);
-  if (rc) return rc;
-  symmetrize_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(h->d_Jh.p, h->d_Kh.p, J, K, n);
+  symmetrize_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(b.Jh, b.Kh, J, K, n, b.scaled ? b.scale : nullptr);
   SF_CK(cudaGetLastError());
   ++launches;
   if (stats) {
@@ -2155,7 +2252,9 @@ int sf_autotune(sf_handle *h, const double *D, int32_t precision, double cutoff,
   cudaStream_t st = (cudaStream_t)stream;
   int rc = build_work(h, precision, cutoff, fp32_cutoff, st);
   if (rc) return rc;
-  rc = prepare_build(h, D, nullptr, nullptr, h->d_D32.p, h->d_Ddd.p, st, nullptr);
+  CallBufs b = handle_bufs(h, false);
+  const double *Dk = D;   // what the kernels read
+  rc = prepare_build(h, false, &Dk, b, false, st, nullptr);
   if (rc) return rc;
   cudaEvent_t e0, e1;
   SF_CK(cudaEventCreate(&e0));
@@ -2168,7 +2267,7 @@ int sf_autotune(sf_handle *h, const double *D, int32_t precision, double cutoff,
     ClassWork w = sl.w;
     w.psplit = std::min(S, pmax);
     w.wsplit = S / w.psplit;
-    auto launch = [&]() { return launch_slice(h, sl, w, D, h->d_D32.p, h->d_Jh.p, h->d_Kh.p, st); };
+    auto launch = [&]() { return launch_slice(h, sl, w, Dk, b.D32, b.Jh, b.Kh, st); };
     cudaError_t e = launch();   // warm-up
     if (e == cudaSuccess) e = cudaEventRecord(e0, st);
     for (int r = 0; r < reps && e == cudaSuccess; ++r) e = launch();
@@ -2182,12 +2281,11 @@ int sf_autotune(sf_handle *h, const double *D, int32_t precision, double cutoff,
   auto time_build = [&](float *ms) -> int {
     int r2 = build_work(h, precision, cutoff, fp32_cutoff, st);
     if (r2) return r2;
-    r2 = run_call(h, false, D, h->d_D32.p, h->d_Ddd.p, h->d_Jh.p, h->d_Kh.p, nullptr, cutoff, fp32_cutoff, st, 0,
-                  nullptr);   // warm-up
+    r2 = run_call(h, false, Dk, b, nullptr, cutoff, fp32_cutoff, st, 0, nullptr, true);   // warm-up
     if (r2) return r2;
     SF_CK(cudaEventRecord(e0, st));
     for (int r = 0; r < reps; ++r) {
-      r2 = run_call(h, false, D, h->d_D32.p, h->d_Ddd.p, h->d_Jh.p, h->d_Kh.p, nullptr, cutoff, fp32_cutoff, st, 0, nullptr);
+      r2 = run_call(h, false, Dk, b, nullptr, cutoff, fp32_cutoff, st, 0, nullptr, true);
       if (r2) return r2;
     }
     SF_CK(cudaEventRecord(e1, st));
@@ -2395,14 +2493,27 @@ int sf_fock_jk_noalloc(sf_handle *h, const double *D, double *J, double *K, int3
   cudaStream_t st = (cudaStream_t)stream;
   const int n = h->nao;
   const size_t nn = (size_t)n * n;
-  double *Jh = scratch, *Kh = scratch + nn;
-  float *Ddd = reinterpret_cast<float *>(scratch + 2 * nn);   // nao^2 float pairs, then nao^2 floats
-  float *D32 = reinterpret_cast<float *>(scratch + 3 * nn);
-  int rc = prepare_build(h, D, Jh, Kh, D32, Ddd, st, nullptr);
+  CallBufs b;
+  const bool apart = std::max(J, K) - std::min(J, K) >= (ptrdiff_t)nn;
+  if (apart) {   // the half matrices are summed in the caller's, D is copied (it may be one of them)
+    b.Jh = J;
+    b.Kh = K;
+    b.copy = true;
+    b.Ds = scratch;
+    b.Ddd = reinterpret_cast<float *>(scratch + nn);   // nao^2 float pairs
+  } else {       // J and K share memory (K is left there): half matrices in the scratch instead
+    b.Jh = scratch;
+    b.Kh = scratch + nn;
+    b.no_dd = true;
+  }
+  b.D32 = reinterpret_cast<float *>(scratch + 2 * nn);   // nao^2 floats
+  b.scale = scratch + kNoAllocScale;
+  int rc = run_call(h, false, D, b, nullptr, cutoff, fp32_cutoff, st, 0, nullptr);
   if (rc) return rc;
-  rc = run_call(h, false, D, D32, Ddd, Jh, Kh, nullptr, cutoff, fp32_cutoff, st, 0, nullptr);
-  if (rc) return rc;
-  symmetrize_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(Jh, Kh, J, K, n);
+  const double *scale = b.scaled ? b.scale : nullptr;
+  const unsigned grid = (unsigned)((nn + 255) / 256);
+  if (apart) symmetrize_in_place_kernel<<<grid, 256, 0, st>>>(J, K, n, scale);
+  else symmetrize_kernel<<<grid, 256, 0, st>>>(b.Jh, b.Kh, J, K, n, scale);
   SF_CK(cudaGetLastError());
   return SF_OK;
 }
@@ -2418,10 +2529,9 @@ int sf_grad_jk(sf_handle *h, const double *D, double *grad, int32_t precision, d
   cudaStream_t st = (cudaStream_t)stream;
   int rc = build_work(h, precision, cutoff, fp32_cutoff, st);
   if (rc) return rc;
-  rc = prepare_build(h, D, nullptr, nullptr, h->d_D32.p, h->d_Ddd.p, st, nullptr);
-  if (rc) return rc;
   // per-launch events in the profiling modes (serialised in mode 2), read by sf_get_slice_info
-  return run_call(h, true, D, h->d_D32.p, h->d_Ddd.p, nullptr, nullptr, grad, cutoff, fp32_cutoff, st, h->profiling, nullptr);
+  CallBufs b = handle_bufs(h, true);
+  return run_call(h, true, D, b, grad, cutoff, fp32_cutoff, st, h->profiling, nullptr);
 }
 
 int sf_grad_stats(sf_handle *h, sf_stats *stats, void *stream) {

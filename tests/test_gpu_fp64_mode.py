@@ -86,3 +86,40 @@ def test_gradient_part_follows_the_density(water):
     bad[3, 4] = bad[4, 3] = float("nan")
     g2, n2 = _forces(fb, bad)
     assert not any(v for (_, k), v in n2.items() if k == 2) and torch.isnan(g2).any()
+
+
+@pytest.mark.parametrize("call", ["handle", "noalloc"])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_density_outside_the_range_of_fp32(water, precision, call):
+    """J and K are linear in the density over FP64's whole range, with part of the build in double-float: powers of
+    two change no digits, FP64 sums of fewer than 1e4 terms come in another order.  Not a number, or infinite, in one
+    element: so are J and K.  The output may be the density's own matrix."""
+    from segfault_py_gb300 import _lib
+    from segfault_py_gb300.fock import _ptr, _stream_ptr
+    fb, D = water
+    n, cut32 = fb.nao, 1e-6
+
+    def jk(D, J=None, K=None):
+        J, K = (torch.full_like(D, 7.0) if m is None else m for m in (J, K))
+        run = _lib.lib().sf_fock_jk_noalloc if call == "noalloc" else \
+            lambda *a: _lib.lib().sf_fock_jk(*a[:-1], None, a[-1])
+        _lib.check(run(fb.handle, _ptr(D), _ptr(J), _ptr(K), _lib.PRECISION[precision], CUT, cut32, _stream_ptr()))
+        return J, K
+
+    ref = fb.jk(D, precision=precision, fp32_cutoff=cut32)
+    assert any(s["precision"] == 2 and s["quartets"] for s in fb.slice_info())
+    for e in (0, -30, 30, -140, 140, -900, 900):
+        for got, r in zip(jk(D * 2.0 ** e), ref):
+            got = got * 2.0 ** (-e // 2) * 2.0 ** (-e - -e // 2)
+            assert float((got - r).abs().max()) <= 1e-12 * float(r.abs().max()), e
+    for bad in (float("nan"), float("inf")):
+        B = D.clone()
+        B[2, 9] = B[9, 2] = bad
+        assert not any(torch.isfinite(m).any() for m in jk(B))
+    own = D.clone()
+    for got, r in zip(jk(own, J=own), ref):
+        assert float((got - r).abs().max()) <= 1e-12 * float(r.abs().max())
+    both = D.clone()
+    jk(D, J=both, K=both)   # one matrix for both: K
+    assert float((both - ref[1]).abs().max()) <= 1e-12 * float(ref[1].abs().max())
+    assert torch.isfinite(jk(torch.zeros_like(D))[0]).all()
