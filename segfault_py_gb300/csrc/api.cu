@@ -1016,18 +1016,22 @@ int cut_lists(sf_handle *h, int prec, double cut, double cut32) {
     }
     // launches timed by the autotuner: their measured times (a latency-bound
     // launch of few quartets costs far more than its work suggests)
-    bool all_timed = !h->slices.empty();
+    // double-float parts of FP64 tiers are not timed: their estimates, in that unit
+    bool all_timed = true;
     std::vector<double> timed(h->slices.size(), 0.0);
-    for (size_t k = 0; k < h->slices.size() && all_timed; ++k) {
+    double ms = 0.0, est = 0.0;
+    for (size_t k = 0; k < h->slices.size(); ++k) {
       const auto &sl = h->slices[k];
-      bool found = false;
+      if (sl.tail) continue;
       for (const sf_tune_entry &e : h->tune)
-        if (!sl.tail && e.cls == sl.cls && e.precision == sl.prec && e.cost == sl.cost_hi && e.ms_tuned > 0.f) {
-          timed[k] = e.ms_tuned;
-          found = true;
-        }
-      all_timed = found;
+        if (e.cls == sl.cls && e.precision == sl.prec && e.cost == sl.cost_hi && e.ms_tuned > 0.f) timed[k] = e.ms_tuned;
+      all_timed &= timed[k] > 0.0;
+      ms += timed[k];
+      est += cost[k];
     }
+    all_timed &= est > 0.0;
+    for (size_t k = 0; k < h->slices.size() && all_timed; ++k)
+      if (h->slices[k].tail) timed[k] = cost[k] * (ms / est);
     if (all_timed) cost = timed;
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });

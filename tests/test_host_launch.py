@@ -133,3 +133,24 @@ def test_gradient_launches_of_the_double_float_part(fake):
     fake.ok(fake.forces(h, "mixed"))
     assert {r.kind for r in fake.launches()} == {0, 1}
     fake.L.sf_destroy(h)
+
+
+@pytest.mark.parametrize("waters,part", [(2, False), (6, True)])
+def test_measured_times_order_the_launches(fake, waters, part):
+    """Measured launch times decide the order and the streams, also where part of the build is in double-float,
+    which is not tuned and goes by its estimate."""
+    from segfault_py_gb300 import _lib
+    h = fake.handle(_table(waters))
+    costs = range(1, 36 * 36 + 1)
+    entries = [_lib.TuneEntry(cls=c, precision=0, cost=k, split=1, ms_default=1.0, ms_tuned=1e4 if c == 20 else 1.0)
+               for c in range(21) for k in costs]
+    arr = (_lib.TuneEntry * len(entries))(*entries)
+    fake.ok(fake.L.sf_set_tuning(h, arr, len(entries)))
+    fake.ok(fake.fock(h, "fp64"))
+    runs = fake.launches()
+    assert any(r.kind == 2 for r in runs) == part
+    assert [r.cls for r in runs if r.kind == 0][0] == 20   # (dd|dd), the cheapest by its estimate
+    if part:   # estimates in the measured times' unit: neither all before nor all after the timed launches
+        kinds = [r.kind for r in runs]
+        assert kinds != sorted(kinds) and kinds != sorted(kinds, reverse=True)
+    fake.L.sf_destroy(h)
