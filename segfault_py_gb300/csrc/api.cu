@@ -906,7 +906,7 @@ int cut_lists(sf_handle *h, int prec, double cut, double cut32) {
       return 1;
     };
     const int fx4 = (pr == 0 && h->fill_acc_x4[prec] >= 0) ? h->fill_acc_x4[prec] : h->fill_x4[prec];
-    const double lanes = (double)std::max(h->nsm, 1) * 4 * 8 * 32 * fx4 / 4.0;
+    const double all_lanes = (double)std::max(h->nsm, 1) * 4 * 8 * 32, lanes = all_lanes * fx4 / 4.0;
     int sfill = pmax * kMaxWsplit;
     double share = 0.0;   // work of a sub-group above which it is split further
     if (pr == 1) {
@@ -938,7 +938,8 @@ int cut_lists(sf_handle *h, int prec, double cut, double cut32) {
       seg.off = q0;
       seg.n = q1 - q0;
       seg.cost_hi = cost;
-      seg.rel_load = load[kind] > 0.0 ? (float)(part.per_prim * lanes / load[kind]) : 0.0f;
+      // not by the fill target: that is tuned for Fock builds
+      seg.rel_load = load[kind] > 0.0 ? (float)(part.per_prim * all_lanes / load[kind]) : 0.0f;
       int St = S;
       for (const sf_tune_entry &e : h->tune)
         if (!p.tail && e.cls == cls && e.precision == kind && e.cost == seg.cost_hi) St = e.split;

@@ -154,3 +154,26 @@ def test_measured_times_order_the_launches(fake, waters, part):
         kinds = [r.kind for r in runs]
         assert kinds != sorted(kinds) and kinds != sorted(kinds, reverse=True)
     fake.L.sf_destroy(h)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed_df"])
+@pytest.mark.parametrize("fill", [0, 1, 16])
+def test_gradient_splits_do_not_follow_the_tuned_fill(fake, precision, fill):
+    """The fill target that the autotuner finds for a mode's Fock builds (0: no extra split) is not the gradient's:
+    its splits go by the work per lane of the whole GPU."""
+    from segfault_py_gb300 import _lib
+    h = fake.handle(_table(3))
+
+    def loads():
+        fake.ok(fake.forces(h, precision, cut32=1e-2))
+        out = {}
+        for r in fake.launches():
+            out.setdefault((r.cls, r.kind), set()).add(r.rel_load)
+        return out
+
+    ref = loads()
+    arr = (_lib.TuneEntry * 2)(*[_lib.TuneEntry(cls=c, precision=_lib.PRECISION[precision], cost=0, split=fill)
+                                 for c in (-1, -2)])
+    fake.ok(fake.L.sf_set_tuning(h, arr, 2))
+    assert loads() == ref
+    fake.L.sf_destroy(h)
