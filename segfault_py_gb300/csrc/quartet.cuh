@@ -1674,8 +1674,10 @@ __device__ __forceinline__ unsigned cluster_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
+// not the .aligned forms: threads come here from loops with different trip counts, and
+// nothing makes a warp's threads arrive together
 __device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 // a 4-byte word at the same shared-memory address in CTA `rank` of the cluster
 __device__ __forceinline__ unsigned ld_cluster(const void *p, unsigned rank) {
