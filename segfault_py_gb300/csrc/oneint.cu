@@ -121,6 +121,14 @@ __host__ __device__ constexpr int tuv_index(int L, int t, int u, int v) {
   return k + v;
 }
 
+// Growth of a kinetic integral over its overlap: T = 1/2 sum_d <d_d a | d_d b>, where a
+// derivative of x_A^la exp(-alpha x_A^2) brings la / x_A - 2 alpha x_A, and alpha |x_A|
+// reaches mu |AB| + alpha / sqrt(p) around P (mu = alpha beta / p; likewise at B)
+__device__ __forceinline__ float kinetic_bound(int la, int lb, float al, float be, float p, float R) {
+  const float r = rsqrtf(p), mr = al * r * (be * r) * R;
+  return 1.5f * (la + 2.0f * (mr + al * r)) * (lb + 2.0f * (mr + be * r));
+}
+
 // S, T, V: one warp per canonical shell pair of the handle's pair table
 // (a, b), l_a >= l_b, reading the primitive-pair records of the two-electron
 // kernels, so that p, P and the product Gaussian cost nothing here.  What
@@ -140,7 +148,7 @@ __host__ __device__ constexpr int tuv_index(int L, int t, int u, int v) {
 // Primitive pairs whose contributions all stay below 1e-17 are skipped (the
 // product Gaussian c_i c_j exp(-mu |AB|^2) (pi/p)^3/2 bounds the overlap, E
 // coefficients grow at most as (|AB| + 1/sqrt(p) + 1)^L, kinetic terms as
-// 3 beta (LB + 2) and attraction as 2 sqrt(p/pi) times the summed charge; the
+// kinetic_bound and attraction as 2 sqrt(p/pi) times the summed charge; the
 // bound itself in FP32).
 // (H2O)16 6-31G* (48 nuclei, 68 k primitive pairs): 0.32 ms; one CTA of 64 threads
 // per pair, with the power series, exp and pow per primitive pair and three
@@ -178,7 +186,7 @@ __device__ __forceinline__ void one_pair(const OneParams &P, int pair, double *s
     const int ip = i0 + sub;
     bool on = ip < np;
     const double *rec = rec0 + (size_t)(on ? ip : 0) * kPrimRec;
-    const double p = rec[0], Pc[3] = {rec[1], rec[2], rec[3]}, kt = rec[4], hp = rec[5], be = rec[7];
+    const double p = rec[0], Pc[3] = {rec[1], rec[2], rec[3]}, kt = rec[4], hp = rec[5], al = rec[6], be = rec[7];
     {
       // kt = c_i c_j exp(-mu R^2) sqrt(2) pi^(5/4) / p
       const float pf = (float)p, g = fabsf((float)kt) * 0.9414f * rsqrtf(pf);   // overlap bound
@@ -186,7 +194,7 @@ __device__ __forceinline__ void one_pair(const OneParams &P, int pair, double *s
       float e = 1.0f;
 #pragma unroll
       for (int k = 0; k < L; ++k) e *= x;
-      const float f = 1.0f + 1.1284f * sqrtf(pf) * (float)zs + 3.0f * (float)be * (LB + 2);
+      const float f = 1.0f + 1.1284f * sqrtf(pf) * (float)zs + kinetic_bound(LA, LB, (float)al, (float)be, pf, R1);
       if (g * e * f < 1e-17f) on = false;   // not on NaN: it has to reach the matrix it belongs to
     }
     if (!__any_sync(0xffffffffu, on)) continue;
@@ -412,7 +420,8 @@ __device__ __forceinline__ void one_pair_grad(const OneParams &P, const double *
       float e = x;
 #pragma unroll
       for (int k = 0; k < L; ++k) e *= x;
-      const float f = (2.0f * mx + L1) * (1.0f + 1.1284f * sqrtf(pf) * zs + 3.0f * mx * (LB + 2));
+      const float f = (2.0f * mx + L1) * (1.0f + 1.1284f * sqrtf(pf) * zs +
+                                          kinetic_bound(LA + 1, LB + 1, (float)al, (float)be, pf, R1));
       if (g * e * f < 1e-15f) on = false;   // not on NaN: it has to reach the forces
     }
     if (!__any_sync(0xffffffffu, on)) continue;
