@@ -446,8 +446,8 @@ struct sf_handle {
   double qmax = 0.0;          // largest Schwarz bound of a pair
   bool dd_range = true;       // every primitive record well inside FP32's range
   std::vector<int> pairmap;   // a*nshell+b -> pair index (a,b canonical)
-  DBuf<int> d_l, d_nprim, d_ao, d_atom, d_spoff;
-  DBuf<double> d_cx, d_cy, d_cz, d_exps, d_coefs;
+  DBuf<int> d_l, d_nprim, d_ao, d_atom;
+  DBuf<double> d_cx, d_cy, d_cz;
   DBuf<int> d_pa, d_pb, d_ppoff, d_pnp;
   DBuf<double> d_pq;
   DBuf<double> d_pp64;
@@ -1923,11 +1923,9 @@ int sf_create(const sf_shell_desc *shells, int32_t nshell, sf_handle **out) {
   SF_CK(h->d_nprim.upload(h->nprim));
   SF_CK(h->d_ao.upload(h->ao));
   SF_CK(h->d_atom.upload(h->atom));
-  SF_CK(h->d_spoff.upload(h->spoff));
   SF_CK(h->d_cx.upload(h->cx));
   SF_CK(h->d_cy.upload(h->cy));
   SF_CK(h->d_cz.upload(h->cz));
-  SF_CK(h->d_exps.upload(h->exps));
   {
     std::vector<float> sqa(h->nshell);
     for (int a = 0; a < h->nshell; ++a) {
@@ -1937,7 +1935,6 @@ int sf_create(const sf_shell_desc *shells, int32_t nshell, sf_handle **out) {
     }
     SF_CK(h->d_sqa.upload(sqa));
   }
-  SF_CK(h->d_coefs.upload(h->coefs));
   const HostTables &T = host_tables();
   SF_CK(h->d_tab64.upload(T.t64));
   SF_CK(h->d_boys.upload(T.boys));

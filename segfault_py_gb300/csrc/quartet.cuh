@@ -332,18 +332,15 @@ __device__ __forceinline__ void rys_roots_all(const KParams &kp, R x, R (&u)[N],
   }
 }
 
-// the FP64 rule from an explicit table and asymptotic constants (also used by
-// the one-electron kernels, whose Boys values are sum_i w_i u_i^m)
 template <int N>
-__device__ __forceinline__ void rys_roots_f64_tab(const double *tab64, const RysAsym &asym, double x,
-                                                  double (&u)[N], double (&w)[N]) {
+__device__ __forceinline__ void rys_roots_all_f64(const KParams &kp, double x, double (&u)[N], double (&w)[N]) {
   using R = double;
   if (!(x < (R)kTabXmax)) {   // NaN too: it has no table row
     const R ix = (R)1 / x, isx = rsqrt_nr(x);
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      u[i] = (R)asym.r[N][i] * ix;
-      w[i] = (R)asym.w[N][i] * isx;
+      u[i] = (R)kp.asym.r[N][i] * ix;
+      w[i] = (R)kp.asym.w[N][i] * isx;
     }
     return;
   }
@@ -351,7 +348,7 @@ __device__ __forceinline__ void rys_roots_f64_tab(const double *tab64, const Rys
   constexpr int D = TabDeg<R>::v;
   const int j = (int)x;
   const R s = (R)2 * (x - (R)j) - (R)1;
-  const V *c = reinterpret_cast<const V *>(tab64 + rys_tab_offset(N, D) + j * (D + 1) * 2 * N);
+  const V *c = reinterpret_cast<const V *>(kp.tab64 + rys_tab_offset(N, D) + j * (D + 1) * 2 * N);
   R f[2 * N];
 #pragma unroll
   for (int i = 0; i < N; ++i) {
@@ -373,11 +370,6 @@ __device__ __forceinline__ void rys_roots_f64_tab(const double *tab64, const Rys
     u[i] = f[i];
     w[i] = f[N + i];
   }
-}
-
-template <int N>
-__device__ __forceinline__ void rys_roots_all_f64(const KParams &kp, double x, double (&u)[N], double (&w)[N]) {
-  rys_roots_f64_tab<N>(kp.tab64, kp.asym, x, u, w);
 }
 
 // one root r of the n-point rule
@@ -551,10 +543,7 @@ __device__ __forceinline__ void rys_2d_dd(dd g0, dd c00, dd c00p, dd b00, dd b10
 // Output I[((ia*(LB+1)+ib)*(LC+1)+ic)*(LD+1)+id].
 template <int LA, int LB, int LC, int LD, typename R>
 __device__ __forceinline__ void rys_2d(R g0, R c00, R c00p, R b00, R b10, R b01, R ab, R cd, R *__restrict__ I) {
-  if constexpr (std::is_same<R, dd>::value) {
-    rys_2d_dd<LA, LB, LC, LD, false>(g0, c00, c00p, b00, b10, b01, ab, cd, I);
-    return;
-  } else {
+  static_assert(!std::is_same<R, dd>::value, "rys_2d_dd");
   constexpr int LAB = LA + LB, LCD = LC + LD;
   R G[LAB + 1][LCD + 1];
   G[0][0] = g0;
@@ -608,7 +597,6 @@ __device__ __forceinline__ void rys_2d(R g0, R c00, R c00p, R b00, R b10, R b01,
         for (int ic = 0; ic <= LC; ++ic) I[((ia * (LB + 1) + ib) * (LC + 1) + ic) * (LD + 1) + id] = t[ic];
       }
     }
-  }
   }
 }
 
@@ -989,22 +977,22 @@ __device__ __forceinline__ void eval_t1(const KParams &kp, const QGeom<R> &g, R 
       // per primitive quartet, so that lo does not grow over a long contraction
 #pragma unroll
       for (int o = 0; o < Q::NABCD; ++o) acc[o] = dd_norm(acc[o]);
-      continue;
-    }
+    } else {
 #pragma unroll
-    for (int r = 0; r < NR; ++r) {
-      const R uu = u[r];
-      const R b00 = (R)0.5 * s.r2 * uu;
-      const R b10 = s.i2p * ((R)1 - s.aq * uu);
-      const R b01 = s.i2q * ((R)1 - s.ap * uu);
-      const R tq = s.aq * uu, tp = s.ap * uu;
-      R Ix[SZ], Iy[SZ], Iz[SZ];
-      rys_2d<LA, LB, LC, LD, R>((R)1, s.pax - tq * s.pqx, s.qcx + tp * s.pqx, b00, b10, b01, g.ABx, g.CDx, Ix);
-      rys_2d<LA, LB, LC, LD, R>((R)1, s.pay - tq * s.pqy, s.qcy + tp * s.pqy, b00, b10, b01, g.ABy, g.CDy, Iy);
-      rys_2d<LA, LB, LC, LD, R>(s.pref * w[r], s.paz - tq * s.pqz, s.qcz + tp * s.pqz, b00, b10, b01, g.ABz,
-                                g.CDz, Iz);
+      for (int r = 0; r < NR; ++r) {
+        const R uu = u[r];
+        const R b00 = (R)0.5 * s.r2 * uu;
+        const R b10 = s.i2p * ((R)1 - s.aq * uu);
+        const R b01 = s.i2q * ((R)1 - s.ap * uu);
+        const R tq = s.aq * uu, tp = s.ap * uu;
+        R Ix[SZ], Iy[SZ], Iz[SZ];
+        rys_2d<LA, LB, LC, LD, R>((R)1, s.pax - tq * s.pqx, s.qcx + tp * s.pqx, b00, b10, b01, g.ABx, g.CDx, Ix);
+        rys_2d<LA, LB, LC, LD, R>((R)1, s.pay - tq * s.pqy, s.qcy + tp * s.pqy, b00, b10, b01, g.ABy, g.CDy, Iy);
+        rys_2d<LA, LB, LC, LD, R>(s.pref * w[r], s.paz - tq * s.pqz, s.qcz + tp * s.pqz, b00, b10, b01, g.ABz,
+                                  g.CDz, Iz);
 #pragma unroll
-      for (int o = 0; o < Q::NABCD; ++o) acc[o] += Ix[Q::toff(o, 0)] * Iy[Q::toff(o, 1)] * Iz[Q::toff(o, 2)];
+        for (int o = 0; o < Q::NABCD; ++o) acc[o] += Ix[Q::toff(o, 0)] * Iy[Q::toff(o, 1)] * Iz[Q::toff(o, 2)];
+      }
     }
   }
 }
