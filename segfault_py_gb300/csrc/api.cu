@@ -17,13 +17,13 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
-#include <thread>
 #include <atomic>
 #include <numeric>
 #include <string>
 #include <vector>
 
 #include "classes.h"
+#include "host_threads.h"
 #include "launch.h"
 #include "segfock.h"
 
@@ -961,10 +961,7 @@ int cut_lists(sf_handle *h, int prec, double cut, double cut32) {
       std::vector<int64_t> hist((size_t)KB * KB), full((size_t)KB * KB);
       for (int c = next++; c < kNumClass; c = next++) build_class(c, hist, full);
     };
-    std::vector<std::thread> pool;
-    for (int t = 1; t < nthr; ++t) pool.emplace_back(worker);
-    worker();
-    for (auto &t : pool) t.join();
+    on_threads(nthr, worker);
     double load[3] = {0.0, 0.0, 0.0};   // per arithmetic
     for (const Part &part : parts) load[part.head.prec] += part.load;
     load32 = load[1];

@@ -32,9 +32,9 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
-#include <thread>
 #include <vector>
 
+#include "host_threads.h"
 #include "sf_internal.h"
 
 namespace sf {
@@ -221,10 +221,7 @@ void rys_build_fine(double *tab) {
       }
     }
   };
-  std::vector<std::thread> pool;
-  for (unsigned t = 1; t < std::min(std::thread::hardware_concurrency(), 8u); ++t) pool.emplace_back(worker);
-  worker();
-  for (auto &t : pool) t.join();
+  on_threads((int)std::min(std::thread::hardware_concurrency(), 8u), worker);
 }
 
 // Boys functions and e^-T (sf_internal.h), interpolated at the Chebyshev nodes

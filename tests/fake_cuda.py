@@ -178,7 +178,7 @@ def make(out_dir):
 
 class Fake:
     def __init__(self, path):
-        self.L = C.CDLL(path)
+        self.path = path
         real, path0, _lib._lib, _lib.LIB_PATH = _lib._lib, _lib.LIB_PATH, None, path
         try:
             self.L = _lib.lib()   # the argument types

@@ -177,3 +177,48 @@ def test_gradient_splits_do_not_follow_the_tuned_fill(fake, precision, fill):
     fake.ok(fake.L.sf_set_tuning(h, arr, 2))
     assert loads() == ref
     fake.L.sf_destroy(h)
+
+
+NO_THREADS = r"""
+#include <dlfcn.h>
+#include <errno.h>
+#include <pthread.h>
+int refuse_threads = 0;
+int pthread_create(pthread_t *t, const pthread_attr_t *a, void *(*f)(void *), void *arg) {
+  static int (*real)(pthread_t *, const pthread_attr_t *, void *(*)(void *), void *);
+  if (refuse_threads) return EAGAIN;
+  if (!real) real = (int (*)(pthread_t *, const pthread_attr_t *, void *(*)(void *), void *))dlsym(RTLD_NEXT, "pthread_create");
+  return real(t, a, f, arg);
+}
+"""
+
+NO_THREADS_RUN = """
+import ctypes, sys
+sys.path[:0] = [%(tests)r, %(repo)r]
+import fake_cuda
+from test_host_launch import _table
+fake = fake_cuda.Fake(%(lib)r)
+ctypes.c_int.in_dll(ctypes.CDLL(%(pre)r), "refuse_threads").value = 1
+h = fake.handle(_table(6))
+fake.ok(fake.fock(h, "fp64"))
+print(len(fake.launches()))
+"""
+
+
+def test_no_threads_to_be_had(fake, tmp_path):
+    """Where the system gives no more threads, the tables and the quartet lists are made on the caller's."""
+    import os
+    import subprocess
+    import sys
+    src, pre = tmp_path / "nothreads.c", tmp_path / "nothreads.so"
+    src.write_text(NO_THREADS)
+    subprocess.run(["gcc", "-D_GNU_SOURCE", "-shared", "-fPIC", str(src), "-o", str(pre), "-ldl"], check=True)
+    here = os.path.dirname(os.path.abspath(__file__))
+    code = NO_THREADS_RUN % dict(tests=here, repo=os.path.dirname(here), lib=fake.path, pre=str(pre))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True,
+                       env=dict(os.environ, LD_PRELOAD=str(pre)))
+    assert r.returncode == 0, r.stderr
+    h = fake.handle(_table(6))
+    fake.ok(fake.fock(h, "fp64"))
+    assert int(r.stdout) == len(fake.launches()) > 0
+    fake.L.sf_destroy(h)
