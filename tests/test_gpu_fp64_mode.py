@@ -123,3 +123,36 @@ def test_density_outside_the_range_of_fp32(water, precision, call):
     jk(D, J=both, K=both)   # one matrix for both: K
     assert float((both - ref[1]).abs().max()) <= 1e-12 * float(ref[1].abs().max())
     assert torch.isfinite(jk(torch.zeros_like(D))[0]).all()
+
+
+def test_double_float_part_by_class(cuda):
+    """All 21 classes with a double-float part against the same quartets in FP64 throughout (a shell outside FP32's
+    range, uncoupled, keeps that handle there).  The part's terms carry 2^-44 and add up to at most ten times the
+    largest element: 1e-12 of it in J and K, 1e-11 in the forces, whose terms reach further above their sums."""
+    from segfault_py_gb300 import _lib
+    from segfault_py_gb300.fock import FockBuilder, _ptr, _stream_ptr
+    from test_gpu_kernel_edges import _table
+    ls = [0, 1, 2] * 36
+    table = _table(ls, [2, 1, 1] * 36, 6, 9.0)
+    n, m = sum((l + 1) * (l + 2) // 2 for l in ls), len(ls)
+    more = dict(table, l=np.append(table["l"], 0), nprim=np.append(table["nprim"], 1), atom=np.append(table["atom"], m),
+                ao_offset=np.append(table["ao_offset"], n), center=np.vstack([table["center"], [[4.0, 4.0, 4.0]]]),
+                prim_offset=np.append(table["prim_offset"], table["prim_offset"][-1] + 1),
+                exps=np.append(table["exps"], 1e10), coefs=np.append(table["coefs"], 1e-3))
+    more = {k: v.astype(table[k].dtype) for k, v in more.items()}
+    D = np.zeros((n + 1, n + 1))
+    D[:n, :n] = _sym(n, 9)
+    out = []
+    for t, size in ((table, n), (more, n + 1)):
+        fb = FockBuilder(t, device=cuda, cutoff=1e-12, precision="fp64")
+        Dd = torch.tensor(np.ascontiguousarray(D[:size, :size]), device=cuda)
+        J, K = fb.jk(Dd)
+        part = {s["cls"] for s in fb.slice_info() if s["precision"] == 2}
+        assert part == (set(range(21)) if size == n else set())
+        g = torch.zeros(3 * (m + 1), dtype=torch.float64, device=cuda)
+        _lib.check(_lib.lib().sf_grad_jk(fb.handle, _ptr(Dd), _ptr(g), _lib.PRECISION["fp64"], 1e-12, 0.0,
+                                         _stream_ptr()))
+        out.append((J[:n, :n].clone(), K[:n, :n].clone(), g[:3 * m].clone()))
+        fb.close()
+    for a, b, tol in zip(*out, (1e-12, 1e-12, 1e-11)):
+        assert float((a - b).abs().max()) <= tol * float(b.abs().max())
