@@ -153,13 +153,16 @@ int sf_fock_jk(sf_handle *h, const double *D, double *J, double *K, int32_t prec
  * Later builds with the same work lists use the recorded shapes.  Returns the
  * number of launches tuned (>= 0) or an error code.  The table can be read
  * out and loaded again (e.g. from a file): sf_set_tuning replaces it (n = 0
- * clears it).  Entries with cls = -1 hold the fill target of precision mode
- * `precision` in `split` (quarters; 0 = no extra split), entries with
- * cls = -2 that of the accurate tier of a mixed mode when it differs. */
+ * clears it).  An entry changes only a launch of its class, kind and cost;
+ * others are kept and change nothing (those for another molecule, or of files
+ * written when cost counted all primitive pairs).  Entries with cls = -1 hold
+ * the fill target of precision mode `precision` in `split` (quarters; 0 = no
+ * extra split), entries with cls = -2 that of the accurate tier of a mixed mode
+ * when it differs. */
 typedef struct {
     int32_t cls;           /* canonical class 0..20 (ss|ss .. dd|dd); -1 / -2: fill target */
     int32_t precision;     /* launch kind: 0 FP64, 1 FP32, 2 double-float; precision mode for cls < 0 */
-    int64_t cost;          /* K_ab*K_cd of the launch's first (costliest) quartet */
+    int64_t cost;          /* K_ab*K_cd (kept primitive pairs) of the launch's first (costliest) quartet */
     int32_t split;         /* chosen S = P*W (power of two)                   */
     float ms_default;      /* measured time with the rule's S                 */
     float ms_tuned;        /* measured time with the chosen S                 */
@@ -227,9 +230,9 @@ void sf_fock_graph_destroy(sf_fock_graph *g);
 
 /* How a Fock build launches its class kernels (no counterpart in the
  * reference, whose scheduler is Pool(8).map over AO quartets, hf.py:45-47):
- *  - SF_LAUNCH_STREAMS (default): one launch per (class, precision, primitive
- *    split) slice, spread over up to 32 side streams forked from the caller's
- *    stream and joined back;
+ *  - SF_LAUNCH_STREAMS (default): one launch per class and arithmetic, its
+ *    primitive splits as segments, spread over up to 32 side streams forked from
+ *    the caller's stream and joined back;
  *  - SF_LAUNCH_PERSISTENT: the FP32 register-path classes run as one
  *    persistent launch per register tier (four tiers of similar register
  *    use), each CTA taking CTA-sized tiles of the tier's lists from a device

@@ -665,14 +665,6 @@ std::vector<int> lpt_streams(const std::vector<double> &cost_desc, int first = 0
   return s;
 }
 
-// Quartet lists of every (class, precision) launch for the given cutoffs.
-// Each list holds the surviving canonical quartets (bra i, ket j) of one
-// class, ordered by decreasing primitive cost K_ab K_cd (then K_ab), stable,
-// so consecutive quartets -- the lanes and groups of one warp -- run the same
-// number of primitive iterations; inside a cost bucket the (i, j) order of the
-// Schwarz-sorted pair lists is kept.  A partition (part, nparts) keeps every
-// nparts-th quartet of each sorted list, which balances cost across parts.
-
 // The FP64 kernels' quartets with a Schwarz bound below this fraction of the square of
 // the largest Q run in double-float.  A double-float quartet carries 2^-48 relative
 // rounding instead of 2^-53, but its tables are the finer ones, and a quartet adds at
@@ -717,6 +709,13 @@ inline int kind_lanes(const ClassInfo &ci, int kind, int wide) {
   return kind == 1 ? ci.t32 : (kind == 2 && wide) ? tdd_wide(ci.la, ci.lb, ci.lc, ci.ld, ci.t64) : ci.t64;
 }
 
+// Quartet lists of every (class, precision) launch for the given cutoffs.
+// Each list holds the surviving canonical quartets (bra i, ket j) of one
+// class, ordered by decreasing primitive cost K_ab K_cd (then K_ab), stable,
+// so consecutive quartets -- the lanes and groups of one warp -- run the same
+// number of primitive iterations; inside a cost bucket the (i, j) order of the
+// Schwarz-sorted pair lists is kept.  A partition (part, nparts) keeps every
+// nparts-th quartet of each sorted list, which balances cost across parts.
 int cut_lists(sf_handle *h, int prec, double cut, double cut32) {
   const double q2 = h->qmax * h->qmax;
   const double tail_cut = h->dd_range && q2 >= kDDTailQ2[0] && q2 <= kDDTailQ2[1] ? kDDTail * q2 : 0.0;

@@ -278,6 +278,8 @@ template <typename V>
 __device__ __forceinline__ double acc_value(V v, double) { return to_f64(v); }
 
 // one-lane classes: primitive sub-groups per quartet from which they share its G_o
+// (2 / 4 / 8: forces of (H2O)8 FP32 + double-float 4.231 / 4.236 / 4.243 ms, (H2O)4 FP64
+// 4.046 / 4.048 / 4.059)
 constexpr int kGradCoop = 4;
 // shared memory before the CTA's sums: the groups' buffers, or the G_o of the
 // quartets of a one-lane class with kGradCoop or more lanes each

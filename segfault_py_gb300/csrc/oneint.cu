@@ -150,7 +150,7 @@ __device__ __forceinline__ float kinetic_bound(int la, int lb, float al, float b
 // coefficients grow at most as (|AB| + 1/sqrt(p) + 1)^L, kinetic terms as
 // kinetic_bound and attraction as 2 sqrt(p/pi) times the summed charge; the
 // bound itself in FP32).
-// (H2O)16 6-31G* (48 nuclei, 68 k primitive pairs): 0.32 ms; one CTA of 64 threads
+// (H2O)16 6-31G* (48 nuclei, 68 k primitive pairs): 0.30 ms; one CTA of 64 threads
 // per pair, with the power series, exp and pow per primitive pair and three
 // threads building E, took 3.8 ms.
 constexpr int kOneWarps = 4;
@@ -359,11 +359,11 @@ cudaError_t launch_one_electron(const OneParams &P, cudaStream_t st) {
 // and keeps the forces in its own shared-memory copy (one per group, so no
 // atomics), flushed once at the end: every pair adds to all 3 natom words.
 // Primitive pairs whose contributions all stay below 1e-15 are skipped (bounds
-// as in one_electron_kernel, times the block maximum of |D|, |W| and the growth
-// of a derivative, 2 max(alpha, beta) + L).
-// (H2O)16 6-31G*: the forces of (H2O)8, FP32 + double-float, 7.6 -> 6.4 ms; before (a CTA per pair, bra and ket Hermite
-// coefficients per primitive pair, one global atomic per nucleus and direction)
-// 3.9 ms.
+// as in one_electron_kernel with one more power on either side, times the block
+// maximum of |D|, |W| and the growth of a derivative, 2 max(alpha, beta) + L).
+// Forces of (H2O)8 6-31G*, FP32 + double-float, 7.6 -> 6.4 ms (before: a CTA per pair,
+// bra and ket Hermite coefficients per primitive pair, one global atomic per nucleus and
+// direction).
 constexpr int kOneGradWarps = 2;
 constexpr int kOneGradAtoms = 128;   // larger molecules add to global memory directly
 

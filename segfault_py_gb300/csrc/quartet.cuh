@@ -1514,7 +1514,10 @@ __device__ __forceinline__ void load_tab32_block(const KParams &kp, int nr, floa
   for (int k = threadIdx.x; k < ntab4; k += blockDim.x) tab4[k] = __ldg(src + k);
 }
 
-constexpr int kCoopLanes = 4;   // lanes from which a one-lane class digests a quartet with all of them
+// Lanes from which a one-lane class digests a quartet with all of them.  2 / 4 / 8: (H2O)4
+// FP64 0.840 / 0.840 / 0.845 ms, (H2O)8 FP32 + double-float replayed 1.053 / 1.054 /
+// 1.056; the buffer is half as large as with 2.
+constexpr int kCoopLanes = 4;
 
 // Digestion by all nl lanes that evaluated a quartet (nl <= 32: qmask; its integrals
 // in buf).  The four warps of a CTA that share one quartet (nl == 32 and W a multiple

@@ -10,7 +10,8 @@ Same names, arguments and iteration as the reference's src/hf/hf.py:
 Convergence is |E_n - E_{n-1}| <= tol, as in the reference.  The difference is
 the Fock build: ERIs are never stored; every iteration calls the GPU J/K
 builder (FockBuilder.jk), and S, T, V come from the GPU one-electron kernel.
-Everything stays on the device in FP64 (eigh, DIIS, energies).
+DIIS and energies stay on the device in FP64, eigenproblems of more than
+HOST_EIGH_MAX orbitals too; smaller ones go to the host's LAPACK.
 ``precision`` ('fp64', 'fp32', 'mixed'), ``cutoff`` and ``fp32_cutoff``
 default to the FockBuilder's settings (fp64, 1e-12, 1e-5 for a new one).
 """
