@@ -288,8 +288,8 @@ constexpr int kClsThreads = 256, kClsPer = 4, kClsChunk = kClsThreads * kClsPer;
 // gives 6.9e-8 / 4.5e-7 Eh/bohr, 1e-3 1.4e-7 / 1.05e-6, 1e-2 1.4e-6 / 9.8e-6
 // (the FP32 tier alone leaves 7e-8 / 3e-7)
 constexpr double kGradFp32Scale = 3e-2;
-// and the largest |D| for which a part of an FP64 gradient runs in double-float (what D
-// D times an integral may reach and keep a float pair's 48 bits)
+// and the largest |D| for which a part of an FP64 gradient runs in double-float: products
+// of two elements and an integral keep a float pair's 48 bits
 constexpr float kGradDDTailDMin = 1e-10f, kGradDDTailDMax = 1e10f;
 
 // M_xy = max |D| over the Cartesian block of shells x, y (FP32 is enough for a bound);
@@ -674,9 +674,10 @@ std::vector<int> lpt_streams(const std::vector<double> &cost_desc, int first = 0
 // McMurchie-Davidson values with no screening, everything in FP64 / with this part:
 // J of (H2O)16 6-31G* 7.1e-15, 3.0e-15 / 4.4e-15, 2.1e-15, K 7.4e-15, 5.5e-15 /
 // 3.6e-15, 3.3e-15; J of hexane 8.3e-15, 3.9e-15 / 9.9e-15, 3.8e-15, K 9.1e-15,
-// 1.4e-14 / 5.0e-15, 1.2e-14 (the largest errors vary by a fifth from run to run).  (An element of two functions
-// far apart, below 1e-6 of the largest, keeps fewer relative digits.)  (H2O)16
-// FP64 58.1 -> 19.9 ms.
+// 1.4e-14 / 5.0e-15, 1.2e-14 (the largest errors vary by a fifth from run to run; mean
+// of 13 molecules, FP64 kernels alone / now: J 3.3e-15, 2.1e-15 / 3.3e-15, 2.0e-15, K
+// 4.0e-15, 4.7e-15 / 3.9e-15, 4.6e-15).  (An element of two functions far apart, below
+// 1e-6 of the largest, keeps fewer relative digits.)  (H2O)16 FP64 58.1 -> 19.9 ms.
 // Gradients: the derivatives of a quartet outgrow its bound by about the square roots of
 // its exponents (classify_kernel), so bounds with that factor, weighted by the density,
 // decide, against the same threshold.  Largest error of the forces against 64-bit-mantissa
@@ -684,7 +685,8 @@ std::vector<int> lpt_streams(const std::vector<double> &cost_desc, int first = 0
 // out: butane 6-31G** 1.3-1.5e-12 / 2.2e-12 / 1.2-2.1e-12, (H2O)8 6-31G* 2.4-3.6e-13 /
 // 5.8e-13 / 3.8-4.4e-13 (ranges over runs of the same build).  FP64 forces of (H2O)4
 // 6-31G* 3.88 -> 4.06 ms, pentane 6-31G** 20.1 -> 20.7, (H2O)8 14.4 against 24.9
-// with everything in FP64; ten or a hundred times the threshold takes as long.
+// with everything in FP64; a tenth to a hundred times the threshold takes as long and
+// has the same errors.
 constexpr double kDDTail = 2e-4;
 // ... and for a largest Q whose square lies in this range, so that no integral that
 // counts comes near the ends of FP32's range
@@ -1243,9 +1245,9 @@ int build_persist(sf_handle *h) {
 // the classification ran for it), for a classified accurate-tier slice of
 // a mixed mode one FP32 launch of its demoted quartets on the next FP32
 // stream, and for the double-float part of an FP64 gradient one FP64 launch of
-// the quartets that the classification took out of it.  In the persistent launch mode (Fock builds, profiling off) the
-// slices of the register tiers are marked covered and one launch per tier
-// runs them, on the FP32 streams.
+// the quartets that the classification took out of it.  In the persistent
+// launch mode (Fock builds, profiling off) the slices of the register tiers are
+// marked covered and one launch per tier runs them, on the FP32 streams.
 int make_plan(sf_handle *h, bool grad, int active, bool no_dd) {
   h->plan.clear();
   h->pplan.clear();
